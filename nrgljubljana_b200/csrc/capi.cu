@@ -1,6 +1,7 @@
 // capi.cu -- the C-ABI of the NRG step core (include/nrg_b200.h): context, device
 // workspace, descriptor staging and the host-side planning of every batched launch.
 #include <algorithm>
+#include <climits>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -867,7 +868,8 @@ int nrg_spec_accumulate(nrg_ctx* c, int npair, const nrg_spec_pair* pairs, const
   auto s = static_cast<cudaStream_t>(stream);
   nrg::CallOrder call_order(c, s);
 
-  // GEMM-derived matrices in workspace.
+  // GEMM-derived matrices in workspace, each for the rectangle of terms that reads it: X and Y of
+  // DM-NRG over kept x kept, op2 rho of FDM-gt over K x D, rho op2 of FDM-ls over D x K.
   std::vector<size_t> xo(npair, 0), yo(npair, 0);
   size_t need = 0;
   for (int p = 0; p < npair; p++) {
@@ -879,10 +881,10 @@ int nrg_spec_accumulate(nrg_ctx* c, int npair, const nrg_spec_pair* pairs, const
       yo[p] = need; need += (size_t)q.kj * q.ki;
     } else if (prm->algo == NRG_SPEC_FDMGT) {
       if (q.ki > q.rdi) return fail(NRG_ERR_ARG, "pair %d: rdi < ki", p);
-      xo[p] = need; need += (size_t)q.nj * q.rdi;
+      xo[p] = need; need += (size_t)(q.nj - q.kj) * q.ki;
     } else {
       if (q.kj > q.rdj) return fail(NRG_ERR_ARG, "pair %d: rdj < kj", p);
-      xo[p] = need; need += (size_t)q.rdj * q.ni;
+      xo[p] = need; need += (size_t)q.kj * (q.ni - q.ki);
     }
   }
   rc = ensure_ws(c, sizeof(double) * std::max<size_t>(need, 1));
@@ -890,22 +892,24 @@ int nrg_spec_accumulate(nrg_ctx* c, int npair, const nrg_spec_pair* pairs, const
   double* W = static_cast<double*>(c->ws);
   GemmPlan gp;
   std::vector<nrg::SpecRegion> regs;
-  auto region = [&](const nrg_spec_pair& q, int kind, int i0, int i1, int j0, int j1, const double* X, int64_t ldx,
-                    const double* Y, int64_t ldy, double coef) {
+  int64_t terms = 0;
+  auto region = [&](const nrg_spec_pair& q, int kind, int i0, int i1, int j0, int j1, const double* X,
+                    const double* Y, double coef) {
     if (i1 <= i0 || j1 <= j0) return;
     nrg::SpecRegion r{};
     r.Ei = q.Ei; r.Ej = q.Ej; r.op1 = q.op1; r.op2 = q.op2; r.X = X; r.Y = Y;
-    r.ld1 = q.ld1; r.ld2 = q.ld2; r.ldx = ldx; r.ldy = ldy;
+    r.ld1 = q.ld1; r.ld2 = q.ld2; r.ldx = i1 - i0; r.ldy = i1 - i0;
     r.i0 = i0; r.i1 = i1; r.j0 = j0; r.j1 = j1;
     r.kind = kind; r.sign = prm->sign; r.coef = coef; r.factor = q.factor; r.T = prm->T;
     r.Emin = prm->Emin; r.Emax = prm->Emax;
+    terms += (int64_t)(i1 - i0) * (j1 - j0);
     regs.push_back(r);
   };
   for (int p = 0; p < npair; p++) {
     const nrg_spec_pair& q = pairs[p];
+    double* X = W + xo[p];
     if (prm->algo == NRG_SPEC_DMNRG) {
       if (q.ki == 0 || q.kj == 0) continue;
-      double* X = W + xo[p];
       double* Y = W + yo[p];
       // X(rj, rm) = sum_ri op2(rj, ri) rho_i(rm, ri)   (algo_DMNRG.hpp:38)
       gp.add_out(X, q.ki, q.kj, q.ki, 0.0);
@@ -913,46 +917,40 @@ int nrg_spec_accumulate(nrg_ctx* c, int npair, const nrg_spec_pair* pairs, const
       // Y(rj, rm) = sum_ri rho_j(rj, ri) op1(ri, rm)   (algo_DMNRG.hpp:41)
       gp.add_out(Y, q.ki, q.kj, q.ki, 0.0);
       gp.add_seg(q.rho_j, q.ldrj, 0, q.op1, q.ld1, 0, q.kj, 1.0);
-      region(q, nrg::kSpecDMNRG, 0, q.ki, 0, q.kj, X, q.ki, Y, q.ki, 0.0);
+      region(q, nrg::kSpecDMNRG, 0, q.ki, 0, q.kj, X, Y, 0.0);
     } else if (prm->algo == NRG_SPEC_FDMGT) {
       // op2_rho = prod_fit(op2, rhoFDM(Ii)) (algo_FDM.hpp:89, numerics.hpp:283-306)
-      double* X = W + xo[p];
-      if (q.rdi > 0 && q.nj > 0) {
-        gp.add_out(X, q.rdi, q.nj, q.rdi, 0.0);
-        gp.add_seg(q.op2, q.ld2, 0, q.rho_i, q.ldri, 0, std::min(q.rdi, q.ni), 1.0);
+      if (q.ki > 0 && q.nj > q.kj) {
+        gp.add_out(X, q.ki, q.nj - q.kj, q.ki, 0.0);
+        gp.add_seg(q.op2 + q.kj * q.ld2, q.ld2, 0, q.rho_i, q.ldri, 0, std::min(q.rdi, q.ni), 1.0);
       }
-      region(q, nrg::kSpecExpI, q.ki, q.ni, 0, q.nj, nullptr, 0, nullptr, 0, prm->wnf);   // D x (D + K)
-      region(q, nrg::kSpecGemmX, 0, q.ki, q.kj, q.nj, X, q.rdi, nullptr, 0, 1.0);         // K x D
+      region(q, nrg::kSpecExpI, q.ki, q.ni, 0, q.nj, nullptr, nullptr, prm->wnf);   // D x (D + K)
+      region(q, nrg::kSpecGemmX, 0, q.ki, q.kj, q.nj, X, nullptr, 1.0);             // K x D
     } else {
       // rho_op2 = prod_fit(rhoFDM(Ij), op2) (algo_FDM.hpp:35)
-      double* X = W + xo[p];
-      if (q.rdj > 0 && q.ni > 0) {
-        gp.add_out(X, q.ni, q.rdj, q.ni, 0.0);
-        gp.add_seg(q.rho_j, q.ldrj, 0, q.op2, q.ld2, 0, std::min(q.rdj, q.nj), 1.0);
+      if (q.kj > 0 && q.ni > q.ki) {
+        gp.add_out(X, q.ni - q.ki, q.kj, q.ni - q.ki, 0.0);
+        gp.add_seg(q.rho_j, q.ldrj, 0, q.op2 + q.ki, q.ld2, 0, std::min(q.rdj, q.nj), 1.0);
       }
       const double ms = (double)(-prm->sign);
-      region(q, nrg::kSpecExpJ, 0, q.ni, q.kj, q.nj, nullptr, 0, nullptr, 0, ms * prm->wnf);  // (D + K) x D
-      region(q, nrg::kSpecGemmX, q.ki, q.ni, 0, q.kj, X, q.ni, nullptr, 0, ms);                // D x K
+      region(q, nrg::kSpecExpJ, 0, q.ni, q.kj, q.nj, nullptr, nullptr, ms * prm->wnf);  // (D + K) x D
+      region(q, nrg::kSpecGemmX, q.ki, q.ni, 0, q.kj, X, nullptr, ms);                  // D x K
     }
   }
-  rc = run_gemm_plan(c, gp, s, nrg::kPhSpecGemm);
-  if (rc) return rc;
   if (regs.empty()) return NRG_OK;
-  std::vector<nrg::SpecTask> tasks;
-  const int64_t chunk = 8192;
-  for (size_t r = 0; r < regs.size(); r++) {
-    const int64_t nt = (int64_t)(regs[r].i1 - regs[r].i0) * (regs[r].j1 - regs[r].j0);
-    for (int64_t t0 = 0; t0 < nt; t0 += chunk) {
-      nrg::SpecTask k{};
-      k.t0 = t0;
-      k.t1 = std::min(nt, t0 + chunk);
-      k.region = (int)r;
-      tasks.push_back(k);
-    }
+  const int rows = nrg::spec_tile_rows(terms);
+  int64_t tiles = 0;
+  for (auto& r : regs) {
+    r.tile0 = (int)tiles;
+    tiles += nrg::spec_tiles(r.i0, r.i1, r.j0, r.j1, rows);
+    if (tiles > INT_MAX) return fail(NRG_ERR_ARG, "too many terms in one call");
   }
   std::vector<char> img;
-  const size_t ro = push(img, regs), to = push(img, tasks);
+  const nrg::StagedGemm g = nrg::stage_gemm(img, gp);
+  const size_t ro = push(img, regs);
   rc = stage_desc(c, img, s);
+  if (rc) return rc;
+  rc = nrg::launch_staged_gemm(c, g, s, nrg::kPhSpecGemm);
   if (rc) return rc;
   nrg::BinParams bp{};
   bp.log10emin = bins->log10emin;
@@ -961,8 +959,8 @@ int nrg_spec_accumulate(nrg_ctx* c, int npair, const nrg_spec_pair* pairs, const
   bp.nbins = bins->nbins;
   const char* base = static_cast<const char*>(c->desc);
   nrg::PhaseScope ps(c, nrg::kPhSpecBin, s);
-  CK(nrg::spec_bin_launch(reinterpret_cast<const nrg::SpecTask*>(base + to), (int)tasks.size(),
-                          reinterpret_cast<const nrg::SpecRegion*>(base + ro), bp, pos, neg, s));
+  CK(nrg::spec_bin_launch(reinterpret_cast<const nrg::SpecRegion*>(base + ro), (int)regs.size(), tiles, rows, bp, pos,
+                          neg, s));
   return NRG_OK;
 }
 
@@ -979,8 +977,8 @@ int nrg_spec_accumulate_mats(nrg_ctx* c, int npair, const nrg_spec_pair* pairs, 
     return fail(NRG_ERR_ARG, "bad algo %d for the Matsubara sums", algo);
   auto s = static_cast<cudaStream_t>(stream);
   nrg::CallOrder call_order(c, s);
-  // FDMmats: op2_rho = prod_fit(op2, rhoFDM(Ii)) (nj x rdi) and rho_op2 = prod_fit(rhoFDM(Ij), op2)
-  // (rdj x ni); DMNRGmats: X and Y of the DM-NRG weights (ki x kj... as NRG_SPEC_DMNRG)
+  // FDMmats: op2_rho = prod_fit(op2, rhoFDM(Ii)) over K x D and rho_op2 = prod_fit(rhoFDM(Ij), op2)
+  // over D x K; DMNRGmats: X and Y of the DM-NRG weights over kept x kept
   std::vector<size_t> xo(npair, 0), yo(npair, 0);
   size_t need = 0;
   for (int p = 0; p < npair; p++) {
@@ -994,22 +992,23 @@ int nrg_spec_accumulate_mats(nrg_ctx* c, int npair, const nrg_spec_pair* pairs, 
     }
     if (algo == NRG_SPEC_FTMATS) continue;
     if (q.ki > q.rdi || q.kj > q.rdj) return fail(NRG_ERR_ARG, "pair %d: rdi < ki or rdj < kj", p);
-    xo[p] = need; need += (size_t)q.nj * q.rdi;
-    yo[p] = need; need += (size_t)q.rdj * q.ni;
+    xo[p] = need; need += (size_t)(q.nj - q.kj) * q.ki;
+    yo[p] = need; need += (size_t)q.kj * (q.ni - q.ki);
   }
   rc = ensure_ws(c, sizeof(double) * std::max<size_t>(need, 1));
   if (rc) return rc;
   double* W = static_cast<double*>(c->ws);
   GemmPlan gp;
   std::vector<nrg::SpecRegion> regs;
-  auto region = [&](const nrg_spec_pair& q, int kind, int i0, int i1, int j0, int j1, const double* X, int64_t ldx,
-                    double coef, int special) {
+  auto region = [&](const nrg_spec_pair& q, int kind, int i0, int i1, int j0, int j1, const double* X, const double* Y,
+                    double coef, double coef2, int special) {
     if (i1 <= i0 || j1 <= j0) return;
     nrg::SpecRegion r{};
-    r.Ei = q.Ei; r.Ej = q.Ej; r.op1 = q.op1; r.op2 = q.op2; r.X = X; r.Y = nullptr;
-    r.ld1 = q.ld1; r.ld2 = q.ld2; r.ldx = ldx; r.ldy = 0;
+    r.Ei = q.Ei; r.Ej = q.Ej; r.op1 = q.op1; r.op2 = q.op2; r.X = X; r.Y = Y;
+    r.ld1 = q.ld1; r.ld2 = q.ld2; r.ldx = i1 - i0; r.ldy = i1 - i0;
     r.i0 = i0; r.i1 = i1; r.j0 = j0; r.j1 = j1;
-    r.kind = kind; r.sign = prm->sign; r.mspecial = special; r.coef = coef; r.factor = q.factor; r.T = prm->T;
+    r.kind = kind; r.sign = prm->sign; r.mspecial = special; r.coef = coef; r.coef2 = coef2; r.factor = q.factor;
+    r.T = prm->T; r.Emin = -1.0; r.Emax = 1e300;  // no energy window
     regs.push_back(r);
   };
   const double ms = (double)(-prm->sign);
@@ -1017,61 +1016,46 @@ int nrg_spec_accumulate_mats(nrg_ctx* c, int npair, const nrg_spec_pair* pairs, 
     const nrg_spec_pair& q = pairs[p];
     double* X = W + xo[p];
     double* Y = W + yo[p];
-    if (algo == NRG_SPEC_DMNRG) {  // Algo_DMNRGmats: the DM-NRG weights over kept x kept, no window
+    if (algo == NRG_SPEC_DMNRG) {  // Algo_DMNRGmats: the DM-NRG weights over kept x kept
       if (q.ki == 0 || q.kj == 0) continue;
       gp.add_out(X, q.ki, q.kj, q.ki, 0.0);
       gp.add_seg(q.op2, q.ld2, 0, q.rho_i, q.ldri, 1, q.ki, 1.0);
       gp.add_out(Y, q.ki, q.kj, q.ki, 0.0);
       gp.add_seg(q.rho_j, q.ldrj, 0, q.op1, q.ld1, 0, q.kj, 1.0);
-      nrg::SpecRegion r{};
-      r.Ei = q.Ei; r.Ej = q.Ej; r.op1 = q.op1; r.op2 = q.op2; r.X = X; r.Y = Y;
-      r.ld1 = q.ld1; r.ld2 = q.ld2; r.ldx = q.ki; r.ldy = q.ki;
-      r.i0 = 0; r.i1 = q.ki; r.j0 = 0; r.j1 = q.kj;
-      r.kind = nrg::kSpecDMNRG; r.sign = prm->sign; r.mspecial = nrg::kMatsDmnrgA; r.factor = q.factor;
-      r.T = prm->T; r.Emin = -1.0; r.Emax = 1e300;
-      regs.push_back(r);
+      region(q, nrg::kSpecDMNRG, 0, q.ki, 0, q.kj, X, Y, 0.0, 0.0, nrg::kMatsDmnrgA);
       continue;
     }
     if (algo == NRG_SPEC_FTMATS) {  // Algo_FTmats: the two exponentials over the pair's states
-      region(q, nrg::kSpecExpI, 0, q.ni, 0, q.nj, nullptr, 0, prm->wnf, nrg::kMatsZero);
-      region(q, nrg::kSpecExpJ, 0, q.ni, 0, q.nj, nullptr, 0, ms * prm->wnf, nrg::kMatsPlusOverT);
+      region(q, nrg::kSpecExpIJ, 0, q.ni, 0, q.nj, nullptr, nullptr, prm->wnf, ms * prm->wnf, nrg::kMatsFtB);
       continue;
     }
-    if (q.rdi > 0 && q.nj > 0) {
-      gp.add_out(X, q.rdi, q.nj, q.rdi, 0.0);
-      gp.add_seg(q.op2, q.ld2, 0, q.rho_i, q.ldri, 0, std::min(q.rdi, q.ni), 1.0);
+    if (q.ki > 0 && q.nj > q.kj) {
+      gp.add_out(X, q.ki, q.nj - q.kj, q.ki, 0.0);
+      gp.add_seg(q.op2 + q.kj * q.ld2, q.ld2, 0, q.rho_i, q.ldri, 0, std::min(q.rdi, q.ni), 1.0);
     }
-    if (q.rdj > 0 && q.ni > 0) {
-      gp.add_out(Y, q.ni, q.rdj, q.ni, 0.0);
-      gp.add_seg(q.rho_j, q.ldrj, 0, q.op2, q.ld2, 0, std::min(q.rdj, q.nj), 1.0);
+    if (q.kj > 0 && q.ni > q.ki) {
+      gp.add_out(Y, q.ni - q.ki, q.kj, q.ni - q.ki, 0.0);
+      gp.add_seg(q.rho_j, q.ldrj, 0, q.op2 + q.ki, q.ld2, 0, std::min(q.rdj, q.nj), 1.0);
     }
     // term1 (D x D): weightA (exp(-Ei/T)) + weightB (-sign exp(-Ej/T)); term2 (i in D, j in K):
     // weightA + (-sign) op1 rho_op2; term3 (i in K, j in D): op1 op2_rho + weightB
-    region(q, nrg::kSpecExpI, q.ki, q.ni, q.kj, q.nj, nullptr, 0, prm->wnf, nrg::kMatsMinusOverT);
-    region(q, nrg::kSpecExpJ, q.ki, q.ni, q.kj, q.nj, nullptr, 0, ms * prm->wnf, nrg::kMatsZero);
-    region(q, nrg::kSpecExpI, q.ki, q.ni, 0, q.kj, nullptr, 0, prm->wnf, nrg::kMatsPlain);
-    region(q, nrg::kSpecGemmX, q.ki, q.ni, 0, q.kj, Y, q.ni, ms, nrg::kMatsPlain);
-    region(q, nrg::kSpecGemmX, 0, q.ki, q.kj, q.nj, X, q.rdi, 1.0, nrg::kMatsPlain);
-    region(q, nrg::kSpecExpJ, 0, q.ki, q.kj, q.nj, nullptr, 0, ms * prm->wnf, nrg::kMatsPlain);
+    region(q, nrg::kSpecExpIJ, q.ki, q.ni, q.kj, q.nj, nullptr, nullptr, prm->wnf, ms * prm->wnf, nrg::kMatsFdmA);
+    region(q, nrg::kSpecExpIX, q.ki, q.ni, 0, q.kj, Y, nullptr, prm->wnf, ms, nrg::kMatsPlain);
+    region(q, nrg::kSpecXExpJ, 0, q.ki, q.kj, q.nj, X, nullptr, 1.0, ms * prm->wnf, nrg::kMatsPlain);
   }
-  rc = run_gemm_plan(c, gp, s, nrg::kPhSpecGemm);
-  if (rc) return rc;
   if (regs.empty()) return NRG_OK;
-  std::vector<nrg::SpecTask> tasks;
-  const int64_t chunk = 4096;
-  for (size_t r = 0; r < regs.size(); r++) {
-    const int64_t nt = (int64_t)(regs[r].i1 - regs[r].i0) * (regs[r].j1 - regs[r].j0);
-    for (int64_t t0 = 0; t0 < nt; t0 += chunk) {
-      nrg::SpecTask k{};
-      k.t0 = t0;
-      k.t1 = std::min(nt, t0 + chunk);
-      k.region = (int)r;
-      tasks.push_back(k);
-    }
+  int64_t chunks = 0;
+  for (auto& r : regs) {
+    r.tile0 = (int)chunks;
+    chunks += nrg::mats_chunks(r.i0, r.i1, r.j0, r.j1);
+    if (chunks > INT_MAX) return fail(NRG_ERR_ARG, "too many terms in one call");
   }
   std::vector<char> img;
-  const size_t ro = push(img, regs), to = push(img, tasks);
+  const nrg::StagedGemm g = nrg::stage_gemm(img, gp);
+  const size_t ro = push(img, regs);
   rc = stage_desc(c, img, s);
+  if (rc) return rc;
+  rc = nrg::launch_staged_gemm(c, g, s, nrg::kPhSpecGemm);
   if (rc) return rc;
   nrg::MatsParams mp{};
   mp.mats = mats;
@@ -1079,8 +1063,8 @@ int nrg_spec_accumulate_mats(nrg_ctx* c, int npair, const nrg_spec_pair* pairs, 
   mp.T = prm->T;
   const char* base = static_cast<const char*>(c->desc);
   nrg::PhaseScope ps(c, nrg::kPhSpecBin, s);
-  CK(nrg::spec_mats_launch(reinterpret_cast<const nrg::SpecTask*>(base + to), (int)tasks.size(),
-                           reinterpret_cast<const nrg::SpecRegion*>(base + ro), mp, re, im, s));
+  CK(nrg::spec_mats_launch(reinterpret_cast<const nrg::SpecRegion*>(base + ro), (int)regs.size(), chunks, mp, re, im,
+                           s));
   return NRG_OK;
 }
 
