@@ -671,7 +671,10 @@ int nrg_gemm3_batch(nrg_ctx* c, int nterm, const nrg_gemm3* terms, void* stream)
     for (int t : glist.back()) need += tsize(t);
   }
   std::vector<std::vector<std::vector<int>>> passes;
-  const size_t cap = std::max(c->ws_size, nrg::ws_available(c)) / sizeof(double);
+  // The device is asked for its free memory only when the arena as it is does not hold the call:
+  // cudaMemGetInfo now and then stalls the host for milliseconds.
+  const bool fits = need <= c->ws_size / sizeof(double);
+  const size_t cap = (fits ? c->ws_size : std::max(c->ws_size, nrg::ws_available(c))) / sizeof(double);
   if (need <= cap) {
     passes.push_back(std::move(glist));
   } else {

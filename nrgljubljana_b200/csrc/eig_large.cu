@@ -1603,7 +1603,12 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
     if (n[b] > kMaxLargeN)
       return fail(NRG_ERR_ARG, "block %d: order %d exceeds the supported maximum %d", b, n[b], kMaxLargeN);
   // Chunk the blocks so that their workspaces fit in the context limit.
-  const size_t limit = ws_available(c);  // chunks fit what the arena can grow to now
+  size_t all_bytes = 0;
+  for (size_t t = 0; t < ord.size(); t++)
+    all_bytes += align_up(sizeof(double) * large_block_doubles(n[ord[t]], (int)t < nts_all), 256);
+  // Chunks fit what the arena can grow to now; a call that fits the arena as it is asks the device
+  // for nothing (cudaMemGetInfo now and then stalls the host for milliseconds).
+  const size_t limit = all_bytes <= c->ws_size ? c->ws_size : ws_available(c);
   size_t pos = 0;
   while (pos < ord.size()) {
     size_t bytes = 0, end = pos;
