@@ -44,6 +44,14 @@ constexpr int kMaxLargeN = 10240;  // the tridiagonalisation's shared memory (68
 constexpr size_t kPrepSmemMax = 200 * 1024;
 constexpr size_t kPrepGlobalB = 80;
 
+// Deflation rotation of the eigenvector rows p and j (rows of the node): (p, j) <- (c p - s j,
+// s p + c j). sup: supports of the two rows before it, p's in bits 0-1 and j's in bits 2-3 (1: the
+// first child's columns, 2: the second's); outside its support a row is zero (and not stored).
+struct DcRot {
+  double c, s;
+  int p, j, sup, pad;
+};
+
 struct LargeBlock {
   double* H;      // input (consumed); then the eigenvector rows of T during divide and
                   // conquer; then the VT factors of the back-transform
@@ -62,6 +70,8 @@ struct LargeBlock {
   int* rank;      // per node: sorted position of grouped entry
   int* perm;      // final eigenvalue order
   char* pscr;     // kPrepGlobalB bytes per row: merge-prep arrays of nodes too large for shared memory
+  int2* slot;     // per node row: (grouped slot, support) of the eigenvector row
+  DcRot* rot;     // per node: deflation rotations, in order
   int* info;
   int n, npanel;
   int ldp, pad_;  // leading dimension of the packed lower triangle in W1 (multiple of 32)
@@ -80,6 +90,7 @@ struct DcNode {
 struct DcState {
   int K, k1, k2, k3;
   double rho;
+  int nrot, pad;
 };
 
 // ---------------------------------------------------------------- tridiagonalisation
@@ -1090,7 +1101,7 @@ __global__ void __launch_bounds__(128) dc_leaf_kernel(const LargeBlock* __restri
 // ---------------------------------------------------------------- divide and conquer: merge prep
 // Shared-memory layout for a node of order N (P = next power of two >= N).
 struct PrepLayout {
-  size_t key, sidx, zs, lst, rcs, rpos, fl, total;
+  size_t key, sidx, zs, lst, flg, fl, total;
 };
 
 __host__ __device__ inline size_t r16(size_t x) { return (x + 15) & ~(size_t)15; }
@@ -1103,21 +1114,50 @@ __host__ __device__ inline PrepLayout prep_layout(int N) {
   L.key = o;  o += r16(sizeof(double) * (size_t)P);   // pole values, sorted
   L.sidx = o; o += r16(sizeof(int) * (size_t)P);      // original position
   L.zs = o;   o += r16(sizeof(double) * (size_t)N);   // z in sorted order
-  L.lst = o;  o += r16(sizeof(int) * (size_t)N);      // non-deflated from the front, deflated from the back
-  L.rcs = o;  o += r16(sizeof(double2) * (size_t)N);  // rotation (c, s)
-  L.rpos = o; o += r16(sizeof(int2) * (size_t)N);     // rotation (pos_p, pos_j), later: grouped slot
-  L.fl = o;   o += r16((size_t)N);                    // support flags per sorted position
+  L.lst = o;  o += r16(sizeof(int) * (size_t)N);      // sorted positions with a coupling above the tolerance
+  L.flg = o;  o += r16(sizeof(int) * (size_t)N);      // those of them that are close to their successor
+  L.fl = o;   o += r16((size_t)N);                    // support per sorted position; 0x80: deflated
   L.total = o;
   return L;
 }
 
+// Exclusive scan over the block of one 64-bit count per thread; `total` gets the sum. `red` holds
+// one word per warp; every thread takes part.
+NRG_DEV unsigned long long block_scan(unsigned long long v, unsigned long long* red, unsigned long long& total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  unsigned long long x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long u = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += u;
+  }
+  __syncthreads();  // the previous call's reads of red
+  if (lane == 31) red[wid] = x;
+  __syncthreads();
+  unsigned long long before = 0;
+  total = 0;
+  for (int w = 0; w < nw; w++) {
+    if (w < wid) before += red[w];
+    total += red[w];
+  }
+  return before + x - v;
+}
+
+// Poles and z of a merge, deflation, grouping of the rows by support. Everything that moves
+// eigenvector rows is left to dc_secular_kernel's row CTAs, which spread over the chip; this
+// kernel, one CTA per node, keeps to O(N) data. The deflation of close poles is a serial
+// recurrence, but only where neighbours are close: whether a pair is close before any rotation
+// is tested for all pairs at once, and one thread follows the recurrence from each such pair to
+// its end. Measured on B200, 40 blocks up to order 480 (4 levels): 0.73 ms with the scan, the
+// grouping and the row copies in one CTA, 0.09 ms so.
 __global__ void __launch_bounds__(512) dc_prep_kernel(const LargeBlock* __restrict__ blocks,
                                                       const DcNode* __restrict__ nodes, DcState* __restrict__ states,
                                                       GemmOut* __restrict__ gouts, GemmSeg* __restrict__ gsegs,
                                                       size_t smem_bytes) {
   extern __shared__ __align__(16) double sm[];
   __shared__ double red[32];
-  __shared__ int cnt[8];
+  __shared__ unsigned long long sred[32];
+  __shared__ int s_nrot;
   const DcNode nd = nodes[blockIdx.x];
   const LargeBlock B = blocks[nd.blk];
   const int n = B.n, a = nd.a, m = nd.m, b = nd.b, N = b - a;
@@ -1132,21 +1172,12 @@ __global__ void __launch_bounds__(512) dc_prep_kernel(const LargeBlock* __restri
   int* sidx = reinterpret_cast<int*>(smc + PL.sidx);
   double* zs = reinterpret_cast<double*>(smc + PL.zs);
   int* lst = reinterpret_cast<int*>(smc + PL.lst);
-  double2* rcs = reinterpret_cast<double2*>(smc + PL.rcs);
-  int2* rpos = reinterpret_cast<int2*>(smc + PL.rpos);
+  int* flg = reinterpret_cast<int*>(smc + PL.flg);
   unsigned char* fl = reinterpret_cast<unsigned char*>(smc + PL.fl);
-  double* Z = B.H;
-  double* G = B.W2;
+  const double* Z = B.H;
+  DcRot* rot = B.rot + a;
 
-  // 1. clear the off-diagonal child blocks of the node
-  const int n1 = m - a, n2 = b - m;
-  for (int idx = tid; idx < n1 * n2; idx += nt) {
-    const int r = idx / n2, c = idx % n2;
-    Z[(size_t)(a + r) * n + m + c] = 0.0;
-    const int r2 = idx / n1, c2 = idx % n1;
-    Z[(size_t)(m + r2) * n + a + c2] = 0.0;
-  }
-  // 2. poles and the rank-one vector z = [last row of child 1; sign(beta) first row of child 2] / sqrt(2)
+  // 1. poles and the rank-one vector z = [last row of child 1; sign(beta) first row of child 2] / sqrt(2)
   const double beta = B.e[m - 1];
   const double rho = 2.0 * fabs(beta);
   const double sg = beta >= 0.0 ? 1.0 : -1.0;
@@ -1155,7 +1186,7 @@ __global__ void __launch_bounds__(512) dc_prep_kernel(const LargeBlock* __restri
     sidx[s] = s;
   }
   __syncthreads();
-  // 3. bitonic sort (key, sidx) ascending
+  // 2. bitonic sort (key, sidx) ascending
   for (int k = 2; k <= P; k <<= 1) {
     for (int jb = k >> 1; jb > 0; jb >>= 1) {
       for (int i = tid; i < P; i += nt) {
@@ -1177,11 +1208,21 @@ __global__ void __launch_bounds__(512) dc_prep_kernel(const LargeBlock* __restri
     }
   }
   // A non-finite pole (the block was already flagged) could move a padding slot forward:
-  // leave such a node untouched rather than index outside it.
+  // merge nothing at such a node rather than index outside it (its rows stay where they are).
   int badidx = 0;
   for (int s = tid; s < N; s += nt) badidx |= (sidx[s] >= N);
   if (__syncthreads_or(badidx)) {
-    if (tid == 0) atomicMin(B.info, -3);
+    for (int s = tid; s < N; s += nt) B.slot[a + s] = make_int2(s, a + s < m ? 1 : 2);
+    if (tid == 0) {
+      atomicMin(B.info, -3);
+      DcState st{};
+      st.rho = rho;
+      states[blockIdx.x] = st;
+      for (int q = 0; q < 2; q++) {
+        gouts[nd.gout + q].M = 0;
+        gsegs[nd.gout + q].K = 0;
+      }
+    }
     return;
   }
   double dmx = 0.0, zmx = 0.0;
@@ -1195,99 +1236,115 @@ __global__ void __launch_bounds__(512) dc_prep_kernel(const LargeBlock* __restri
   }
   dmx = block_max(dmx, red);
   zmx = block_max(zmx, red);
-  // 4. deflation scan (serial)
-  if (tid == 0) {
-    const double tol = 8.0 * kEps * fmax(dmx, zmx);
-    int K = 0, nd_ = 0, nrot = 0;
-    if (rho * zmx <= tol) {
-      for (int s = 0; s < N; s++) lst[N - 1 - (nd_++)] = s;
-    } else {
-      int p = -1;
-      for (int s = 0; s < N; s++) {
-        if (rho * fabs(zs[s]) <= tol) {
-          lst[N - 1 - (nd_++)] = s;
-          continue;
-        }
-        if (p < 0) {
-          p = s;
-          continue;
-        }
-        const double zp = zs[p], zj = zs[s];
-        const double t = hypot(zp, zj);
-        const double c = zj / t, sn = zp / t;
-        if (fabs((key[s] - key[p]) * c * sn) <= tol) {
-          // rotate rows (p, s): z_p -> 0, z_s -> t; p deflates
-          rcs[nrot] = make_double2(c, sn);
-          rpos[nrot] = make_int2(p, s);
-          nrot++;
-          const double dp = key[p], ds = key[s];
-          key[p] = c * c * dp + sn * sn * ds;
-          key[s] = sn * sn * dp + c * c * ds;
-          zs[s] = t;
-          zs[p] = 0.0;
-          fl[s] |= fl[p];
-          fl[p] |= fl[s];
-          lst[N - 1 - (nd_++)] = p;
-          p = s;
-        } else {
-          lst[K++] = p;
-          p = s;
-        }
-      }
-      if (p >= 0) lst[K++] = p;
+  const double tol = 8.0 * kEps * fmax(dmx, zmx);
+  const bool none = rho * zmx <= tol;  // nothing couples the children
+  // 3. deflation of small couplings; the rest in order. Thread t has the positions [s0, s1).
+  const int per = (N + nt - 1) / nt, s0 = min(N, tid * per), s1 = min(N, s0 + per);
+  unsigned long long total;
+  int cnt = 0;
+  for (int s = s0; s < s1; s++) {
+    if (none || rho * fabs(zs[s]) <= tol) fl[s] |= 0x80;
+    else cnt++;
+  }
+  int o = (int)block_scan(cnt, sred, total);
+  for (int s = s0; s < s1; s++)
+    if (!(fl[s] & 0x80)) lst[o++] = s;
+  const int L0 = (int)total;
+  __syncthreads();
+  // 4. close neighbours: for p, s = lst[q], lst[q+1] the rotation that zeroes z_p couples the two
+  //    poles by (d_s - d_p) c sn
+  auto close_pair = [&](int p, int s, double& t, double& c, double& sn) {
+    const double zp = zs[p], zj = zs[s];
+    t = hypot(zp, zj);
+    c = zj / t;
+    sn = zp / t;
+    return fabs((key[s] - key[p]) * c * sn) <= tol;
+  };
+  const int perl = (L0 + nt - 1) / nt, q0 = min(L0, tid * perl), q1 = min(L0, q0 + perl);
+  cnt = 0;
+  unsigned cl = 0;  // one bit per position: perl <= 20 (the launch's thread count grows with N)
+  for (int q = q0; q < q1; q++) {
+    double t, c, sn;
+    if (q + 1 < L0 && close_pair(lst[q], lst[q + 1], t, c, sn)) {
+      cl |= 1u << (q - q0);
+      cnt++;
     }
-    cnt[0] = K;
-    cnt[1] = nd_;
-    cnt[2] = nrot;
+  }
+  o = (int)block_scan(cnt, sred, total);
+  for (int q = q0; q < q1; q++)
+    if (cl >> (q - q0) & 1) flg[o++] = q;
+  const int F = (int)total;
+  __syncthreads();
+  // 5. the chains of rotations (p, s): z_p -> 0, z_s -> t; p deflates, and s goes on with its new
+  //    pole and coupling
+  if (tid == 0) {
+    int nrot = 0, done = 0;  // list positions below `done` are settled
+    for (int f = 0; f < F; f++) {
+      int q = flg[f];
+      if (q < done) continue;
+      while (q + 1 < L0) {
+        const int p = lst[q], s = lst[q + 1];
+        double t, c, sn;
+        if (!close_pair(p, s, t, c, sn)) break;
+        DcRot R;
+        R.c = c;
+        R.s = sn;
+        R.p = sidx[p];
+        R.j = sidx[s];
+        R.sup = fl[p] | fl[s] << 2;
+        R.pad = 0;
+        rot[nrot++] = R;
+        const double dp = key[p], ds = key[s];
+        key[p] = c * c * dp + sn * sn * ds;
+        key[s] = sn * sn * dp + c * c * ds;
+        zs[s] = t;
+        zs[p] = 0.0;
+        const unsigned char u = fl[p] | fl[s];
+        fl[s] = u;
+        fl[p] = u | 0x80;
+        q++;
+      }
+      done = q;
+    }
+    s_nrot = nrot;
   }
   __syncthreads();
-  const int K = cnt[0], ndefl = cnt[1], nrot = cnt[2];
-  // 5. apply the deflation rotations to the eigenvector rows, in order
-  for (int r = 0; r < nrot; r++) {
-    const double c = rcs[r].x, sn = rcs[r].y;
-    const size_t rp = (size_t)(a + sidx[rpos[r].x]) * n, rj = (size_t)(a + sidx[rpos[r].y]) * n;
-    for (int col = a + tid; col < b; col += nt) {
-      const double zp = Z[rp + col], zj = Z[rj + col];
-      Z[rp + col] = c * zp - sn * zj;
-      Z[rj + col] = sn * zp + c * zj;
-    }
-    __syncthreads();
+  // 6. the non-deflated entries grouped by support: child 1 only, both, child 2 only (counts
+  //    packed in one word: types 1, 3, 2 in 16 bits each, deflated entries in the top 16)
+  unsigned long long w = 0;
+  for (int s = s0; s < s1; s++) {
+    const int f = fl[s];
+    w += 1ull << ((f & 0x80) ? 48 : f == 1 ? 0 : f == 3 ? 16 : 32);
   }
-  // 6. group the non-deflated entries by support: child 1 only, both, child 2 only
-  if (tid == 0) {
-    int k1 = 0, k2 = 0, k3 = 0;
-    for (int t = 0; t < K; t++) {
-      const int f = fl[lst[t]];
-      if (f == 1) k1++;
-      else if (f == 3) k2++;
-      else k3++;
-    }
-    int g1 = 0, g2 = k1, g3 = k1 + k2;
-    for (int t = 0; t < K; t++) {
-      const int s = lst[t];
-      const int f = fl[s];
-      const int g = (f == 1) ? g1++ : (f == 3) ? g2++ : g3++;
+  w = block_scan(w, sred, total);
+  const int k1 = (int)(total & 0xffff), k2 = (int)(total >> 16 & 0xffff), k3 = (int)(total >> 32 & 0xffff);
+  const int K = k1 + k2 + k3;
+  int g1 = (int)(w & 0xffff), g2 = (int)(w >> 16 & 0xffff), g3 = (int)(w >> 32 & 0xffff), gd = (int)(w >> 48);
+  for (int s = s0; s < s1; s++) {
+    const int f = fl[s];
+    int g;
+    if (f & 0x80) {
+      g = K + gd++;
+      B.lam[a + g] = key[s];
+    } else {
+      const int t = g1 + g2 + g3;  // rank among the non-deflated poles
+      g = f == 1 ? g1++ : f == 3 ? k1 + g2++ : k1 + k2 + g3++;
       B.rank[a + g] = t;
       B.dgrp[a + g] = key[s];
       B.zgrp[a + g] = zs[s];
       B.dsort[a + t] = key[s];
-      // remember where the row goes: reuse rpos.x as the grouped slot of sorted position s
-      rpos[s].x = g;
     }
-    for (int q = 0; q < ndefl; q++) {
-      const int s = lst[N - 1 - q];
-      B.lam[a + K + q] = key[s];
-      rpos[s].x = K + q;
-    }
-    cnt[3] = k1;
-    cnt[4] = k2;
-    cnt[5] = k3;
+    B.slot[a + sidx[s]] = make_int2(g, f & 3);
+  }
+  if (tid == 0) {
     DcState st;
     st.K = K;
     st.k1 = k1;
     st.k2 = k2;
     st.k3 = k3;
     st.rho = rho;
+    st.nrot = s_nrot;
+    st.pad = 0;
     states[blockIdx.x] = st;
     // the two merge GEMMs: rows of child-1 columns from types 1+2, child-2 columns from 2+3
     gouts[nd.gout].M = K;
@@ -1297,31 +1354,103 @@ __global__ void __launch_bounds__(512) dc_prep_kernel(const LargeBlock* __restri
     gsegs[nd.gout + 1].A = B.evecs + (size_t)a * n + a + k1;
     gsegs[nd.gout + 1].B = B.W2 + (size_t)(a + k1) * n + m;
   }
-  __syncthreads();
-  // 7. copy the rows into grouped order in G (non-deflated first, then deflated)
-  const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-  for (int s = warp; s < N; s += nwarps) {
-    const size_t src = (size_t)(a + sidx[s]) * n, dst = (size_t)(a + rpos[s].x) * n;
-    for (int col = a + lane; col < b; col += 32) G[dst + col] = Z[src + col];
+}
+
+// ---------------------------------------------------------------- divide and conquer: row moves
+constexpr int kMoveCols = 32;  // columns of a row CTA's slab
+
+// The node's eigenvector rows with the deflation rotations applied, in grouped order
+// (non-deflated first, then deflated) in W2. One CTA owns a slab of 32 columns of all rows, so
+// the rotations of a slab need no other CTA. A child's rows are stored for its own columns
+// only; what the merge GEMMs read of a grouped row is its support, and only deflated rows are
+// written out to the full width.
+NRG_DEV void dc_move_rows(const LargeBlock& B, const DcNode& nd, const DcState& st, int slab) {
+  const int n = B.n, a = nd.a, b = nd.b, N = b - a, c0 = a + slab * kMoveCols;
+  if (c0 >= b) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int col = c0 + lane;
+  const bool act = col < b;
+  const int half = col < nd.m ? 1 : 2;
+  if (st.nrot > 0) {  // uniform over the CTA
+    if (warp == 0) {
+      const DcRot* rot = B.rot + a;
+      int lastj = -1;
+      double zl = 0.0;
+      constexpr int U = 8;  // rotations whose rows are loaded together: a row that an earlier
+                            // rotation changed is always the one before's j, held in zl
+      for (int r0 = 0; r0 < st.nrot; r0 += U) {
+        DcRot R[U];
+        double zp[U], zj[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if (r0 + u < st.nrot) R[u] = rot[r0 + u];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          zp[u] = zj[u] = 0.0;
+          if (r0 + u < st.nrot && act) {
+            const int before = u ? R[u - 1].j : lastj;
+            if (R[u].p != before && (R[u].sup & half)) zp[u] = B.H[(size_t)(a + R[u].p) * n + col];
+            if (R[u].sup >> 2 & half) zj[u] = B.H[(size_t)(a + R[u].j) * n + col];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          if (r0 + u < st.nrot) {
+            const double x = R[u].p == lastj ? zl : zp[u];
+            zl = R[u].s * x + R[u].c * zj[u];
+            lastj = R[u].j;
+            if (act && ((R[u].sup | R[u].sup >> 2) & half)) {
+              B.H[(size_t)(a + R[u].p) * n + col] = R[u].c * x - R[u].s * zj[u];
+              B.H[(size_t)(a + R[u].j) * n + col] = zl;
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  constexpr int R = 4;  // rows in flight per warp
+  for (int s = warp * R; s < N; s += nw * R) {
+    int2 sl[R];
+    double x[R];
+#pragma unroll
+    for (int u = 0; u < R; u++) {
+      sl[u] = s + u < N ? B.slot[a + s + u] : make_int2(0, 0);
+      x[u] = (s + u < N && act && (sl[u].y & half)) ? B.H[(size_t)(a + s + u) * n + col] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < R; u++)
+      if (s + u < N && act && ((sl[u].y & half) || sl[u].x >= st.K)) B.W2[(size_t)(a + sl[u].x) * n + col] = x[u];
   }
 }
 
 // ---------------------------------------------------------------- divide and conquer: secular equation
 // Root j of 1 + rho sum_i z_i^2 / (d_i - lambda) = 0 with poles d ascending. One warp per
-// root, lanes over i. On exit Dt[j][g] = d_g - lambda_j for every grouped entry g.
+// root, lanes over i. On exit Dt[j][g] = d_g - lambda_j for every grouped entry g. The CTAs
+// blockIdx.y >= ysec move the node's eigenvector rows beside it (dc_move_rows).
+// The iteration starts from the root of the two-pole model that the midpoint's values give, and
+// the last root, which lies right of every pole, takes the model's root on that side: the other
+// one is outside the bracket, and bisection in its place took 45-100 steps (the longest warp of
+// the launch) where now every root takes at most ten.
+// Measured on B200, 40 blocks up to order 480 (4 levels): 0.59 ms before, 0.14 ms now with the
+// row moves in it.
 __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __restrict__ blocks,
                                                          const DcNode* __restrict__ nodes,
-                                                         const DcState* __restrict__ states) {
+                                                         const DcState* __restrict__ states, int ysec) {
   const DcNode nd = nodes[blockIdx.x];
   const DcState st = states[blockIdx.x];
   const LargeBlock B = blocks[nd.blk];
+  if ((int)blockIdx.y >= ysec) {
+    dc_move_rows(B, nd, st, blockIdx.y - ysec);
+    return;
+  }
   const int K = st.K;
   if (K == 0) return;
   const int n = B.n, a = nd.a;
   const double rho = st.rho;
   const int lane = threadIdx.x & 31;
   const int wg = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int wstride = gridDim.y * (blockDim.x >> 5);
+  const int wstride = ysec * (blockDim.x >> 5);
   const double* ds = B.dsort + a;
   const double* dg = B.dgrp + a;
   const double* zg = B.zgrp + a;
@@ -1338,14 +1467,22 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __res
       }
       continue;
     }
-    if (j < K - 1) {
-      const double dj = ds[j], mid = 0.5 * (ds[j + 1] - dj);
-      double s = 0.0;
+    const bool last = j == K - 1;
+    if (!last) {
+      p1 = j;
+      p2 = j + 1;
+      const double dj = ds[j], gap = ds[j + 1] - dj, mid = 0.5 * gap;
+      double s = 0.0, z1 = 0.0, z2 = 0.0;  // the function at the midpoint; the two poles' residues
       for (int i = lane; i < K; i += 32) {
         const double z = zg[i];
+        const int r = rk[i];
+        if (r == p1) z1 = z * z;
+        if (r == p2) z2 = z * z;
         s += z * z / ((dg[i] - dj) - mid);
       }
       const double f = 1.0 + rho * warp_sum(s);
+      z1 = rho * warp_sum(z1);
+      z2 = rho * warp_sum(z2);
       if (f >= 0.0) {
         dorg = dj;
         lo = 0.0;
@@ -1355,8 +1492,13 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __res
         lo = -mid;
         hi = 0.0;
       }
-      p1 = j;
-      p2 = j + 1;
+      // the other poles' part is taken as constant: c + z1 / (d1 - x) + z2 / (d2 - x) = 0
+      const double c = f + (z1 - z2) / mid;
+      const double A1 = (f >= 0.0 ? c * gap : -c * gap) + z1 + z2;
+      const double A0 = f >= 0.0 ? z1 * gap : -z2 * gap;
+      const double disc = sqrt(fabs(A1 * A1 - 4.0 * c * A0));
+      tau = A1 > 0.0 ? 2.0 * A0 / (A1 + disc) : (A1 - disc) / (2.0 * c);
+      if (!(tau > lo && tau < hi)) tau = 0.5 * (lo + hi);
     } else {
       double s = 0.0;
       for (int i = lane; i < K; i += 32) s += zg[i] * zg[i];
@@ -1365,8 +1507,8 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __res
       hi = rho * warp_sum(s);
       p1 = K - 2;
       p2 = K - 1;
+      tau = 0.5 * hi;
     }
-    tau = 0.5 * (lo + hi);
     const double d1 = ds[p1] - dorg, d2 = ds[p2] - dorg;
     for (int it = 0; it < 100; it++) {
       double psi = 0.0, dpsi = 0.0, phi = 0.0, dphi = 0.0;
@@ -1389,7 +1531,8 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __res
       const double err = 8.0 * (fabs(psi) + fabs(phi)) + 2.0 + 3.0 * fabs(tau) * (dpsi + dphi);
       if (fabs(f) <= kEps * err) break;
       if (f < 0.0) lo = tau; else hi = tau;
-      // two-pole rational model through poles p1, p2 matching f and f'
+      // two-pole rational model through poles p1, p2 matching f and f'; its root between the
+      // poles, or for the last root the one right of both
       const double del1 = d1 - tau, del2 = d2 - tau;
       const double cc = f - del1 * dpsi - del2 * dphi;
       const double s1 = del1 * del1 * dpsi, s2 = del2 * del2 * dphi;
@@ -1400,7 +1543,8 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __res
         eta = A0 / A1;
       } else {
         const double disc = sqrt(fabs(A1 * A1 - 4.0 * cc * A0));
-        eta = (A1 <= 0.0) ? (A1 - disc) / (2.0 * cc) : 2.0 * A0 / (A1 + disc);
+        if (last) eta = (A1 >= 0.0) ? (A1 + disc) / (2.0 * cc) : 2.0 * A0 / (A1 - disc);
+        else eta = (A1 <= 0.0) ? (A1 - disc) / (2.0 * cc) : 2.0 * A0 / (A1 + disc);
       }
       double tn = tau + eta;
       if (!(tn > lo && tn < hi)) tn = 0.5 * (lo + hi);
@@ -1416,35 +1560,37 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __res
 // z-hat by the Gu-Eisenstat product formula (into dgrp, free after the secular solve), then
 // u_j(g) = zhat_g / (d_g - lambda_j), normalised, written over Dt in place (same grouped
 // column order). Both kernels spread a node over gridDim.y CTAs.
+// A CTA takes 32 columns g and splits the product over the roots between its eight warps (the
+// chain of K dependent multiplications and divisions was the whole time of small batches: 0.52 ms
+// of a step of 40 blocks up to order 480 with one thread per column, both kernels, 0.12 ms now).
 __global__ void __launch_bounds__(256) dc_zhat_kernel(const LargeBlock* __restrict__ blocks,
                                                       const DcNode* __restrict__ nodes,
                                                       const DcState* __restrict__ states) {
+  __shared__ double part[8][32];
   const DcNode nd = nodes[blockIdx.x];
   const DcState st = states[blockIdx.x];
+  const int K = st.K, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = blockIdx.y * 32 + lane;
+  if ((int)blockIdx.y * 32 >= K) return;  // uniform over the CTA
   const LargeBlock B = blocks[nd.blk];
-  const int K = st.K;
   const int n = B.n, a = nd.a;
   const double* ds = B.dsort + a;
-  const double* zg = B.zgrp + a;
-  const int* rk = B.rank + a;
   const double* Dt = B.evecs + (size_t)a * n + a;
-  const double rho = st.rho;
-  for (int g = blockIdx.y * blockDim.x + threadIdx.x; g < K; g += gridDim.y * blockDim.x) {
-    const int i = rk[g];
+  double p = 1.0;
+  if (g < K) {
+    const int i = B.rank[a + g];
     const double di = ds[i];
-    double p0 = -Dt[(size_t)(K - 1) * n + g] / rho, p1 = 1.0;
-    int j = 0;
-    for (; j + 1 < i; j += 2) {  // two independent product chains
-      p0 *= -Dt[(size_t)j * n + g] / (ds[j] - di);
-      p1 *= -Dt[(size_t)(j + 1) * n + g] / (ds[j + 1] - di);
-    }
-    for (; j < i; j++) p0 *= -Dt[(size_t)j * n + g] / (ds[j] - di);
-    for (; j + 1 < K - 1; j += 2) {
-      p0 *= -Dt[(size_t)j * n + g] / (ds[j + 1] - di);
-      p1 *= -Dt[(size_t)(j + 1) * n + g] / (ds[j + 2] - di);
-    }
-    for (; j < K - 1; j++) p0 *= -Dt[(size_t)j * n + g] / (ds[j + 1] - di);
-    B.dgrp[a + g] = copysign(sqrt(fabs(p0 * p1)), zg[g]);
+#pragma unroll 4
+    for (int j = warp; j < K - 1; j += 8) p *= -Dt[(size_t)j * n + g] / (ds[j < i ? j : j + 1] - di);
+    if (warp == 0) p *= -Dt[(size_t)(K - 1) * n + g] / st.rho;
+  }
+  part[warp][lane] = p;
+  __syncthreads();
+  if (warp == 0 && g < K) {
+    double q = 1.0;
+#pragma unroll
+    for (int v = 0; v < 8; v++) q *= part[v][lane];
+    B.dgrp[a + g] = copysign(sqrt(fabs(q)), B.zgrp[a + g]);
   }
 }
 
@@ -1536,33 +1682,84 @@ struct PanelRef {
   long long gt_off;
 };
 
-__global__ void __launch_bounds__(NBT) tfactor_kernel(const LargeBlock* __restrict__ blocks,
-                                                      const PanelRef* __restrict__ panels) {
+// The columns of T depend on one another, but T = [T1, -T1 G12 T2; 0, T2] for any split: the 16 x 16
+// diagonal blocks come from the recurrence, one warp each, and are merged 16 -> 32 -> 64 -> 128 by
+// two small DMMA products per merge, in place of G in shared memory. A reflector with tau = 0
+// has a zero row and column in T, which the products keep. Measured on B200: 40 blocks up to
+// order 480 (66 panels) 226 us with the 128-step recurrence in one CTA, 39 us now; 1400 blocks of
+// order 601-900 13.3 and 2.1 ms.
+constexpr int kTfThreads = 256;
+constexpr int kTfLd = NBT + 4, kTfLx = NBT / 2 + 4;
+
+// Tile of 8 x 8 of A B (A rows m0.., B columns n0.., inner index k0 <= k < k1, multiples of 4).
+NRG_DEV void tf_tile(const double* A, int lda, const double* Bm, int ldb, int m0, int n0, int k0, int k1, double& d0,
+                     double& d1) {
+  const int lane = threadIdx.x & 31, fr = lane >> 2, fc = lane & 3;
+  d0 = d1 = 0.0;
+  for (int k = k0; k < k1; k += 4) dmma884(d0, d1, A[(m0 + fr) * lda + k + fc], Bm[(k + fc) * ldb + n0 + fr]);
+}
+
+__global__ void __launch_bounds__(kTfThreads) tfactor_kernel(const LargeBlock* __restrict__ blocks,
+                                                             const PanelRef* __restrict__ panels) {
   extern __shared__ __align__(16) double tsm[];
   const PanelRef P = panels[blockIdx.x];
   const LargeBlock B = blocks[P.blk];
-  const int nb = P.nb, t = threadIdx.x, lt = NBT + 1;
-  double* Ts = tsm;           // NBT x (NBT+1)
-  double* w = tsm + NBT * lt;  // NBT
+  const int nb = P.nb, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double* Ts = tsm;                // NBT x kTfLd: G above the diagonal, then T
+  double* X = tsm + NBT * kTfLd;   // G12 T2 of the merges of one level
   const double* G = B.GT + P.gt_off;
   double* T = B.GT + P.gt_off + (size_t)nb * nb;
-  for (int r = 0; r < nb; r++) Ts[r * lt + t] = 0.0;
+  const int nbr = (nb + 15) / 16 * 16;
+  for (int r = warp; r < nbr; r += kTfThreads / 32)
+    for (int c = lane; c < nbr; c += 32) Ts[r * kTfLd + c] = (c > r && c < nb) ? G[(size_t)r * nb + c] : 0.0;
   __syncthreads();
-  for (int q = 0; q < nb; q++) {
-    const double tq = B.tau[P.k0 + q];
-    // w = -tau_q G[0:q, q]; T[0:q, q] = T[0:q, 0:q] w
-    if (t < q) w[t] = -tq * G[t * nb + q];
-    __syncthreads();
-    if (t < q) {
+  if (16 * warp < nbr) {  // diagonal block of 16: lane t holds row t
+    const int o = 16 * warp;
+    double row[16];
+#pragma unroll
+    for (int q = 0; q < 16; q++) {
+      const double tq = (o + q < nb) ? B.tau[P.k0 + o + q] : 0.0;
       double s = 0.0;
-      for (int r = t; r < q; r++) s += Ts[t * lt + r] * w[r];
-      Ts[t * lt + q] = s;
+#pragma unroll
+      for (int r = 0; r < q; r++) {
+        const double w = -tq * Ts[(o + r) * kTfLd + o + q];
+        if (r >= lane) s += row[r] * w;
+      }
+      row[q] = lane == q ? tq : lane < q ? s : 0.0;
     }
-    if (t == q) Ts[q * lt + q] = tq;
+    __syncwarp();
+    if (lane < 16) {
+#pragma unroll
+      for (int q = 0; q < 16; q++) Ts[(o + lane) * kTfLd + o + q] = row[q];
+    }
+  }
+  __syncthreads();
+  const int fr = lane >> 2, fc = lane & 3;
+  for (int h = 16; h < nbr; h *= 2) {  // merge neighbours of order h (the last one may be shorter)
+    const int q8 = h / 8, per = q8 * q8, nm = (nbr + 2 * h - 1) / (2 * h);
+    for (int u = warp; u < nm * per; u += kTfThreads / 32) {
+      const int o = (u / per) * 2 * h, i = (u % per) / q8 * 8, j = (u % per) % q8 * 8;
+      if (o + h + j >= nbr) continue;
+      double d0, d1;
+      tf_tile(Ts + o * kTfLd + o + h, kTfLd, Ts + (o + h) * kTfLd + o + h, kTfLd, i, j, 0, j + 8, d0, d1);
+      double* x = X + ((u / per) * h + i + fr) * kTfLx + j + 2 * fc;
+      x[0] = d0;
+      x[1] = d1;
+    }
+    __syncthreads();
+    for (int u = warp; u < nm * per; u += kTfThreads / 32) {
+      const int o = (u / per) * 2 * h, i = (u % per) / q8 * 8, j = (u % per) % q8 * 8;
+      if (o + h + j >= nbr) continue;
+      double d0, d1;
+      tf_tile(Ts + o * kTfLd + o, kTfLd, X + (u / per) * h * kTfLx, kTfLx, i, j, i, h, d0, d1);
+      double* y = Ts + (o + i + fr) * kTfLd + o + h + j + 2 * fc;
+      y[0] = -d0;
+      y[1] = -d1;
+    }
     __syncthreads();
   }
-  if (t < nb)
-    for (int r = 0; r < nb; r++) T[r * nb + t] = Ts[r * lt + t];
+  for (int r = warp; r < nb; r += kTfThreads / 32)
+    for (int c = lane; c < nb; c += 32) T[(size_t)r * nb + c] = Ts[r * kTfLd + c];
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
@@ -1581,7 +1778,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 size_t large_block_doubles(int n, bool two_stage) {
   const size_t ldp = (size_t)(n + 31) / 32 * 32;
-  return (size_t)n * ldp + (size_t)n * n + 8 * (size_t)n + 2 * (size_t)NBT * n + 2 * (size_t)n + 64 * 13 +
+  return (size_t)n * ldp + (size_t)n * n + 8 * (size_t)n + 2 * (size_t)NBT * n + 7 * (size_t)n + 64 * 15 +
          (prep_layout(n).total > kPrepSmemMax ? (kPrepGlobalB * (size_t)n + 7) / 8 : 0) +
          (two_stage ? band_extra_doubles(n) + 4 * 64 : 0);
 }
@@ -1656,6 +1853,8 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
       L.perm = ip + nb_;
       L.pscr = prep_layout(nb_).total > kPrepSmemMax
                    ? reinterpret_cast<char*>(take((kPrepGlobalB * (size_t)nb_ + 7) / 8)) : nullptr;
+      L.slot = reinterpret_cast<int2*>(take(nb_));
+      L.rot = reinterpret_cast<DcRot*>(take(4 * (size_t)nb_));
       L.info = info_dev + b;
       L.n = nb_;
       if ((int)(t - pos) < nts) {
@@ -2093,21 +2292,21 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
       NRG_CK(cudaFuncSetAttribute(dc_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ps));
       {
         PhaseScope sc(c, kPhDcPrep, s);
-        dc_prep_kernel<<<nn, 512, ps, s>>>(dblk, dn, dst, go, gs, ps);
+        dc_prep_kernel<<<nn, maxN <= 128 ? 128 : maxN <= 512 ? 256 : 512, ps, s>>>(dblk, dn, dst, go, gs, ps);
         NRG_CK(cudaGetLastError());
       }
-      // one warp per root (8 per CTA), at most 64 CTAs per node
-      const int ysplit = std::max(1, std::min(64, (maxN + 7) / 8));
+      // one warp per root (8 per CTA), at most 256 CTAs per node, and a CTA per slab of the rows
+      const int ysec = std::max(1, std::min(256, (maxN + 7) / 8)), ymove = (maxN + kMoveCols - 1) / kMoveCols;
       {
         PhaseScope sc(c, kPhDcSecular, s);
-        dc_secular_kernel<<<dim3(nn, ysplit), 256, 0, s>>>(dblk, dn, dst);
+        dc_secular_kernel<<<dim3(nn, ysec + ymove), 256, 0, s>>>(dblk, dn, dst, ysec);
         NRG_CK(cudaGetLastError());
       }
       {
         PhaseScope sc(c, kPhDcVectors, s, 2);
-        dc_zhat_kernel<<<dim3(nn, std::max(1, (maxN + 255) / 256)), 256, 0, s>>>(dblk, dn, dst);
+        dc_zhat_kernel<<<dim3(nn, (maxN + 31) / 32), 256, 0, s>>>(dblk, dn, dst);
         NRG_CK(cudaGetLastError());
-        dc_vectors_kernel<<<dim3(nn, ysplit), 256, 0, s>>>(dblk, dn, dst);
+        dc_vectors_kernel<<<dim3(nn, ysec), 256, 0, s>>>(dblk, dn, dst);
         NRG_CK(cudaGetLastError());
       }
       rc = launch_staged_gemm(c, lvl_gemm[h], s, kPhDcGemm);
@@ -2135,9 +2334,9 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
     if (rc) return rc;
     if (!panels.empty()) {
       PhaseScope sc(c, kPhBtTfactor, s);
-      const size_t ts = sizeof(double) * ((size_t)NBT * (NBT + 1) + NBT);
+      const size_t ts = sizeof(double) * ((size_t)NBT * kTfLd + (size_t)(NBT / 2) * kTfLx);
       NRG_CK(cudaFuncSetAttribute(tfactor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ts));
-      tfactor_kernel<<<(int)panels.size(), NBT, ts, s>>>(dblk, reinterpret_cast<const PanelRef*>(dbase + pan_off));
+      tfactor_kernel<<<(int)panels.size(), kTfThreads, ts, s>>>(dblk, reinterpret_cast<const PanelRef*>(dbase + pan_off));
       NRG_CK(cudaGetLastError());
     }
     rc = launch_staged_gemm(c, vt_g, s, kPhBtGemm);
