@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <numeric>
 #include <string>
@@ -312,9 +313,11 @@ int nrg_destroy(nrg_ctx* c) {
   if (c->fork_ev) cudaEventDestroy(c->fork_ev);
   if (c->join_ev) cudaEventDestroy(c->join_ev);
   if (c->side) cudaStreamDestroy(c->side);
-  if (c->fork2_ev) cudaEventDestroy(c->fork2_ev);
-  if (c->join2_ev) cudaEventDestroy(c->join2_ev);
-  if (c->side2) cudaStreamDestroy(c->side2);
+  if (c->tri_fork) cudaEventDestroy(c->tri_fork);
+  for (int i = 0; i < nrg_ctx::kTriStreams; i++) {
+    if (c->tri_join[i]) cudaEventDestroy(c->tri_join[i]);
+    if (c->tri[i]) cudaStreamDestroy(c->tri[i]);
+  }
   if (c->fork3_ev) cudaEventDestroy(c->fork3_ev);
   if (c->join3_ev) cudaEventDestroy(c->join3_ev);
   if (c->side3) cudaStreamDestroy(c->side3);
@@ -361,48 +364,57 @@ int nrg_diag_batch(nrg_ctx* c, int nblk, const int* n, double* const* H, double*
     CK(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming));
   }
+  std::function<int()> solve_small;  // launches the small-block solver
   if (!small.empty()) {
-    // Largest first, so that the long CTAs start early.
-    std::stable_sort(small.begin(), small.end(), [n](int a, int b) { return n[a] > n[b]; });
-    std::vector<nrg::EigBlock> blk(small.size());
-    for (size_t t = 0; t < small.size(); t++) {
-      const int b = small[t];
-      nrg::EigBlock& e = blk[t];
-      std::memset(&e, 0, sizeof e);
-      e.H = H[b];
-      e.evals = evals[b];
-      e.evecs = evecs[b];
-      e.info = c->info_dev + b;
-      e.n = n[b];
-    }
-    std::vector<char> img;
-    const size_t off = push(img, blk);
-    cudaStream_t ss = s;
-    char* base;
-    if (fork) {
-      CK(cudaEventRecord(c->fork_ev, s));
-      CK(cudaStreamWaitEvent(c->side, c->fork_ev, 0));
-      ss = c->side;
-      rc = nrg::stage_desc_side(c, img);
-      base = static_cast<char*>(c->desc_side);
-    } else {
-      rc = stage_desc(c, img, s);
-      base = static_cast<char*>(c->desc);
-    }
-    if (rc) return rc;
-    {
-      nrg::PhaseScope ps(c, nrg::kPhEigSmall, ss);
-      CK(nrg::eig_small_launch(reinterpret_cast<const nrg::EigBlock*>(base + off), (int)small.size(),
-                               n[small[0]], ss));
-    }
-    if (fork) CK(cudaEventRecord(c->join_ev, ss));
+    solve_small = [&]() -> int {
+      // Largest first, so that the long CTAs start early.
+      std::stable_sort(small.begin(), small.end(), [n](int a, int b) { return n[a] > n[b]; });
+      std::vector<nrg::EigBlock> blk(small.size());
+      for (size_t t = 0; t < small.size(); t++) {
+        const int b = small[t];
+        nrg::EigBlock& e = blk[t];
+        std::memset(&e, 0, sizeof e);
+        e.H = H[b];
+        e.evals = evals[b];
+        e.evecs = evecs[b];
+        e.info = c->info_dev + b;
+        e.n = n[b];
+      }
+      std::vector<char> img;
+      const size_t off = push(img, blk);
+      cudaStream_t ss = s;
+      char* base;
+      int r;
+      if (fork) {
+        ss = c->side;
+        r = nrg::stage_desc_side(c, img);
+        base = static_cast<char*>(c->desc_side);
+      } else {
+        r = stage_desc(c, img, s);
+        base = static_cast<char*>(c->desc);
+      }
+      if (r) return r;
+      {
+        nrg::PhaseScope ps(c, nrg::kPhEigSmall, ss);
+        CK(nrg::eig_small_launch(reinterpret_cast<const nrg::EigBlock*>(base + off), (int)small.size(),
+                                 n[small[0]], ss));
+      }
+      if (fork) CK(cudaEventRecord(c->join_ev, ss));
+      return NRG_OK;
+    };
   }
-  if (!large.empty()) {
-    rc = nrg::eig_large_run(c, large, n, H, evals, evecs, c->info_dev, s);
-    if (fork) {
-      const cudaError_t e = cudaStreamWaitEvent(s, c->join_ev, 0);  // join even on failure
-      if (!rc && e != cudaSuccess) rc = fail(NRG_ERR_CUDA, "join of the side stream: %s", cudaGetErrorString(e));
-    }
+  if (fork) {
+    CK(cudaEventRecord(c->fork_ev, s));
+    CK(cudaStreamWaitEvent(c->side, c->fork_ev, 0));
+    // eig_large_run calls it once its first reductions are launched: the clusters of the large
+    // blocks need whole GPCs free, the small blocks fit anywhere
+    CK(cudaEventRecord(c->join_ev, c->side));  // in case of an error before that
+    rc = nrg::eig_large_run(c, large, n, H, evals, evecs, c->info_dev, s, solve_small);
+    const cudaError_t e = cudaStreamWaitEvent(s, c->join_ev, 0);  // join even on failure
+    if (!rc && e != cudaSuccess) rc = fail(NRG_ERR_CUDA, "join of the side stream: %s", cudaGetErrorString(e));
+    if (rc) return rc;
+  } else {
+    rc = large.empty() ? solve_small() : nrg::eig_large_run(c, large, n, H, evals, evecs, c->info_dev, s, nullptr);
     if (rc) return rc;
   }
   CK(cudaMemcpyAsync(info, c->info_dev, sizeof(int) * (size_t)nblk, cudaMemcpyDeviceToHost, s));

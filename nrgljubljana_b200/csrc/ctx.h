@@ -42,10 +42,11 @@ struct nrg_ctx {
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   void* desc_side = nullptr;  // descriptor staging of the side stream
   size_t desc_side_size = 0;
-  // third stream: the one-CTA tridiagonalisation of mid-size blocks beside the cluster and
-  // bulk-copy reductions of larger blocks
-  cudaStream_t side2 = nullptr;
-  cudaEvent_t fork2_ev = nullptr, join2_ev = nullptr;
+  // streams of the shared-memory reductions (one per cluster size) beside one another and
+  // beside the streaming reduction of larger blocks
+  static constexpr int kTriStreams = 4;
+  cudaStream_t tri[kTriStreams] = {};
+  cudaEvent_t tri_fork = nullptr, tri_join[kTriStreams] = {};
   // fourth stream: the two-stage reduction of the largest blocks beside the one-stage ones
   cudaStream_t side3 = nullptr;
   cudaEvent_t fork3_ev = nullptr, join3_ev = nullptr;

@@ -911,159 +911,318 @@ __global__ void __launch_bounds__(kMidThreads) tridiag_smem_kernel(const LargeBl
   if (__syncthreads_or(bad) && tid == 0) atomicMin(B.info, -2);
 }
 
-// ---------------------------------------------------------------- cluster tridiagonalisation
-// Blocks with mid_max_n < n <= cluster_max_n (nrg_tuning): the packed lower triangle is spread over the
-// shared memory of a thread-block cluster of C CTAs (column j lives in CTA j mod C) and the
-// unblocked Householder reduction runs there; the CTAs read each other's shared memory
-// (distributed shared memory, plain loads, no bulk copies). Two cluster barriers per column:
-//   A  column k is final in its owner, and every CTA has finished reading the partial
-//      products of the previous column;
-//      every CTA reads column k from its owner and builds the same reflector v itself; each
-//      CTA forms its share of A v: per row, the part left of the diagonal from its own
-//      columns; per owned column (one warp), the part from the diagonal down;
-//   B  every CTA sums the shares of all CTAs for every row in a fixed order (so all CTAs
-//      hold the same w) and updates its own columns.
-// Output as tridiag_kernel.
-constexpr int kClThreads = 512;
+// ---------------------------------------------------------------- tridiagonalisation in shared memory
+// Blocks with small_max_n < n <= cluster_max_n (nrg_tuning): the full symmetric matrix is spread
+// by columns over the shared memory of a cluster of C CTAs (column j lives in CTA j mod C; C = 1
+// for the smallest), and the unblocked Householder reduction runs there. It is bound by the
+// chain of n columns, so a column costs one exchange between the CTAs:
+//   each CTA holds the previous reflector v, its w and the whole column k, and builds the new
+//   reflector itself (the same arithmetic in every CTA, so all agree to the last bit);
+//   it applies the previous rank-2 update to its columns and in the same pass forms their
+//   products with the new reflector -- with both triangles stored a column's product is complete
+//   in its CTA, so no partial sums cross the cluster, at 1.5 times the arithmetic of one triangle;
+//   for each of its columns it sends the product and the element of row k+1 (the next column,
+//   by symmetry) to every CTA by st.async, and waits on its own mbarrier for n-k-1 such pairs.
+// Pair buffers alternate between consecutive columns: a CTA can send pairs of column k+2 only
+// after it received all of column k+1's, which each other CTA sends after reading column k's.
+// The reflector is kept unscaled (u = v / scale, so that the product does not wait for the
+// scaling). The rows of a column are summed in the same order whatever C is.
+// Measured on B200 (one block, us per column): n = 456 in 16 CTAs 2.4 (5.4 with two cluster barriers
+// per column over one triangle), n = 300 1.9 in 16 and 2.3 in 8, n = 224 1.6 in 16, 1.9 in 8, 2.5 in
+// 4, 3.7 in 2, n = 128 1.5 in 16, 1.8 in 4, 3.1 in 1; 256 threads are 8% faster than 512.
+// Output as tridiag_kernel: d, e, tau, and v_k in row k of W1 (unit at k+1, zeros from the start
+// of its back-transform panel up to k).
+constexpr int kDsmThreads = 256;
+constexpr int kDsmWarps = kDsmThreads / 32;
+constexpr int kDsmMaxN = 640;                        // the largest cluster_max_n; what shared memory holds ends at 607
+constexpr int kDsmRows = (kDsmMaxN + kDsmThreads - 1) / kDsmThreads;  // rows of the vectors per thread
+constexpr int kRowSplit = 4, kColSplit = kDsmWarps / kRowSplit;
 
-// Offset of owned column t (global column j = r + t*C) in the local storage of CTA r.
-__host__ __device__ inline long long cl_loff(int t, int r, int C, int n) {
-  return (long long)t * (n - r) - (long long)C * t * (t - 1) / 2;
+__host__ __device__ inline int dsm_cols(int n, int C) { return (n + C - 1) / C; }
+
+// Doubles of shared memory of one CTA of a C-cluster for a block of order n: pairs (2 buffers), v,
+// w, u, partial products, row k+1, reduction scratch, columns.
+__host__ __device__ inline size_t dsm_smem_doubles(int n, int C) {
+  const size_t T = dsm_cols(n, C), Tp = (T + 7) / 8 * 8;
+  return 4 * (size_t)n + 3 * (size_t)n + (kRowSplit + 1) * Tp + 64 + T * n;
 }
 
-// Doubles of shared memory a CTA of a C-cluster needs for a block of order n.
-__host__ __device__ inline long long cl_smem_doubles(int n, int C) {
-  const int T0 = (n + C - 1) / C;  // columns of CTA 0, the largest share
-  return ((cl_loff(T0, 0, C, n) + 1) & ~1LL) + 4LL * n + 64;
+inline bool dsm_fits(int n, int C) {
+  return n <= kDsmMaxN && sizeof(double) * dsm_smem_doubles(n, C) + 512 <= 232448;
 }
 
-__global__ void __launch_bounds__(kClThreads) tridiag_cluster_kernel(const LargeBlock* __restrict__ blocks,
-                                                                     int lmax) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cl = cg::this_cluster();
-  const int C = (int)cl.num_blocks(), r = (int)cl.block_rank();
-  const LargeBlock B = blocks[blockIdx.x / C];
-  extern __shared__ __align__(16) double sm[];
-  const int n = B.n, ld = B.ldp, tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-  double* Pl = sm;          // owned columns, packed
-  double* v = Pl + lmax;    // n
-  double* w = v + n;        // n
-  double* yp = w + n;       // n: row part of this CTA's share of A v
-  double* yc = yp + n;      // n: column part (entries of owned columns)
-  double* red = yc + n;     // 64 (two halves for block_sum_1b)
-  int phase = 0;
-  const int T = (n - r + C - 1) / C;
-  for (int t = warp; t < T; t += nwarps) {
-    const int j = r + t * C;
-    const double* src = B.H + (size_t)j * n;
-    double* dst = Pl + cl_loff(t, r, C, n) - j;
-    for (int i = j + lane; i < n; i += 32) dst[i] = src[i];
+NRG_DEV unsigned cluster_addr(unsigned smem_addr, unsigned rank) {
+  unsigned a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+  return a;
+}
+
+// Stores the pair (x, y) to shared memory of a CTA of the cluster and counts 16 bytes on that
+// CTA's mbarrier.
+NRG_DEV void st_async_pair(unsigned addr, double x, double y, unsigned bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(addr),
+               "l"(__double_as_longlong(x)), "l"(__double_as_longlong(y)), "r"(bar)
+               : "memory");
+}
+
+// mbar_wait with acquire at cluster scope (the data come from other CTAs).
+NRG_DEV bool mbar_wait_cluster(uint64_t* bar, unsigned parity, int bound = (1 << 22)) {
+  const unsigned a = smem_u32(bar);
+  for (int it = 0; it < bound; it++) {
+    unsigned done;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, "
+        "p;\n}\n"
+        : "=r"(done)
+        : "r"(a), "r"(parity)
+        : "memory");
+    if (done) return true;
   }
+  return false;
+}
+
+// Sum over the warp, in every lane, by two DMMAs with a matrix of ones: the first sums over the
+// lanes of equal l/4, the second over the eight groups. The chain is a third of the five
+// shuffle-and-add steps' (a dependent FP64 add alone takes some 30 cycles).
+NRG_DEV double warp_sum_mma(double x) {
+  double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;
+  dmma884(d0, d1, 1.0, x);
+  dmma884(e0, e1, 1.0, d0 + d1);
+  return e0;
+}
+
+// block_sum_1b with warp_sum_mma for both levels (at most 32 warps).
+NRG_DEV double block_sum_mma(double x, double* red, int& phase) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  x = warp_sum_mma(x);
+  double* b = red + 32 * (phase & 1);
+  phase++;
+  if (lane == 0) b[wid] = x;
+  __syncthreads();
+  return warp_sum_mma(lane < nw ? b[lane] : 0.0);
+}
+
+// slab_colsum8 by DMMAs: a matrix with a one in row c and its product with the lanes' x[c] put the
+// sums over the lanes of equal l/4 into row c; a last one sums each row.
+NRG_DEV double colsum8_mma(const double (&x)[8], int lane) {
+  double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0, e0 = 0.0, e1 = 0.0;
+#pragma unroll
+  for (int c = 0; c < 8; c += 2) {
+    dmma884(a0, a1, lane >> 2 == c ? 1.0 : 0.0, x[c]);
+    dmma884(b0, b1, lane >> 2 == c + 1 ? 1.0 : 0.0, x[c + 1]);
+  }
+  dmma884(e0, e1, (a0 + a1) + (b0 + b1), 1.0);
+  return e0;
+}
+
+template <int C>
+__global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const LargeBlock* __restrict__ blocks) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) double sm[];
+  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ double sc[4];  // tau and scale of a reflector, by the parity of the next column
+  const int r = blockIdx.x % C;  // rank in the cluster
+  const LargeBlock B = blocks[blockIdx.x / C];
+  const int n = B.n, ld = B.ldp, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int T = (n - r + C - 1) / C, Tp = (dsm_cols(n, C) + 7) / 8 * 8;  // owned columns
+  double2* buf = reinterpret_cast<double2*>(sm);  // 2 x n pairs (product, column element)
+  double* v = sm + 4 * (size_t)n;                 // previous reflector
+  double* w = v + n;                              // and its w
+  double* u = w + n;                              // new reflector, unscaled, before the shift of u[k+1]
+  double* part = u + n;                           // kRowSplit x Tp
+  double* rowk = part + kRowSplit * Tp;           // Tp: row k+1 of the owned columns
+  double* red = rowk + Tp;                        // 64
+  double* M = red + 64;                           // T columns of n
   double* A = B.W1;
-  for (int k = 0; k < n - 2; k++) {
-    cl.sync();  // A
-    const int o = k % C;
-    // column k from its owner: colr[i] = A(i, k)
-    const double* colr = cl.map_shared_rank(Pl + cl_loff(k / C, o, C, n) - k, o);
-    double ps = 0.0;
-    for (int i = k + 2 + tid; i < n; i += nt) {
-      const double x = colr[i];
-      ps = fma(x, x, ps);
-    }
-    const double sigma = block_sum_1b(ps, red, phase);
-    const double alpha = colr[k + 1];
-    double tau = 0.0, beta = alpha, scale = 1.0;
-    if (sigma > 0.0) {
-      beta = -copysign(sqrt(alpha * alpha + sigma), alpha);
-      tau = (beta - alpha) / beta;
-      scale = 1.0 / (alpha - beta);
-    }
-    for (int i = k + 1 + tid; i < n; i += nt) {
-      const double vi = (i == k + 1) ? 1.0 : colr[i] * scale;
-      v[i] = vi;
-      if (r == o) A[(size_t)k * ld + i] = vi;
-    }
-    if (r == o) {
-      const int kb0 = (k / NBT) * NBT;
-      for (int i = kb0 + 1 + tid; i <= k; i += nt) A[(size_t)k * ld + i] = 0.0;
-      if (tid == 0) {
-        B.d[k] = colr[k];
-        B.e[k] = beta;
-        B.tau[k] = tau;
-      }
-    }
-    __syncthreads();
-    if (tau == 0.0) continue;  // the same in every CTA
-    // this CTA's share of A v over rows/columns k+1..n-1
-    const int t0 = (k + 1 - r > 0) ? (k + 1 - r + C - 1) / C : 0;  // first owned column >= k+1
-    for (int i = k + 1 + tid; i < n; i += nt) {
-      double s = 0.0;
-      long long addr = cl_loff(t0, r, C, n) - (r + t0 * C) + i;  // A(i, c) for c = r + t0*C
-      for (int t = t0, c = r + t0 * C; c < i; t++, c += C) {
-        s = fma(Pl[addr], v[c], s);
-        addr += (n - r - (long long)t * C) - C;
-      }
-      yp[i] = s;
-    }
-    for (int t = t0 + warp; t < T; t += nwarps) {
-      const int j = r + t * C;
-      const double* col = Pl + cl_loff(t, r, C, n) - j;
-      double dot = 0.0;
-      for (int i = j + lane; i < n; i += 32) dot = fma(col[i], v[i], dot);
-      dot = warp_sum(dot);
-      if (lane == 0) yc[j] = dot;
-    }
-    cl.sync();  // B
-    double pd = 0.0;
-    for (int i = k + 1 + tid; i < n; i += nt) {
-      double y = 0.0;
-      for (int q = 0; q < C; q++) y += cl.map_shared_rank(yp, q)[i];
-      y += cl.map_shared_rank(yc, i % C)[i];
-      const double wi = tau * y;
-      w[i] = wi;
-      pd = fma(wi, v[i], pd);
-    }
-    const double Kc = 0.5 * tau * block_sum_1b(pd, red, phase);  // its barrier also publishes w
-    // rank-2 update of the owned trailing columns with w' = w - Kc v
-    {
-      int t = t0, off = tid;
-      while (t < T && off >= n - (r + t * C)) {
-        off -= n - (r + t * C);
-        t++;
-      }
-      long long p = cl_loff(t0, r, C, n) + tid;
-      while (t < T) {
-        const int j = r + t * C, i = j + off;
-        const double wj = w[j] - Kc * v[j], wi = w[i] - Kc * v[i];
-        Pl[p] -= v[i] * wj + wi * v[j];
-        p += nt;
-        off += nt;
-        while (t < T && off >= n - (r + t * C)) {
-          off -= n - (r + t * C);
-          t++;
-        }
-      }
-    }
+  int phase = 0;
+  bool dead = false;  // a wait ran out: the block is flagged and nothing is waited for any more
+
+  for (int t = warp; t < T; t += kDsmWarps) {  // column j: row j of H from the diagonal, column j above it
+    const int j = r + t * C;
+    double* dst = M + (size_t)t * n;
+    for (int i = j + lane; i < n; i += 32) dst[i] = B.H[(size_t)j * n + i];
+  }
+  for (int i = warp; i < n; i += kDsmWarps)
+    for (int t = lane; t < T; t += 32)
+      if (r + t * C > i) M[(size_t)t * n + i] = B.H[(size_t)i * n + r + t * C];
+  for (int i = tid; i < n; i += kDsmThreads) {
+    buf[i] = make_double2(0.0, B.H[i]);
+    v[i] = w[i] = 0.0;
   }
   if (tid == 0) {
-    if (r == (n - 2) % C) {
-      const double* col = Pl + cl_loff((n - 2) / C, r, C, n) - (n - 2);
-      B.d[n - 2] = col[n - 2];
-      B.e[n - 2] = col[n - 1];
-      B.tau[n - 2] = 0.0;
+    sc[0] = 0.0;
+    sc[1] = 1.0;
+  }
+  if constexpr (C > 1) {
+    if (tid == 0) {
+      mbar_init(bars, 1);
+      mbar_init(bars + 1, 1);
+      fence_mbar_init();
     }
-    if (r == (n - 1) % C) {
-      const double* col = Pl + cl_loff((n - 1) / C, r, C, n) - (n - 1);
-      B.d[n - 1] = col[n - 1];
-      B.e[n - 1] = 0.0;
-      B.tau[n - 1] = 0.0;
+    cg::this_cluster().sync();
+  } else {
+    __syncthreads();
+  }
+
+  double ur[kDsmRows] = {};             // u of this thread's rows (of the previous column)
+  double alpha = 0.0, beta = 0.0;       // previous reflector
+  for (int k = 0; k < n - 1; k++) {
+    const double2* pb = buf + (size_t)(k & 1) * n;
+    const double tau = sc[2 * (k & 1)], scale = sc[2 * (k & 1) + 1], f = tau * scale;
+    double vr[kDsmRows];
+#pragma unroll
+    for (int q = 0; q < kDsmRows; q++) {
+      const int i = tid + q * kDsmThreads;
+      vr[q] = 0.0;
+      if (k > 0 && i >= k && i < n) {
+        vr[q] = i == k ? 1.0 : scale * ur[q];
+        if (C == 1 || (i >> 5) % C == r) A[(size_t)(k - 1) * ld + i] = vr[q];
+      }
+    }
+    if (k > 0) {
+      if (r == k % C)
+        for (int i = ((k - 1) / NBT) * NBT + 1 + tid; i < k; i += kDsmThreads) A[(size_t)(k - 1) * ld + i] = 0.0;
+      if (tid == 0 && r == 0) {
+        B.e[k - 1] = beta;
+        B.tau[k - 1] = tau;
+      }
+    }
+    if constexpr (C > 1) {
+      if (k > 0 && !dead && !mbar_wait_cluster(bars + (k & 1), ((k - 1) >> 1) & 1)) {
+        dead = true;
+        if (tid == 0) atomicExch(B.info, -5);
+      }
+    }
+    // (1) previous reflector: w = f y - K v with f = tau scale
+    double y[kDsmRows], cc[kDsmRows], pd = 0.0;
+#pragma unroll
+    for (int q = 0; q < kDsmRows; q++) {
+      const int i = tid + q * kDsmThreads;
+      y[q] = cc[q] = 0.0;
+      if (i >= k && i < n) {
+        const double2 p = pb[i];
+        y[q] = f * p.x;
+        cc[q] = p.y;
+        pd = fma(y[q], vr[q], pd);
+      }
+    }
+    const double yk = f * pb[k].x;
+    const double Kc = 0.5 * tau * block_sum_mma(pd, red, phase);
+    // (2) column k after that update; reflector for rows k+1..n-1 (dlarfg convention)
+    const double wk = k > 0 ? yk - Kc : 0.0;
+    double ps = 0.0;
+#pragma unroll
+    for (int q = 0; q < kDsmRows; q++) {
+      const int i = tid + q * kDsmThreads;
+      if (i >= k && i < n) {
+        const double wi = y[q] - Kc * vr[q];
+        const double ai = k > 0 ? cc[q] - vr[q] * wk - wi : cc[q];
+        v[i] = vr[q];
+        w[i] = wi;
+        u[i] = ai;
+        ur[q] = ai;
+        if (i >= k + 2) ps = fma(ai, ai, ps);
+      }
+    }
+    const double sigma = block_sum_mma(ps, red, phase);  // its barrier also publishes v, w and u
+    alpha = u[k + 1];
+    if (tid == 0 && r == 0) B.d[k] = u[k];
+    if (k == n - 2) {
+      if (tid == 0 && r == 0) {
+        B.e[k] = alpha;
+        B.tau[k] = 0.0;
+      }
+      if (tid == 0 && r == (n - 1) % C) {
+        B.d[n - 1] = M[(size_t)((n - 1) / C) * n + n - 1] - 2.0 * v[n - 1] * w[n - 1];
+        B.e[n - 1] = 0.0;
+        B.tau[n - 1] = 0.0;
+      }
+      break;
+    }
+    beta = sigma > 0.0 ? -copysign(sqrt(alpha * alpha + sigma), alpha) : alpha;
+    const double u1 = alpha - beta;  // u[k+1]
+#pragma unroll
+    for (int q = 0; q < kDsmRows; q++)
+      if (tid + q * kDsmThreads == k + 1) ur[q] = u1;
+    // the two divisions of the reflector are needed for the next column only: the warp with the
+    // least work makes them beside the products
+    if (tid == kDsmThreads - 1) {
+      double tau1 = 0.0, scale1 = 1.0;
+      if (sigma > 0.0) {
+        tau1 = (beta - alpha) / beta;
+        scale1 = 1.0 / u1;
+      }
+      sc[2 * ((k + 1) & 1)] = tau1;
+      sc[2 * ((k + 1) & 1) + 1] = scale1;
+    }
+    // (3) previous update of the owned columns j > k and their products with u
+    const int t0 = (k + 1 - r > 0) ? (k + 1 - r + C - 1) / C : 0;
+    const int wr = warp % kRowSplit, wc = warp / kRowSplit;
+    const int s0 = (k + 1) >> 5, s1 = (n - 1) >> 5;
+    for (int tg = t0 + 8 * wc; tg < T; tg += 8 * kColSplit) {
+      const int nv = min(8, T - tg);
+      double vj[8], wj[8], cs[8];
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+        const int j = r + (tg + (c < nv ? c : 0)) * C;
+        vj[c] = v[j];
+        wj[c] = w[j];
+        cs[c] = 0.0;
+      }
+      // row chunks s with s mod kRowSplit = wr, whatever k and C are; lanes above row k+1 or below
+      // row n-1 and columns beyond the last read something finite and store nothing
+      for (int s = s0 + ((wr - s0) & (kRowSplit - 1)); s <= s1; s += kRowSplit) {
+        const int i = min(32 * s + lane, n - 1);
+        const bool act = i > k && 32 * s + lane < n;
+        const double vi = v[i], wi = w[i], ui = act ? (i == k + 1 ? u1 : u[i]) : 0.0;
+        double* col = M + (size_t)tg * n + i;
+        double x[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) x[c] = col[(size_t)(c < nv ? c : 0) * n];
+#pragma unroll
+        for (int c = 0; c < 8; c++) x[c] = fma(-vi, wj[c], x[c]);
+#pragma unroll
+        for (int c = 0; c < 8; c++) x[c] = fma(-wi, vj[c], x[c]);
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+          cs[c] = fma(x[c], ui, cs[c]);
+          if (act && c < nv) col[(size_t)c * n] = x[c];
+        }
+        if (act && i == k + 1) {
+#pragma unroll
+          for (int c = 0; c < 8; c++)
+            if (c < nv) rowk[tg + c] = x[c];
+        }
+      }
+      __syncwarp();
+      const double sum = colsum8_mma(cs, lane);
+      const int c = lane >> 2;
+      if ((lane & 3) == 0 && c < nv) part[wr * Tp + tg + c] = sum;
+    }
+    __syncthreads();
+    // (4) each owned column's product and element of row k+1 to every CTA
+    double2* nb = buf + (size_t)((k + 1) & 1) * n;
+    if constexpr (C > 1) {
+      uint64_t* bar = bars + ((k + 1) & 1);
+      if (tid == 0) mbar_expect_tx(bar, 16u * (unsigned)(n - k - 1));
+      const int items = (T - t0) * C;
+      for (int it = tid; it < items; it += kDsmThreads) {
+        const int t = t0 + it / C, dst = it % C;
+        static_assert(kRowSplit == 4, "pairwise sum of the row parts");
+        const double yj = (part[t] + part[Tp + t]) + (part[2 * Tp + t] + part[3 * Tp + t]);
+        st_async_pair(cluster_addr(smem_u32(nb + r + t * C), dst), yj, rowk[t], cluster_addr(smem_u32(bar), dst));
+      }
+    } else {
+      for (int t = t0 + tid; t < T; t += kDsmThreads)
+        nb[t] = make_double2((part[t] + part[Tp + t]) + (part[2 * Tp + t] + part[3 * Tp + t]), rowk[t]);
+      __syncthreads();
     }
   }
-  cl.sync();  // the last remote reads are done; d and e are complete
+  if constexpr (C > 1) cg::this_cluster().sync();  // d and e are complete; no CTA leaves while pairs are under way
+  else __syncthreads();
   if (r == 0) {
     int bad = 0;
-    for (int i = tid; i < n; i += nt) bad |= !(isfinite(B.d[i]) && isfinite(B.e[i]));
+    for (int i = tid; i < n; i += kDsmThreads) bad |= !(isfinite(B.d[i]) && isfinite(B.e[i]));
     if (__syncthreads_or(bad) && tid == 0) atomicMin(B.info, -2);
   }
 }
@@ -1783,10 +1942,117 @@ size_t large_block_doubles(int n, bool two_stage) {
          (two_stage ? band_extra_doubles(n) + 4 * 64 : 0);
 }
 
+// Largest order that a cluster of 16 holds.
+int dsm_max_order() {
+  static const int n = [] {
+    int k = kDsmMaxN;
+    while (!dsm_fits(k, 16)) k--;
+    return k;
+  }();
+  return n;
+}
+
+// Microseconds of a block's reduction in a C-cluster (B200, see tridiag_dsm_kernel).
+double dsm_us(int n, int C) { return n * (1.42 + 7.5e-5 * n * n / C); }
+
+// How the blocks [lo, hi) (sorted by falling order, the first within dsm_max_order) are reduced:
+// C[q] CTAs for block q, 0 for the one-CTA kernel over the packed triangle (tridiag_smem_kernel);
+// blocks before `first` go to the streaming reduction.
+struct DsmPlan {
+  int first;
+  std::vector<int> C;
+};
+
+DsmPlan dsm_plan(const LargeBlock* b, int lo, int hi, int mid_max_n, int nsm) {
+  DsmPlan p{lo, std::vector<int>(hi, 0)};
+  int sum = 0;
+  for (int q = lo; q < hi; q++) {
+    int C = 1;
+    while (!dsm_fits(b[q].n, C)) C *= 2;
+    p.C[q] = C;
+    sum += C;
+  }
+  if (sum <= nsm) {
+    // Few blocks: bound by the longest chain, so the block whose reduction takes longest gets
+    // twice the CTAs as long as the clusters fit the SMs at once.
+    for (;;) {
+      int best = -1;
+      double tb = 0.0;
+      for (int q = lo; q < hi; q++)
+        if (dsm_us(b[q].n, p.C[q]) > tb) tb = dsm_us(b[q].n, p.C[best = q]);
+      if (best < 0 || p.C[best] == 16 || sum + p.C[best] > nsm) return p;
+      sum += p.C[best];
+      p.C[best] *= 2;
+    }
+  }
+  // Many: bound by the SMs' time. Blocks that fit one CTA's packed triangle stay in one CTA (two
+  // would take 1.3 times the SM time of that kernel from order 160 on, and it half as much again
+  // as the full square below). Of the larger ones a C-cluster holds C SMs for dsm_us; the
+  // streaming reduction takes the chip's bandwidth for their bytes, but its largest block has one
+  // SM (15 GB/s, 4/3 n^3 bytes). Measured on B200, 300 blocks up to order 1024 (60 of them of order
+  // 225-600): the reductions 91 ms with all streamed, 55 with those in clusters (the 37 larger
+  // ones).
+  int mid = lo;
+  while (mid < hi && b[mid].n > mid_max_n) mid++;
+  double clu = 0.0, bytes = 0.0;
+  for (int q = lo; q < mid; q++) {
+    clu += p.C[q] * dsm_us(b[q].n, p.C[q]) / nsm;
+    bytes += 4.0 / 3.0 * b[q].n * (double)b[q].n * b[q].n;
+  }
+  if (mid > lo) {
+    const double n0 = b[lo].n, stream = std::max(bytes / 4.4e6, 4.0 / 3.0 * n0 * n0 * n0 / 1.5e4);
+    if (stream < clu + dsm_us(b[lo].n, p.C[lo])) p.first = mid;
+  }
+  for (int q = mid; q < hi; q++)
+    if (p.C[q] > 1) p.C[q] = 0;
+  return p;
+}
+
+cudaError_t reduce_in_smem_launch(const LargeBlock* d_blk, int maxn, int count, int C, cudaStream_t s) {
+  if (C == 0) {
+    const size_t smem = sizeof(double) * ((size_t)maxn * (maxn + 1) / 2 + 2 * (size_t)maxn + 64);
+    cudaError_t e = cudaFuncSetAttribute(tridiag_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    tridiag_smem_kernel<<<count, kMidThreads, smem, s>>>(d_blk);
+    return cudaGetLastError();
+  }
+  const void* fn = C == 16 ? (const void*)tridiag_dsm_kernel<16> : C == 8 ? (const void*)tridiag_dsm_kernel<8>
+                   : C == 4 ? (const void*)tridiag_dsm_kernel<4> : C == 2 ? (const void*)tridiag_dsm_kernel<2>
+                                                                          : (const void*)tridiag_dsm_kernel<1>;
+  const size_t smem = sizeof(double) * dsm_smem_doubles(maxn, C);
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess && C == 16) e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(count * C));
+  cfg.blockDim = dim3(kDsmThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)C;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  void* kargs[] = {(void*)&d_blk};
+  return cudaLaunchKernelExC(&cfg, fn, kargs);
+}
+
+int tri_streams(nrg_ctx* c) {
+  if (c->tri_fork) return NRG_OK;
+  for (int i = 0; i < nrg_ctx::kTriStreams; i++) {
+    if (!c->tri[i]) NRG_CK(cudaStreamCreateWithFlags(&c->tri[i], cudaStreamNonBlocking));
+    if (!c->tri_join[i]) NRG_CK(cudaEventCreateWithFlags(&c->tri_join[i], cudaEventDisableTiming));
+  }
+  NRG_CK(cudaEventCreateWithFlags(&c->tri_fork, cudaEventDisableTiming));
+  return NRG_OK;
+}
+
 }  // namespace
 
 int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, double* const* H, double* const* evals,
-                  double* const* evecs, int* info_dev, cudaStream_t s) {
+                  double* const* evecs, int* info_dev, cudaStream_t s, const std::function<int()>& beside) {
   std::vector<int> ord(which);
   std::stable_sort(ord.begin(), ord.end(), [n](int x, int y) { return n[x] > n[y]; });
   const int mid_max_n = c->tune.mid_max_n, cluster_max_n = c->tune.cluster_max_n;
@@ -2100,8 +2366,7 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
     }
 
     // ---- 1. tridiagonalisation: blocks beyond cluster_max_n (sorted first) stream through
-    //         TMA, blocks beyond mid_max_n are spread over the shared memory of a cluster,
-    //         the rest are reduced in the shared memory of one CTA
+    //         TMA, the rest are reduced in the shared memory of a cluster or one CTA
     {
       int nsm = 148;
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
@@ -2110,66 +2375,27 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
       const LargeBlock* d1 = dblk + nts;
       const int nb1 = nb - nts;
       int nbig = 0;
-      while (nbig < nb1 && b1[nbig].n > cluster_max_n) nbig++;
-      int nclu = nbig;
-      while (nclu < nb1 && b1[nclu].n > mid_max_n) nclu++;
-      // One cluster size for all cluster blocks (one launch): the smallest of 2, 4, 8 that
-      // fits the largest of them, raised while the cluster CTAs still fit the SMs once. The
-      // clusters serve latency: when they would not all fit the SMs at once (a batch of many
-      // blocks), the blocks go to the bulk-copy kernel, whose two CTAs per SM give more
-      // throughput.
-      int C = 0;
-      if (nclu > nbig) {
-        for (int q = 2; q <= 8 && !C; q *= 2)
-          if (sizeof(double) * cl_smem_doubles(b1[nbig].n, q) <= 232448) C = q;
-        if (C == 0) return fail(NRG_ERR_ARG, "internal: no cluster size for n=%d", b1[nbig].n);
-        if (C * (nclu - nbig) > nsm) {
-          nbig = nclu;  // throughput regime
-          C = 0;
-        } else {
-          while (C < 8 && 2 * C * (nclu - nbig) <= nsm) C *= 2;
+      while (nbig < nb1 && b1[nbig].n > std::min(cluster_max_n, dsm_max_order())) nbig++;
+      const DsmPlan dp = dsm_plan(b1, nbig, nb1, mid_max_n, nsm);
+      nbig = dp.first;
+      // Launches that can run side by side go to streams of their own: the streaming reduction of
+      // the largest blocks on s, each cluster size and the one-CTA kernel beside it, largest first
+      // (clusters need SMs of one GPC free at once).
+      struct Launch { int C, q0, q1; };  // C = 0: tridiag_smem_kernel
+      std::vector<Launch> ls;
+      for (int C = 16; C >= 0; C = C > 1 ? C / 2 : C - 1)
+        for (int q0 = nbig, q1; q0 < nb1; q0 = q1) {
+          for (q1 = q0 + 1; q1 < nb1 && dp.C[q1] == dp.C[q0]; q1++) {}
+          if (dp.C[q0] == C) ls.push_back({C, q0, q1});
         }
+      const bool fork = ls.size() + (nbig > 0) > 1;
+      if (fork) {
+        rc = tri_streams(c);
+        if (rc) return rc;
+        NRG_CK(cudaEventRecord(c->tri_fork, s));
       }
-      const bool fork = nb1 > nclu && (nbig > 0 || nclu > nbig);
-      if (fork && !c->side2) {
-        NRG_CK(cudaStreamCreateWithFlags(&c->side2, cudaStreamNonBlocking));
-        NRG_CK(cudaEventCreateWithFlags(&c->fork2_ev, cudaEventDisableTiming));
-        NRG_CK(cudaEventCreateWithFlags(&c->join2_ev, cudaEventDisableTiming));
-      }
-      PhaseScope ps(c, kPhTridiag, s, (nbig ? 2 : 0) + (nclu > nbig ? 1 : 0) + (nb1 > nclu ? 1 : 0));
-      if (nb1 > nclu) {  // one CTA per block, on the third stream when other launches run beside it
-        cudaStream_t ss = s;
-        if (fork) {
-          NRG_CK(cudaEventRecord(c->fork2_ev, s));
-          NRG_CK(cudaStreamWaitEvent(c->side2, c->fork2_ev, 0));
-          ss = c->side2;
-        }
-        const int mn = b1[nclu].n;
-        const size_t smem = sizeof(double) * ((size_t)mn * (mn + 1) / 2 + 2 * (size_t)mn + 64);
-        NRG_CK(cudaFuncSetAttribute(tridiag_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        tridiag_smem_kernel<<<nb1 - nclu, kMidThreads, smem, ss>>>(d1 + nclu);
-        NRG_CK(cudaGetLastError());
-        if (fork) NRG_CK(cudaEventRecord(c->join2_ev, ss));
-      }
-      if (nclu > nbig) {
-        const long long ld0 = cl_smem_doubles(b1[nbig].n, C);  // the largest block sets the layout
-        const int lmax = (int)(ld0 - (4LL * b1[nbig].n + 64));
-        const size_t smem = sizeof(double) * (size_t)ld0;
-        NRG_CK(cudaFuncSetAttribute(tridiag_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)((nclu - nbig) * C));
-        cfg.blockDim = dim3(kClThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = s;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)C;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        NRG_CK(cudaLaunchKernelEx(&cfg, tridiag_cluster_kernel, d1 + nbig, lmax));
-      }
+      PhaseScope ps(c, kPhTridiag, s, (nbig ? 2 : 0) + (int)ls.size());
+      unsigned used = 0;  // side streams with a launch
       if (nbig) {
         auto tri_bytes = [&](int st) {
           return 1024 + sizeof(double) * ((size_t)kTriWarps * st * kSlabD + 2 * (size_t)b1[0].n +
@@ -2266,7 +2492,25 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
           NRG_CK(cudaGetLastError());
         }
       }
-      if (fork) NRG_CK(cudaStreamWaitEvent(s, c->join2_ev, 0));
+      for (size_t q = 0; q < ls.size(); q++) {
+        cudaStream_t ss = s;
+        const size_t side = q + (nbig > 0);  // 0: stream s
+        if (side > 0) {
+          const int i = (int)(side - 1) % nrg_ctx::kTriStreams;
+          ss = c->tri[i];
+          if (!(used >> i & 1)) NRG_CK(cudaStreamWaitEvent(ss, c->tri_fork, 0));
+          used |= 1u << i;
+        }
+        NRG_CK(reduce_in_smem_launch(d1 + ls[q].q0, b1[ls[q].q0].n, ls[q].q1 - ls[q].q0, ls[q].C, ss));
+      }
+      for (int i = 0; i < nrg_ctx::kTriStreams; i++)
+        if (used >> i & 1) NRG_CK(cudaEventRecord(c->tri_join[i], c->tri[i]));
+      if (beside && pos == 0) {  // the small-block solver takes what SMs are left
+        rc = beside();
+        if (rc) return rc;
+      }
+      for (int i = 0; i < nrg_ctx::kTriStreams; i++)
+        if (used >> i & 1) NRG_CK(cudaStreamWaitEvent(s, c->tri_join[i], 0));
     }
     if (fork3) NRG_CK(cudaStreamWaitEvent(s, c->join3_ev, 0));  // the two-stage blocks are tridiagonal
     // ---- 2. divide and conquer

@@ -1,0 +1,50 @@
+"""The shared-memory reductions at the orders where a cluster of 1, 2, 4, 8 or 16 CTAs is just full or
+one too small, in batches that choose the largest clusters (few blocks) and the smallest (many),
+against the oracle's dsyev; and the same block to the last bit whatever cluster it gets."""
+import numpy as np
+import pytest
+
+from eigcheck import check_eig
+
+pytestmark = pytest.mark.gpu
+
+EDGES = [65, 164, 165, 230, 231, 323, 324, 448, 449, 600]
+
+
+@pytest.fixture(scope="module")
+def nb():
+    import nrgljubljana_b200 as m
+    m.context()
+    return m
+
+
+def blocks_of(sizes, seed):
+    rng = np.random.default_rng(seed)
+    out = []
+    for k, n in enumerate(sizes):
+        a = rng.standard_normal((n, n))
+        h = np.triu(a + a.T)
+        if k % 3 == 1:  # a column that is already reduced (tau = 0), and a decoupled half
+            h[0, 2:] = 0.0
+            h[: n // 2, n // 2:] = 0.0
+        out.append(h)
+    return out
+
+
+@pytest.mark.parametrize("copies", [1, 4])
+def test_cluster_edges(nb, oracle, copies):
+    sizes = EDGES * copies  # one of each: the clusters grow; four: more CTAs than SMs
+    blocks = blocks_of(sizes, 31 + copies)
+    got = nb.diagonalisations(blocks)
+    for h, g in list(zip(blocks, got))[: len(EDGES)]:
+        w, v = oracle.diagonalise(h)
+        check_eig(h, g.val, g.vec, w, v, oracle)
+
+
+@pytest.mark.parametrize("n", [100, 301, 448])
+def test_same_result_in_any_cluster(nb, n):
+    blocks = blocks_of([n] * 12, 7 * n)
+    together = nb.diagonalisations(blocks)
+    for k in (0, 1, 11):
+        alone = nb.diagonalisations([blocks[k]])[0]
+        assert np.array_equal(alone.val, together[k].val) and np.array_equal(alone.vec, together[k].vec)
