@@ -9,7 +9,7 @@
 //                         (panel width NB); the symmetric matrix-vector product streams
 //                         the lower triangle from HBM once per column, the panel update
 //                         is a rank-2NB update of the trailing lower triangle.
-//   2. divide and conquer on T: leaves (<= kLeaf) by implicit QL in shared memory, merges
+//   2. divide and conquer on T: leaves (<= kLeaf) by one in shared memory, merges
 //      by rank-one tearing (Cuppen), deflation (small z and close poles with Givens
 //      rotations), secular-equation roots with a two-pole rational model safeguarded by
 //      bisection, Gu-Eisenstat recomputation of z for orthogonal vectors, and the merge
@@ -37,7 +37,7 @@ namespace {
 constexpr int kTriThreads = 128;
 constexpr int NB = 16;     // tridiagonalisation panel width
 constexpr int NBT = 128;   // back-transform panel width
-constexpr int kLeaf = 32;  // divide-and-conquer leaves have at most this order
+constexpr int kLeaf = 64;  // divide-and-conquer leaves have at most this order
 constexpr int kMaxLargeN = 10240;  // the tridiagonalisation's shared memory (68 KB + 16 n bytes) fits to here
 // Merge nodes whose prep arrays exceed this many bytes keep them in global scratch (kPrepGlobalB
 // bytes per row of the block) instead of shared memory.
@@ -981,16 +981,6 @@ NRG_DEV bool mbar_wait_cluster(uint64_t* bar, unsigned parity, int bound = (1 <<
   return false;
 }
 
-// Sum over the warp, in every lane, by two DMMAs with a matrix of ones: the first sums over the
-// lanes of equal l/4, the second over the eight groups. The chain is a third of the five
-// shuffle-and-add steps' (a dependent FP64 add alone takes some 30 cycles).
-NRG_DEV double warp_sum_mma(double x) {
-  double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;
-  dmma884(d0, d1, 1.0, x);
-  dmma884(e0, e1, 1.0, d0 + d1);
-  return e0;
-}
-
 // block_sum_1b with warp_sum_mma for both levels (at most 32 warps).
 NRG_DEV double block_sum_mma(double x, double* red, int& phase) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -1228,32 +1218,44 @@ __global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const Large
 }
 
 // ---------------------------------------------------------------- divide and conquer: leaves
-__global__ void __launch_bounds__(128) dc_leaf_kernel(const LargeBlock* __restrict__ blocks,
-                                                      const DcLeaf* __restrict__ leaves) {
-  __shared__ double Z[kLeaf * (kLeaf + 1)];
-  __shared__ double d[kLeaf], e[kLeaf], C[2 * kLeaf], S[2 * kLeaf];
-  __shared__ int ctl[8];
+// One CTA per leaf of order <= 64: the leaf is itself solved by divide and conquer in shared memory
+// (smem_dc). Measured on B200: leaves of order 32 by implicit QL took 0.40 ms of a step of 40 blocks up to
+// order 480, these 0.10 ms, with a merge level less to follow (0.1 ms).
+constexpr int kLeafLd = kLeaf + 1;
+
+__global__ void __launch_bounds__(kCtaEigThreads) dc_leaf_kernel(const LargeBlock* __restrict__ blocks,
+                                                                 const DcLeaf* __restrict__ leaves) {
+  extern __shared__ __align__(16) double sm[];
+  __shared__ int ctl[12];
   const DcLeaf L = leaves[blockIdx.x];
   const LargeBlock B = blocks[L.blk];
-  const int n = B.n, a0 = L.a0, nl = L.a1 - L.a0, ld = kLeaf + 1, tid = threadIdx.x;
-  for (int i = tid; i < nl; i += blockDim.x) {
-    double di = B.d[a0 + i];
-    if (i == 0 && a0 > 0) di -= fabs(B.e[a0 - 1]);             // rank-one tearing at the left cut
-    if (i == nl - 1 && L.a1 < n) di -= fabs(B.e[L.a1 - 1]);    // and at the right cut
-    d[i] = di;
-    e[i] = (i < nl - 1) ? B.e[a0 + i] : 0.0;
+  const int n = B.n, a0 = L.a0, nl = L.a1 - L.a0, tid = threadIdx.x;
+  double* Z = sm;
+  double* U = Z + kLeaf * kLeafLd;
+  double* d = U + kLeaf * kLeafLd;
+  double* e = d + kLeaf;
+  int bad = 0;
+  if (tid < nl) {
+    double di = B.d[a0 + tid];
+    if (tid == 0 && a0 > 0) di -= fabs(B.e[a0 - 1]);             // rank-one tearing at the left cut
+    if (tid == nl - 1 && L.a1 < n) di -= fabs(B.e[L.a1 - 1]);    // and at the right cut
+    d[tid] = di;
+    e[tid] = (tid < nl - 1) ? B.e[a0 + tid] : 0.0;
+    bad = !(isfinite(di) && isfinite(e[tid]));
   }
-  for (int idx = tid; idx < nl * nl; idx += blockDim.x) {
-    const int r = idx / nl, c = idx % nl;
-    Z[r * ld + c] = (r == c) ? 1.0 : 0.0;
+  if (__syncthreads_or(bad)) {  // the reduction has flagged the block; anything finite will do
+    if (tid < nl) {
+      d[tid] = 0.0;
+      e[tid] = 0.0;
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  const int st = smem_ql(d, e, nl, Z, ld, nl, C, S, ctl);
+  const int st = smem_dc<kLeaf / 32>(d, e, nl, Z, U, kLeafLd, e + kLeaf, ctl);
   if (st && tid == 0) atomicMax(B.info, st);
-  for (int r = tid; r < nl; r += blockDim.x) B.lam[a0 + r] = d[r];
-  for (int idx = tid; idx < nl * nl; idx += blockDim.x) {
-    const int r = idx / nl, c = idx % nl;  // row r of Zt = column r of Z
-    B.H[(size_t)(a0 + r) * n + a0 + c] = Z[c * ld + r];
+  if (tid < nl) B.lam[a0 + tid] = d[tid];
+  for (int idx = tid; idx < nl * nl; idx += kCtaEigThreads) {
+    const int r = idx / nl, c = idx % nl;
+    B.H[(size_t)(a0 + r) * n + a0 + c] = Z[r * kLeafLd + c];
   }
 }
 
@@ -1395,7 +1397,7 @@ __global__ void __launch_bounds__(512) dc_prep_kernel(const LargeBlock* __restri
   }
   dmx = block_max(dmx, red);
   zmx = block_max(zmx, red);
-  const double tol = 8.0 * kEps * fmax(dmx, zmx);
+  const double tol = 8.0 * kEps * fmax(dmx, rho * zmx);  // relative to the merged matrix
   const bool none = rho * zmx <= tol;  // nothing couples the children
   // 3. deflation of small couplings; the rest in order. Thread t has the positions [s0, s1).
   const int per = (N + nt - 1) / nt, s0 = min(N, tid * per), s1 = min(N, s0 + per);
@@ -1651,12 +1653,7 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __res
         lo = -mid;
         hi = 0.0;
       }
-      // the other poles' part is taken as constant: c + z1 / (d1 - x) + z2 / (d2 - x) = 0
-      const double c = f + (z1 - z2) / mid;
-      const double A1 = (f >= 0.0 ? c * gap : -c * gap) + z1 + z2;
-      const double A0 = f >= 0.0 ? z1 * gap : -z2 * gap;
-      const double disc = sqrt(fabs(A1 * A1 - 4.0 * c * A0));
-      tau = A1 > 0.0 ? 2.0 * A0 / (A1 + disc) : (A1 - disc) / (2.0 * c);
+      tau = secular_start(f, f + (z1 - z2) / mid, gap, z1, z2);
       if (!(tau > lo && tau < hi)) tau = 0.5 * (lo + hi);
     } else {
       double s = 0.0;
@@ -1671,16 +1668,15 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __res
     const double d1 = ds[p1] - dorg, d2 = ds[p2] - dorg;
     for (int it = 0; it < 100; it++) {
       double psi = 0.0, dpsi = 0.0, phi = 0.0, dphi = 0.0;
+#pragma unroll 4
       for (int i = lane; i < K; i += 32) {
-        const double del = (dg[i] - dorg) - tau;
-        const double t = zg[i] / del;
-        if (rk[i] <= p1) {
-          psi = fma(zg[i], t, psi);
-          dpsi = fma(t, t, dpsi);
-        } else {
-          phi = fma(zg[i], t, phi);
-          dphi = fma(t, t, dphi);
-        }
+        const double z = zg[i], t = z / ((dg[i] - dorg) - tau);
+        const bool left = rk[i] <= p1;
+        const double zl = left ? z : 0.0, tl = left ? t : 0.0, zr = left ? 0.0 : z, tr = left ? 0.0 : t;
+        psi = fma(zl, t, psi);
+        dpsi = fma(tl, t, dpsi);
+        phi = fma(zr, t, phi);
+        dphi = fma(tr, t, dphi);
       }
       psi = rho * warp_sum(psi);
       dpsi = rho * warp_sum(dpsi);
@@ -1690,22 +1686,7 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __res
       const double err = 8.0 * (fabs(psi) + fabs(phi)) + 2.0 + 3.0 * fabs(tau) * (dpsi + dphi);
       if (fabs(f) <= kEps * err) break;
       if (f < 0.0) lo = tau; else hi = tau;
-      // two-pole rational model through poles p1, p2 matching f and f'; its root between the
-      // poles, or for the last root the one right of both
-      const double del1 = d1 - tau, del2 = d2 - tau;
-      const double cc = f - del1 * dpsi - del2 * dphi;
-      const double s1 = del1 * del1 * dpsi, s2 = del2 * del2 * dphi;
-      const double A1 = cc * (del1 + del2) + s1 + s2;
-      const double A0 = cc * del1 * del2 + s1 * del2 + s2 * del1;
-      double eta;
-      if (cc == 0.0) {
-        eta = A0 / A1;
-      } else {
-        const double disc = sqrt(fabs(A1 * A1 - 4.0 * cc * A0));
-        if (last) eta = (A1 >= 0.0) ? (A1 + disc) / (2.0 * cc) : 2.0 * A0 / (A1 - disc);
-        else eta = (A1 <= 0.0) ? (A1 - disc) / (2.0 * cc) : 2.0 * A0 / (A1 + disc);
-      }
-      double tn = tau + eta;
+      double tn = tau + secular_step(f, dpsi, dphi, d1 - tau, d2 - tau, last);
       if (!(tn > lo && tn < hi)) tn = 0.5 * (lo + hi);
       if (tn == tau) break;
       tau = tn;
@@ -2516,7 +2497,9 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
     // ---- 2. divide and conquer
     {
       PhaseScope ps(c, kPhDcLeaf, s);
-      dc_leaf_kernel<<<(int)leaves.size(), 128, 0, s>>>(dblk, reinterpret_cast<const DcLeaf*>(dbase + leaf_off));
+      const size_t ls = sizeof(double) * 2 * (kLeaf * kLeafLd + kLeaf) + dc_scratch_bytes(kLeaf);
+      NRG_CK(cudaFuncSetAttribute(dc_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ls));
+      dc_leaf_kernel<<<(int)leaves.size(), kCtaEigThreads, ls, s>>>(dblk, reinterpret_cast<const DcLeaf*>(dbase + leaf_off));
       NRG_CK(cudaGetLastError());
     }
     for (size_t h = 0; h < levels.size(); h++) {

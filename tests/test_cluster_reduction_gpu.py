@@ -48,3 +48,30 @@ def test_same_result_in_any_cluster(nb, n):
     for k in (0, 1, 11):
         alone = nb.diagonalisations([blocks[k]])[0]
         assert np.array_equal(alone.val, together[k].val) and np.array_equal(alone.vec, together[k].vec)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-140, 1e140])
+def test_one_cta_solver_orders(nb, oracle, scale):
+    """Every order the one-CTA solver can be given (its merge trees and tile remainders differ), with
+    random, graded, degenerate and decoupled matrices, at the scale where squares nearly overflow."""
+    rng = np.random.default_rng(3)
+    ctx = nb.Context()
+    ctx.set_tuning(small_max_n=96)
+    blocks = []
+    for n in range(1, 97):
+        a = rng.standard_normal((n, n))
+        h = np.triu(a + a.T)
+        if n % 4 == 1:
+            h = np.diag(np.repeat(rng.standard_normal((n + 2) // 3), 3)[:n])  # exactly degenerate
+        elif n % 4 == 2:
+            h = np.triu(a * 0.1, 1) + np.diag(2.0 ** (-np.arange(n) / 2.0))
+        elif n % 4 == 3:
+            h[: n // 2, n // 2:] = 0.0
+        blocks.append(h * scale)
+    got = nb.diagonalisations(blocks, ctx=ctx, check_upper=False)
+    for h, g in zip(blocks, got):
+        w, v = oracle.diagonalise(h)
+        if scale == 1.0:
+            check_eig(h, g.val, g.vec, w, v, oracle)
+        else:  # check_eig's norms underflow or overflow; the scaled problem is the same one
+            check_eig(h / scale, g.val / scale, g.vec, w / scale, v, oracle)
