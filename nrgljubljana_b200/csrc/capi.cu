@@ -101,8 +101,10 @@ void GemmPlan::add_out(double* C, int64_t ldc, int M, int N, double beta) {
   o.seg0 = (int)segs.size();
   o.nseg = 0;
   o.tile0 = tiles;
+  o.tile0s = tiles_s;
   o.beta = beta;
-  tiles += ((M + kGemmBM - 1) / kGemmBM) * ((N + kGemmBN - 1) / kGemmBN);
+  tiles += gemm_tiles(M, N, kGemmBM, kGemmBN);
+  tiles_s += gemm_tiles(M, N, kGemmSmallBM, kGemmSmallBM);
   outs.push_back(o);
 }
 
@@ -127,6 +129,7 @@ StagedGemm stage_gemm(std::vector<char>& img, const GemmPlan& p) {
   g.segs_off = push(img, p.segs);
   g.nout = (int)p.outs.size();
   g.tiles = p.tiles;
+  g.tiles_s = p.tiles_s;
   return g;
 }
 
@@ -182,7 +185,7 @@ int launch_staged_gemm(nrg_ctx* c, const StagedGemm& g, cudaStream_t s, int phas
   PhaseScope ps(c, phase, s);
   const char* base = static_cast<const char*>(c->desc);
   NRG_CK(gemm_batch_launch(reinterpret_cast<const GemmOut*>(base + g.outs_off),
-                           reinterpret_cast<const GemmSeg*>(base + g.segs_off), g.nout, g.tiles, s));
+                           reinterpret_cast<const GemmSeg*>(base + g.segs_off), g.nout, g.tiles, g.tiles_s, s));
   return NRG_OK;
 }
 

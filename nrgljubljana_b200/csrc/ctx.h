@@ -89,7 +89,7 @@ size_t push(std::vector<char>& img, const std::vector<T>& v) {
 struct GemmPlan {
   std::vector<GemmOut> outs;
   std::vector<GemmSeg> segs;
-  int tiles = 0;
+  int tiles = 0, tiles_s = 0;  // of 64 x 64 and of 32 x 32
   void add_out(double* C, int64_t ldc, int M, int N, double beta);
   void add_seg(const double* A, int64_t lda, int transA, const double* B, int64_t ldb, int transB, int K,
                double alpha);
@@ -99,7 +99,7 @@ struct GemmPlan {
 // and other descriptors share one staging copy.
 struct StagedGemm {
   size_t outs_off = 0, segs_off = 0;
-  int nout = 0, tiles = 0;
+  int nout = 0, tiles = 0, tiles_s = 0;
 };
 StagedGemm stage_gemm(std::vector<char>& img, const GemmPlan& p);
 int launch_staged_gemm(nrg_ctx* c, const StagedGemm& g, cudaStream_t s, int phase);

@@ -30,20 +30,22 @@ struct RowScale {
 cudaError_t row_scale_launch(const RowScale* d_terms, int nterm, int64_t total, cudaStream_t stream);
 
 // One output C (M x N, row-major, ldc): C = beta*C + sum over its segments. Tiles of
-// 64 x 64 are numbered from tile0 in row-major tile order.
+// 64 x 64 are numbered from tile0 in row-major tile order, tiles of 32 x 32 from tile0s.
 struct GemmOut {
   double* C;
   int64_t ldc;
   int M, N;
   int seg0, nseg;
-  int tile0, pad_;
+  int tile0, tile0s;
   double beta;
 };
 
-constexpr int kGemmBM = 64, kGemmBN = 64, kGemmBK = 16, kGemmThreads = 128;
+constexpr int kGemmBM = 64, kGemmBN = 64, kGemmSmallBM = 32, kGemmBK = 16, kGemmThreads = 128;
+constexpr int kGemmSmallTiles = 592;  // calls of at most this many 64 x 64 tiles use 32 x 32 ones
+inline int gemm_tiles(int M, int N, int bm, int bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn); }
 
 // Launch over nout outputs whose descriptors already live in device memory.
-cudaError_t gemm_batch_launch(const GemmOut* d_outs, const GemmSeg* d_segs, int nout, int ntiles,
+cudaError_t gemm_batch_launch(const GemmOut* d_outs, const GemmSeg* d_segs, int nout, int ntiles, int ntiles_s,
                               cudaStream_t stream);
 // One output C = beta*C + alpha op(A) op(B) with descriptors passed as kernel parameters.
 cudaError_t gemm_one_launch(const GemmOut& o, const GemmSeg& g, cudaStream_t stream);
