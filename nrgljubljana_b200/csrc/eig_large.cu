@@ -5,7 +5,9 @@
 // of copy_results (ascending eigenvalues, eigenvectors as rows, c++/diag.hpp:41-58).
 //
 // Pipeline per chunk of blocks (all blocks of the chunk advance together):
-//   1. tridiag_kernel     one CTA per block: blocked Householder reduction A = Q T Q^T
+//   1. reduction to tridiagonal form, one of several by order and number of the blocks (in
+//      shared memory, by groups of CTAs through L2, in two stages, or, for many large blocks,)
+//      tridiag_kernel     one CTA per block: blocked Householder reduction A = Q T Q^T
 //                         (panel width NB); the symmetric matrix-vector product streams
 //                         the lower triangle from HBM once per column, the panel update
 //                         is a rank-2NB update of the trailing lower triangle.
@@ -72,6 +74,7 @@ struct LargeBlock {
   char* pscr;     // kPrepGlobalB bytes per row: merge-prep arrays of nodes too large for shared memory
   int2* slot;     // per node row: (grouped slot, support) of the eigenvector row
   DcRot* rot;     // per node: deflation rotations, in order
+  double* gx;     // exchange buffers of tridiag_grid_kernel
   int* info;
   int n, npanel;
   int ldp, pad_;  // leading dimension of the packed lower triangle in W1 (multiple of 32)
@@ -610,194 +613,6 @@ __global__ void __launch_bounds__(kTriThreads, MINB) tridiag_kernel(const LargeB
   if (__syncthreads_or(bad) && tid == 0) atomicMin(B.info, -2);
 }
 
-// ---------------------------------------------------------------- large blocks, few of them
-// One thread-block cluster per block: the blocked reduction of tridiag_kernel with the TMA
-// slabs of A v and the tiles of the panel update split over the warps of every CTA of the
-// cluster. The column work (current column, reflector) is repeated by every CTA on its own
-// copy of the vectors; each CTA writes its slice of rows to global memory. The parts of A v
-// and of the dot products are summed through distributed shared memory: after the first
-// barrier each CTA reduces its slice of rows, after the second the scalar y^T v is summed;
-// the third makes the column of W visible to the cluster, a fourth follows each panel update.
-// Every CTA executes the same sequence of barriers whatever the data.
-constexpr int kTclC = 8;  // CTAs per cluster (16 when the blocks are few)
-
-template <int STAGES>
-__global__ void __launch_bounds__(kTriThreads, 1) tridiag_tcl_kernel(const LargeBlock* __restrict__ blocks,
-                                                                     const CUtensorMap* __restrict__ tmaps) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cl = cg::this_cluster();
-  extern __shared__ __align__(16) double sm[];
-  __shared__ __align__(8) uint64_t bars[kTriWarps * STAGES];
-  const int C = (int)cl.num_blocks(), rk = (int)cl.block_rank();
-  const int bi = blockIdx.x / C;
-  const LargeBlock B = blocks[bi];
-  const int n = B.n, ld = B.ldp, tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-  const int gw = rk * nwarps + warp, gnw = C * nwarps;
-  double* A = B.W1;
-  double* W = B.W2;
-  // The arrays that other CTAs read (y, dots, pps) sit at fixed offsets from the start of the
-  // dynamic shared memory, so that map_shared_rank finds them at the same offsets in every
-  // CTA; the 1024-byte aligned TMA ring comes last (its padding depends on where the CTA's
-  // shared memory window starts, which differs between CTAs sharing an SM).
-  double* y = sm;                                   // n: this CTA's part of A v; its slice: the reduced y
-  double* dots = y + n;                             // 2NB: this CTA's part of W^T v, V^T v
-  double* pps = dots + 2 * NB;                      // 2: this CTA's part of y^T v
-  double* v = pps + 2;                              // n: current column, then the reflector
-  double* part = v + n;                             // nwarps * 2NB
-  double* cwv = part + nwarps * 2 * NB;             // 2NB: the sums
-  double* red = cwv + 2 * NB;                       // 64 (two halves for block_sum_1b)
-  double* ring = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(red + 64) + 1023) & ~(uintptr_t)1023);
-  int phase = 0;
-  unsigned parity = 0;
-  if (lane == 0) {
-    for (int st = 0; st < STAGES; st++) mbar_init(bars + warp * STAGES + st, 1);
-    fence_mbar_init();
-    tmap_acquire(tmaps + bi);  // lane 0 issues this warp's bulk copies
-  }
-  __syncthreads();
-
-  for (int p0 = 0; p0 < n - 2; p0 += NB) {
-    const int pe = min(p0 + NB, n - 2);
-    for (int k = p0; k < pe; k++) {
-      const int j = k - p0;
-      // (1) current column k (rows k..n-1) = stored column minus the pending panel terms
-      {
-        double wk[NB], vk[NB];
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-          wk[q] = (q < j) ? __ldcg(W + (size_t)q * n + k) : 0.0;
-          vk[q] = (q < j) ? __ldcg(A + (size_t)(p0 + q) * ld + k) : 0.0;
-        }
-        for (int i = k + tid; i < n; i += nt) {
-          double a = __ldcg(A + (size_t)k * ld + i);
-#pragma unroll
-          for (int q = 0; q < NB; q++)
-            if (q < j) a -= __ldcg(A + (size_t)(p0 + q) * ld + i) * wk[q] + __ldcg(W + (size_t)q * n + i) * vk[q];
-          v[i] = a;
-          y[i] = 0.0;
-        }
-      }
-      __syncthreads();
-      // (2) Householder reflector for rows k+1..n-1 (dlarfg convention, v[k+1] = 1)
-      double ps = 0.0;
-      for (int i = k + 2 + tid; i < n; i += nt) ps += v[i] * v[i];
-      const double alpha = v[k + 1];  // before the barrier: thread 0 sets v[k+1] = 1 below
-      const double sigma = block_sum_1b(ps, red, phase);
-      double tau = 0.0, beta = alpha, scale = 1.0;
-      if (sigma > 0.0) {
-        beta = -copysign(sqrt(alpha * alpha + sigma), alpha);
-        tau = (beta - alpha) / beta;
-        scale = 1.0 / (alpha - beta);
-      }
-      if (rk == 0 && tid == 0) {
-        B.d[k] = v[k];
-        B.e[k] = beta;
-        B.tau[k] = tau;
-      }
-      for (int i = k + 2 + tid; i < n; i += nt) v[i] *= scale;
-      if (tid == 0) v[k + 1] = 1.0;
-      __syncthreads();
-      // column k of A is written back only in (5): other CTAs may still be reading it in (1)
-      // (3) this CTA's part of A v and of the dot products W^T v, V^T v over its slice of rows
-      const int ch1 = (n - k - 1 + C - 1) / C, lo1 = k + 1 + rk * ch1, hi1 = min(n, lo1 + ch1);
-      if (tau != 0.0) symv_lower<STAGES>(tmaps + bi, n, k + 1, v, y, ring, bars, parity, B.info, gw, gnw);
-      {
-        double pw[NB], pv[NB];
-#pragma unroll
-        for (int q = 0; q < NB; q++) pw[q] = pv[q] = 0.0;
-        if (tau != 0.0 && j > 0) {
-          for (int i = lo1 + tid; i < hi1; i += nt) {
-            const double vi = v[i];
-#pragma unroll
-            for (int q = 0; q < NB; q++)
-              if (q < j) {
-                pw[q] = fma(__ldcg(W + (size_t)q * n + i), vi, pw[q]);
-                pv[q] = fma(__ldcg(A + (size_t)(p0 + q) * ld + i), vi, pv[q]);
-              }
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-          const double a = warp_sum(pw[q]);
-          const double b = warp_sum(pv[q]);
-          if (lane == 0) {
-            part[warp * 2 * NB + q] = a;
-            part[warp * 2 * NB + NB + q] = b;
-          }
-        }
-        __syncthreads();
-        if (tid < 2 * NB) {
-          double t = 0.0;
-          for (int w = 0; w < nwarps; w++) t += part[w * 2 * NB + tid];
-          dots[tid] = t;
-        }
-      }
-      cl.sync();  // (B1) the parts of A v and of the dot products are complete
-      // (4) this CTA's slice: y = (sum of the parts - V (W^T v) - W (V^T v)) tau
-      if (tid < 2 * NB) {
-        double t = 0.0;
-        for (int q = 0; q < C; q++) t += cl.map_shared_rank(dots, q)[tid];
-        cwv[tid] = t;
-      }
-      __syncthreads();
-      double pp = 0.0;
-      if (tau != 0.0) {
-        double cw[NB], cv[NB];
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-          cw[q] = (q < j) ? cwv[q] : 0.0;
-          cv[q] = (q < j) ? cwv[NB + q] : 0.0;
-        }
-        for (int i = lo1 + tid; i < hi1; i += nt) {
-          double yi = 0.0;
-          for (int q = 0; q < C; q++) yi += cl.map_shared_rank(y, q)[i];
-#pragma unroll
-          for (int q = 0; q < NB; q++)
-            if (q < j) yi -= __ldcg(A + (size_t)(p0 + q) * ld + i) * cw[q] + __ldcg(W + (size_t)q * n + i) * cv[q];
-          yi *= tau;
-          pp = fma(yi, v[i], pp);
-          y[i] = yi;  // only this CTA's slice is read from here on, and only by this CTA
-        }
-      }
-      const double ppb = block_sum_1b(pp, red, phase);
-      if (tid == 0) pps[0] = ppb;
-      cl.sync();  // (B2) every CTA has its slice of y and its part of y^T v
-      double yv = 0.0;
-      for (int q = 0; q < C; q++) yv += cl.map_shared_rank(pps, q)[0];
-      const double Kc = 0.5 * tau * yv;
-      for (int i = lo1 + tid; i < hi1; i += nt) {
-        W[(size_t)j * n + i] = (tau != 0.0) ? y[i] - Kc * v[i] : 0.0;
-        A[(size_t)k * ld + i] = v[i];  // the reflector, unit at k+1
-      }
-      if (rk == 0) {  // zeros from the start of its back-transform panel down to the diagonal
-        const int kb0 = (k / NBT) * NBT;
-        for (int i = kb0 + 1 + tid; i <= k; i += nt) A[(size_t)k * ld + i] = 0.0;
-      }
-      cl.sync();  // (B3) column j of W and column k of the reflectors are visible to the cluster
-    }
-    panel_update<true>(A, W, n, ld, p0, pe - p0, pe, gw, gnw);
-    fence_proxy_async_global();  // the next products read the updated trailing block by bulk copies
-    cl.sync();                   // (B4)
-    fence_proxy_async_global();
-  }
-  if (rk == 0) {
-    if (tid == 0) {
-      B.d[n - 2] = __ldcg(A + (size_t)(n - 2) * ld + n - 2);
-      B.e[n - 2] = __ldcg(A + (size_t)(n - 2) * ld + n - 1);
-      B.d[n - 1] = __ldcg(A + (size_t)(n - 1) * ld + n - 1);
-      B.e[n - 1] = 0.0;
-      B.tau[n - 2] = 0.0;
-      B.tau[n - 1] = 0.0;
-    }
-    __syncthreads();
-    int bad = 0;
-    for (int i = tid; i < n; i += nt) bad |= !(isfinite(B.d[i]) && isfinite(B.e[i]));
-    if (__syncthreads_or(bad) && tid == 0) atomicMin(B.info, -2);
-  }
-  cl.sync();  // no CTA leaves while another may still read its shared memory
-}
-
 // ---------------------------------------------------------------- mid-size tridiagonalisation
 // Blocks with small_max_n < n <= mid_max_n (nrg_tuning): the whole lower triangle fits in shared memory,
 // packed by columns (column j holds rows j..n-1 at pcol(j)), so the unblocked Householder
@@ -1214,6 +1029,494 @@ __global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const Large
     int bad = 0;
     for (int i = tid; i < n; i += kDsmThreads) bad |= !(isfinite(B.d[i]) && isfinite(B.e[i]));
     if (__syncthreads_or(bad) && tid == 0) atomicMin(B.info, -2);
+  }
+}
+
+// ---------------------------------------------------------------- large blocks, few of them
+// The blocked reduction of one block by a group of G CTAs (one per SM, all of them resident: one
+// cooperative launch for every group). What bounds it is the chain of n columns, two exchanges
+// through L2 per column, and for the largest blocks the bytes of the trailing matrix per column.
+//   The full symmetric matrix is kept (W1[j ld + i] = A(i, j)), twice the triangle's bytes: then
+//   CTA r's columns j = r + t G give complete products A(:, j) v -- no partial vectors to add up over
+//   the group -- by plain 16-byte loads with v in shared memory, and the CTA is the only one that
+//   reads or updates its columns.
+//   Per column k of a panel of kGNB every CTA has the whole column in shared memory and builds the
+//   reflector v itself. It publishes its part of W^T v and V^T v, forms the products of its columns
+//   (which cover that exchange), then its rows of t = tau (A v - V (W^T v) - W (V^T v)) and of the
+//   next column without the terms in K = tau/2 t^T v and t(k+1), and publishes these beside its part
+//   of K: the one exchange that is waited for. The next column is b + (2 K - t(k+1)) v, W = t - K v.
+//   At the panel's end, after a barrier, each CTA updates its columns by V W^T + W V^T on the FP64
+//   tensor cores.
+// An exchanged number travels in 16 bytes with the column it belongs to, and its readers poll it: a
+// barrier (fence, counter, poll, and the loads behind it) took 2 us, twice per column. Each buffer
+// is written again only after its writer has received what every reader sends after reading it.
+constexpr int kGridThreads = 512;
+constexpr int kGridWarps = kGridThreads / 32;
+constexpr int kGNB = 16;           // panel width
+constexpr int kGridMaxT = 256;     // columns per CTA
+constexpr int kGridSeg = 8;        // most row segments of a product
+constexpr int kGridMaxG = 160;     // most CTAs of a group
+
+struct GridGroup {
+  int cta0, G;        // its CTAs
+  int job0, njob;     // its blocks, one after another: jobs[job0 ..]
+};
+
+
+// Doubles of global scratch per block (pairs: number, tag): next column, parts of K, parts of the dot
+// products, then t(k+1) and row k+1 of V and W.
+__host__ __device__ inline size_t grid_scratch_doubles(int n) {
+  return 2 * ((size_t)n + kGridMaxG + (size_t)kGridMaxG * 2 * kGNB + 2 * kGNB + 1);
+}
+__host__ __device__ inline size_t grid_smem_doubles(int ldp, int T) {
+  return (size_t)ldp + 64 + (2 * kGNB + 2 + kGridSeg) * (size_t)T + 4 * kGNB + 64 + 32;
+}
+
+// Barrier over the group's CTAs: the counter reaches `target` when all have arrived. False if the
+// bounded wait ran out (the block is flagged, and the caller stops waiting).
+NRG_DEV bool group_barrier(unsigned* ctr, unsigned target, bool wait) {
+  __syncthreads();
+  int ok = 1;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
+    if (wait) {
+      ok = 0;
+      for (int it = 0; it < (1 << 24); it++) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
+        if ((int)(v - target) >= 0) {
+          ok = 1;
+          break;
+        }
+      }
+      __threadfence();
+    }
+  }
+  return __syncthreads_and(threadIdx.x != 0 || ok) != 0;
+}
+
+// One 16-byte access each, so number and tag are always of the same store.
+NRG_DEV void tag_store(double2* p, double x, unsigned tag) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(p),
+               "l"(__double_as_longlong(x)), "l"((long long)tag)
+               : "memory");
+}
+NRG_DEV bool tag_load(const double2* p, unsigned tag, double& x) {
+  long long a, b;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}\n"
+               : "=l"(a), "=l"(b)
+               : "l"(p)
+               : "memory");
+  x = __longlong_as_double(a);
+  return b == (long long)tag;
+}
+// Bounded poll of one number; live turns false when the bound runs out (the caller flags the block and
+// no later poll waits).
+NRG_DEV double tag_wait(const double2* p, unsigned tag, bool& live) {
+  double x = 0.0;
+  bool ok = tag_load(p, tag, x);
+  for (int it = 0; !ok && live; it++) {
+    ok = tag_load(p, tag, x);
+    if (it >= 1 << 24) live = false;
+  }
+  return x;
+}
+
+// Lower-triangle input (rows of H from the diagonal on) to the full symmetric W1, 32 x 32 tiles.
+__global__ void __launch_bounds__(256) pack_full_kernel(const LargeBlock* __restrict__ blocks) {
+  __shared__ double tile[32][33];
+  const LargeBlock B = blocks[blockIdx.z];
+  const int n = B.n, ld = B.ldp, i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;  // j0 <= i0: H(j, i), i >= j
+  if (j0 == 0)  // no tag of an earlier reduction is left in the exchange buffers
+    for (size_t q = blockIdx.x * 256 + threadIdx.x; q < grid_scratch_doubles(n); q += (size_t)gridDim.x * 256) B.gx[q] = 0.0;
+  if (i0 >= ld || j0 >= n || j0 > i0) return;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int r = ty; r < 32; r += 8) {
+    const int j = j0 + r, i = i0 + tx;
+    tile[r][tx] = j < n && i < n && i >= j ? B.H[(size_t)j * n + i] : 0.0;
+  }
+  __syncthreads();
+  for (int r = ty; r < 32; r += 8) {
+    const int j = j0 + r, i = i0 + tx;  // column j, rows i: below the diagonal
+    if (j < n) {
+      const double x = i0 != j0 || tx >= r ? tile[r][tx] : tile[tx][r];
+      B.W1[(size_t)j * ld + i] = x;
+    }
+    if (i0 != j0) {  // column i, rows j: above it
+      const int jj = i0 + r, ii = j0 + tx;
+      if (jj < n) B.W1[(size_t)jj * ld + ii] = tile[tx][r];
+    }
+  }
+}
+
+// Sum over the lanes of x[c] for c = (lane >> 3) & 3, in every lane.
+NRG_DEV double colsum4(double (&x)[4], int lane) {
+#pragma unroll
+  for (int s = 2, o = 16; s >= 1; s >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int q = 0; q < s; q++) {
+      const double send = up ? x[q] : x[q + s];
+      const double keep = up ? x[q + s] : x[q];
+      x[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+  return x[0];
+}
+
+// Products of a CTA's columns t0 .. T-1 with the vector vf: items of four columns x a segment of the rows
+// (S of them, chunks of 64 rows from `base`), parts of the sums in yp.
+__device__ __forceinline__ void grid_products(const double* A, int yp_off, int ld, int r, int G, int T, int Tm, int t0,
+                                           int ng, int S, int base, int nch) {
+  extern __shared__ __align__(16) double sm[];
+  const double* vf = sm;
+  double* yp = sm + yp_off;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int it = warp; it < ng * S; it += kGridWarps) {
+    const int tg = t0 + 4 * (it / S), s = it % S, c0 = nch * s / S, c1 = nch * (s + 1) / S;
+    const double* col[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) col[c] = A + (size_t)(r + (tg + c < T ? tg + c : tg) * G) * ld + base + 2 * lane;
+    const double2* vp = reinterpret_cast<const double2*>(vf + base + 2 * lane);
+    double sum[4] = {};
+    const int cf = min(c1, (ld - base) / 64);  // a last chunk may have 32 rows only
+    int ch = c0;
+    for (; ch + 4 <= cf; ch += 4) {  // sixteen loads a lane before the first is used
+      double2 x[4][4], v[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) x[u][c] = __ldcg(reinterpret_cast<const double2*>(col[c] + 64 * (ch + u)));
+#pragma unroll
+      for (int u = 0; u < 4; u++) v[u] = vp[32 * (ch + u)];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) sum[c] = fma(x[u][c].x, v[u].x, fma(x[u][c].y, v[u].y, sum[c]));
+    }
+    for (; ch < cf; ch++) {
+      const double2 v = vp[32 * ch];
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const double2 x = __ldcg(reinterpret_cast<const double2*>(col[c] + 64 * ch));
+        sum[c] = fma(x.x, v.x, fma(x.y, v.y, sum[c]));
+      }
+    }
+    if (ch < c1 && lane < 16) {
+      const double2 v = vp[32 * ch];
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const double2 x = __ldcg(reinterpret_cast<const double2*>(col[c] + 64 * ch));
+        sum[c] = fma(x.x, v.x, fma(x.y, v.y, sum[c]));
+      }
+    }
+    __syncwarp();
+    const double y = colsum4(sum, lane);
+    const int c = lane >> 3;
+    if ((lane & 7) == 0 && tg + c < T) yp[s * Tm + tg + c] = y;
+  }
+}
+
+// A(i, j) -= V(i, :) W(j, :)^T + W(i, :) V(j, :)^T for a CTA's columns j = r + t G >= pe and the rows i >= pe.
+__device__ __forceinline__ void grid_panel_update(double* A, const double* W, int vo_off, int n, int ld, int r, int G,
+                                               int T, int Tm, int t0, int p0, int pe, int nbp) {
+  extern __shared__ __align__(16) double sm[];
+  const double* Vo = sm + vo_off;
+  const double* Wo = Vo + kGNB * Tm;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int fr = lane >> 2, fc = lane & 3;
+  for (int i0 = (pe & ~31) + 32 * warp; i0 < n; i0 += 32 * kGridWarps) {
+    double bf[2 * kGNB / 4][4];  // [V; W] rows q of the 32 rows i
+#pragma unroll
+    for (int ks = 0; ks < 2 * kGNB / 4; ks++) {
+      const int q = 4 * ks + fc, qq = q < kGNB ? q : q - kGNB;
+      const double* row = q < kGNB ? A + (size_t)(p0 + qq) * ld : W + (size_t)qq * n;
+#pragma unroll
+      for (int ni = 0; ni < 4; ni++) {
+        const int i = i0 + 8 * ni + fr;
+        bf[ks][ni] = qq < nbp && i >= pe && i < n ? __ldcg(row + i) : 0.0;
+      }
+    }
+    for (int tg = t0; tg < T; tg += 8) {
+      const int t = tg + fr;
+      double* col = A + (size_t)(r + (t < T ? t : t0) * G) * ld + i0 + 2 * fc;
+      double acc[4][2];
+#pragma unroll
+      for (int ni = 0; ni < 4; ni++) {
+        const double2 x = __ldcg(reinterpret_cast<const double2*>(col + 8 * ni));
+        acc[ni][0] = x.x;
+        acc[ni][1] = x.y;
+      }
+#pragma unroll
+      for (int ks = 0; ks < 2 * kGNB / 4; ks++) {
+        const int q = 4 * ks + fc, qq = q < kGNB ? q : q - kGNB;
+        const double a = t < T && qq < nbp ? -(q < kGNB ? Wo : Vo)[qq * Tm + t] : 0.0;
+#pragma unroll
+        for (int ni = 0; ni < 4; ni++) dmma884(acc[ni][0], acc[ni][1], a, bf[ks][ni]);
+      }
+      if (t < T) {
+#pragma unroll
+        for (int ni = 0; ni < 4; ni++)
+          __stcg(reinterpret_cast<double2*>(col + 8 * ni), make_double2(acc[ni][0], acc[ni][1]));
+      }
+    }
+  }
+}
+
+// ROWS: rows of a column per thread (8: orders up to 4096, 20: up to 10240).
+template <int ROWS>
+__global__ void __launch_bounds__(kGridThreads, 1) tridiag_grid_kernel(const LargeBlock* __restrict__ blocks,
+                                                                       const GridGroup* __restrict__ groups, int ngroup,
+                                                                       const int* __restrict__ jobs, unsigned* ctrs) {
+  extern __shared__ __align__(16) double sm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int g = 0;
+  while (g + 1 < ngroup && groups[g + 1].cta0 <= (int)blockIdx.x) g++;
+  const GridGroup gr = groups[g];
+  const int G = gr.G, r = (int)blockIdx.x - gr.cta0;
+  if (r >= G) return;
+  unsigned* ctr = ctrs + 32 * g;
+  unsigned epoch = 0;
+  bool live = true;
+  int phase = 0;
+  for (int jb = 0; jb < gr.njob; jb++) {
+    const LargeBlock B = blocks[jobs[gr.job0 + jb]];
+    const int n = B.n, ld = B.ldp, T = (n - r + G - 1) / G, Tm = (n + G - 1) / G;
+    double* A = B.W1;
+    double* W = B.W2;
+    double* vf = sm;                    // ld + 64: current reflector, zero outside k+1 .. n-1
+    double* Vo = vf + ld + 64;          // kGNB x Tm: the panel's reflectors at this CTA's rows
+    double* Wo = Vo + kGNB * Tm;
+    double* to = Wo + kGNB * Tm;        // Tm: t
+    double* co = to + Tm;               // Tm: elements of row k+1
+    double* yp = co + Tm;               // kGridSeg x Tm
+    double* cd = yp + kGridSeg * Tm;    // 2 kGNB: W^T v, V^T v
+    double* k1 = cd + 2 * kGNB;         // 2 kGNB: row k+1 of V and W
+    double* red = k1 + 2 * kGNB;        // 64
+    double* sc = red + 64;              // t(k) of the previous reflector; parts of K by warp from 8 on
+    double2* gb = reinterpret_cast<double2*>(B.gx);  // next column
+    double2* gk = gb + n;                            // parts of K
+    double2* gd = gk + kGridMaxG;                    // parts of the dot products
+    double2* gy = gd + kGridMaxG * 2 * kGNB;         // t(k+1), row k+1 of V, of W
+    // parts of K of reflector k, from every CTA (all threads call it; sum in every thread)
+    auto sum_k = [&](int k) {
+      if (warp <= (G - 1) >> 5) {
+        const double s = warp_sum_mma(tid < G ? tag_wait(gk + tid, k + 1, live) : 0.0);
+        if (lane == 0) sc[8 + warp] = s;
+      }
+    };
+    auto k_of = [&]() {
+      double s = 0.0;
+      for (int q = 0; q <= (G - 1) >> 5; q++) s += sc[8 + q];
+      return s;
+    };
+    auto publish_column = [&](int c) {  // column c of the updated matrix, by rows of this CTA's columns
+      for (int t = tid; t < T; t += kGridThreads)
+        if (r + t * G >= c) tag_store(gb + r + t * G, __ldcg(A + (size_t)(r + t * G) * ld + c), c + 1);
+    };
+    for (int i = tid; i < ld + 64; i += kGridThreads) vf[i] = 0.0;
+    publish_column(0);
+    int p0 = 0;
+    double tau = 0.0, scale = 1.0;
+    for (int k = 0; k < n - 2; k++) {
+      const int j = k - p0;
+      const int t0 = k + 1 - r > 0 ? (k + 1 - r + G - 1) / G : 0;  // its first column beyond k
+      // (1) this column: b and K from the group; the previous column's W (own rows); its reflector
+      double b[ROWS];
+      unsigned pending = 0;  // every load goes out before the first is looked at
+#pragma unroll
+      for (int q = 0; q < ROWS; q++) {
+        const int i = k + tid + q * kGridThreads;
+        if (k + q * kGridThreads >= n) break;  // uniform
+        b[q] = 0.0;
+        if (i < n && !tag_load(gb + i, k + 1, b[q])) pending |= 1u << q;
+      }
+      while (pending && live) {
+#pragma unroll
+        for (int q = 0; q < ROWS; q++)
+          if (pending >> q & 1) {
+            b[q] = tag_wait(gb + k + tid + q * kGridThreads, k + 1, live);
+            pending &= ~(1u << q);
+          }
+      }
+      if (j > 0) {
+        sum_k(k - 1);
+        if (tid == kGridThreads - 1) sc[0] = tag_wait(gy, k, live);
+      }
+      __syncthreads();
+      const double Kc = j > 0 ? k_of() : 0.0, vc = j > 0 ? 2.0 * Kc - sc[0] : 0.0, vs = vc * scale;
+      double ps = 0.0;
+#pragma unroll
+      for (int q = 0; q < ROWS; q++) {
+        const int i = k + tid + q * kGridThreads;
+        if (k + q * kGridThreads >= n) break;  // uniform
+        if (i < n) {
+          // the previous reflector is 1 at k and scale u beyond
+          const double a = i == k ? b[q] + vc : fma(vs, vf[i], b[q]);
+          vf[i] = a;
+          if (i >= k + 2) ps = fma(a, a, ps);
+        }
+      }
+      const double sigma = block_sum_mma(ps, red, phase);
+      const double dk = vf[k], alpha = vf[k + 1];
+      const double beta = sigma > 0.0 ? -copysign(sqrt(alpha * alpha + sigma), alpha) : alpha;
+      const double u1 = alpha - beta;
+      if (j > 0)
+        for (int t = tid; t < T; t += kGridThreads) {
+          const int i = r + t * G;
+          if (i >= k) {
+            const double vi = Vo[(j - 1) * Tm + t], wi = to[t] - Kc * vi;
+            Wo[(j - 1) * Tm + t] = wi;
+            __stcg(A + (size_t)(k - 1) * ld + i, vi);
+            __stcg(W + (size_t)(j - 1) * n + i, wi);
+          }
+        }
+      __syncthreads();  // alpha is read, W is complete
+      if (tid == 0) {
+        vf[k] = 0.0;
+        vf[k + 1] = u1;
+      }
+      if (r == k % G)  // zeros from the start of its back-transform panel down to the diagonal
+        for (int i = (k / NBT) * NBT + 1 + tid; i <= k; i += kGridThreads) A[(size_t)k * ld + i] = 0.0;
+      // elements of row k+1 of the own columns, for the next column; T <= kGridMaxT < kGridThreads
+      const bool last = j == kGNB - 1 || k == n - 3;
+      const double ck1 = !last && t0 + tid < T ? __ldcg(A + (size_t)(r + (t0 + tid) * G) * ld + k + 1) : 0.0;
+      // the owner of row k+1 publishes its V and W
+      if ((k + 1) % G == r && tid < 2 * j) {
+        const int q = tid < j ? tid : tid - j;
+        tag_store(gy + 1 + (tid < j ? q : kGNB + q), (tid < j ? Vo : Wo)[q * Tm + t0], k + 1);
+      }
+      __syncthreads();
+      // parts of W^T u and V^T u over the own rows
+      // (the first column of a panel has none, but the exchange has to take place: one dummy)
+      const int nd = max(2 * j, 1);
+      for (int q = warp; q < nd; q += kGridWarps) {
+        const double* x = q < j ? Wo + q * Tm : Vo + (q - j) * Tm;
+        double s = 0.0;
+        if (j > 0)
+          for (int t = t0 + lane; t < T; t += 32) s = fma(x[t], vf[r + t * G], s);
+        s = warp_sum_mma(s);
+        if (lane == 0) tag_store(gd + (size_t)(q < j || j == 0 ? q : kGNB + q - j) * kGridMaxG + r, s, k + 1);
+      }
+      // (2) products of the own columns with u: items of four columns x a segment of the rows
+      const int ng = (T - t0 + 3) / 4, S = ng > 0 ? max(1, min(kGridSeg, kGridWarps / ng)) : 1;
+      const int base = (k + 1) & ~63, nch = (n - base + 63) / 64;
+      grid_products(A, (int)(yp - sm), ld, r, G, T, Tm, t0, ng, S, base, nch);
+      // the reflector's divisions, beside the slower warps' products
+      tau = 0.0;
+      scale = 1.0;
+      if (sigma > 0.0) {
+        tau = (beta - alpha) / beta;
+        scale = 1.0 / u1;
+      }
+      if (tid == 0 && r == 0) {
+        B.d[k] = dk;
+        B.e[k] = beta;
+        B.tau[k] = tau;
+      }
+      if (t0 + tid < T) co[t0 + tid] = ck1;
+      // (3) the sums of the dot products, row k+1 of V and W; t and the next column at the own rows
+      for (int q = warp; q < nd; q += kGridWarps) {
+        const double2* row = gd + (size_t)(q < j || j == 0 ? q : kGNB + q - j) * kGridMaxG;
+        constexpr int kL = (kGridMaxG + 31) / 32;
+        double x[kL], s = 0.0;
+        bool ok[kL];
+#pragma unroll
+        for (int c = 0; c < kL; c++) {
+          x[c] = 0.0;
+          ok[c] = lane + 32 * c >= G || tag_load(row + lane + 32 * c, k + 1, x[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < kL; c++) {
+          if (!ok[c]) x[c] = tag_wait(row + lane + 32 * c, k + 1, live);
+          s += x[c];
+        }
+        s = warp_sum_mma(s);
+        if (lane == 0) cd[q < j || j == 0 ? q : kGNB + q - j] = scale * s;
+      }
+      if (tid < 2 * j) {
+        const int q = tid < j ? tid : kGNB + tid - j;
+        k1[q] = tag_wait(gy + 1 + q, k + 1, live);
+      }
+      __syncthreads();
+      // lanes per row: the sums over the panel are chains
+      const int left = T - t0, L = left <= kGridThreads / 8 ? 8 : left <= kGridThreads / 4 ? 4 : 2;
+      const int tl = tid % L;
+      double pk = 0.0;
+      for (int u = tid / L; u < (left + 31) / 32 * 32; u += kGridThreads / L) {  // whole warps
+        const bool in = u < left;
+        const int t = t0 + (in ? u : 0), i = r + t * G;
+        double y = 0.0, c = 0.0;
+        if (in)
+          for (int q = tl; q < j; q += L) {
+            const double vq = Vo[q * Tm + t], wq = Wo[q * Tm + t];
+            y = fma(vq, cd[q], fma(wq, cd[kGNB + q], y));
+            c = fma(vq, k1[kGNB + q], fma(wq, k1[q], c));
+          }
+        for (int o = L >> 1; o > 0; o >>= 1) {
+          y += __shfl_xor_sync(0xffffffffu, y, o);
+          c += __shfl_xor_sync(0xffffffffu, c, o);
+        }
+        if (in && tl == 0) {
+          double a = yp[t];
+          for (int s = 1; s < S; s++) a += yp[s * Tm + t];
+          y = tau * (scale * a - y);
+          to[t] = y;
+          const double vi = i == k + 1 ? 1.0 : scale * vf[i];
+          Vo[j * Tm + t] = vi;
+          pk = fma(y, vi, pk);
+          if (!last) tag_store(gb + i, co[t] - c - y, k + 2);
+          if (i == k + 1) tag_store(gy, y, k + 1);
+        }
+      }
+      pk = block_sum_mma(pk, red, phase);
+      if (tid == 0) tag_store(gk + r, 0.5 * tau * pk, k + 1);
+      if (!last) continue;
+      // (4) end of the panel: its last W, then the update of the own columns
+      sum_k(k);
+      __syncthreads();
+      const double Kl = k_of();
+      const int pe = k + 1, nbp = j + 1;
+      for (int t = t0 + tid; t < T; t += kGridThreads) {
+        const int i = r + t * G;
+        const double vi = Vo[j * Tm + t], wi = to[t] - Kl * vi;
+        Wo[j * Tm + t] = wi;
+        __stcg(A + (size_t)k * ld + i, vi);
+        __stcg(W + (size_t)j * n + i, wi);
+      }
+      epoch++;
+      if (!group_barrier(ctr, epoch * (unsigned)G, live)) live = false;
+      grid_panel_update(A, W, (int)(Vo - sm), n, ld, r, G, T, Tm, t0, p0, pe, nbp);
+      __syncthreads();
+      p0 = pe;
+      if (k < n - 3) publish_column(pe);
+    }
+    if (!live) atomicExch(B.info, -5);  // a wait ran out (any thread's)
+    // the last 2 x 2, by its columns' owners
+    __syncthreads();
+    if (tid == 0) {
+      if (r == (n - 2) % G) {
+        B.d[n - 2] = __ldcg(A + (size_t)(n - 2) * ld + n - 2);
+        B.e[n - 2] = __ldcg(A + (size_t)(n - 2) * ld + n - 1);
+        B.tau[n - 2] = 0.0;
+      }
+      if (r == (n - 1) % G) {
+        B.d[n - 1] = __ldcg(A + (size_t)(n - 1) * ld + n - 1);
+        B.e[n - 1] = 0.0;
+        B.tau[n - 1] = 0.0;
+      }
+    }
+    epoch++;
+    if (!group_barrier(ctr, epoch * (unsigned)G, live)) live = false;
+    if (r == 0) {
+      int bad = 0;
+      for (int i = tid; i < n; i += kGridThreads) bad |= !(isfinite(__ldcg(B.d + i)) && isfinite(__ldcg(B.e + i)));
+      if (__syncthreads_or(bad) && tid == 0) atomicMin(B.info, -2);
+    }
+    __syncthreads();
   }
 }
 
@@ -1918,7 +2221,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 size_t large_block_doubles(int n, bool two_stage) {
   const size_t ldp = (size_t)(n + 31) / 32 * 32;
-  return (size_t)n * ldp + (size_t)n * n + 8 * (size_t)n + 2 * (size_t)NBT * n + 7 * (size_t)n + 64 * 15 +
+  return (size_t)n * ldp + (size_t)n * n + 8 * (size_t)n + 2 * (size_t)NBT * n + 7 * (size_t)n + 64 * 16 + grid_scratch_doubles(n) +
          (prep_layout(n).total > kPrepSmemMax ? (kPrepGlobalB * (size_t)n + 7) / 8 : 0) +
          (two_stage ? band_extra_doubles(n) + 4 * 64 : 0);
 }
@@ -1944,7 +2247,7 @@ struct DsmPlan {
   std::vector<int> C;
 };
 
-DsmPlan dsm_plan(const LargeBlock* b, int lo, int hi, int mid_max_n, int nsm) {
+DsmPlan dsm_plan(const LargeBlock* b, int lo, int hi, int mid_max_n, int nsm, bool may_stream) {
   DsmPlan p{lo, std::vector<int>(hi, 0)};
   int sum = 0;
   for (int q = lo; q < hi; q++) {
@@ -1980,12 +2283,82 @@ DsmPlan dsm_plan(const LargeBlock* b, int lo, int hi, int mid_max_n, int nsm) {
     clu += p.C[q] * dsm_us(b[q].n, p.C[q]) / nsm;
     bytes += 4.0 / 3.0 * b[q].n * (double)b[q].n * b[q].n;
   }
-  if (mid > lo) {
+  if (mid > lo && may_stream) {
     const double n0 = b[lo].n, stream = std::max(bytes / 4.4e6, 4.0 / 3.0 * n0 * n0 * n0 / 1.5e4);
     if (stream < clu + dsm_us(b[lo].n, p.C[lo])) p.first = mid;
   }
   for (int q = mid; q < hi; q++)
     if (p.C[q] > 1) p.C[q] = 0;
+  return p;
+}
+
+// Microseconds of a block's reduction by a group of G CTAs (B200, see tridiag_grid_kernel): the chain of
+// columns and the bytes an SM streams, 75 GB/s from L2 and 30 when the chip streams from HBM.
+double grid_us(int n, int G, double gbs) { return n * (5.2 + 8.0 / 3.0 * n * n / (1e3 * gbs * G)); }
+int grid_min_ctas(int n) { return (n + kGridMaxT - 1) / kGridMaxT; }
+int grid_max_ctas(int n) { return std::min(kGridMaxG, std::max(grid_min_ctas(n), n / 16)); }
+
+struct GridPlan {
+  std::vector<GridGroup> groups;
+  std::vector<int> jobs;
+  int ctas = 0;
+  size_t smem = 0;
+  double us = 0.0;  // of the slowest group
+};
+
+// Groups for the blocks [0, count) (sorted by falling order) on nsm SMs: the shortest makespan, in steps of
+// 5%, for which the blocks fit, each the first group that still has time for it or else a new one of
+// the least size that is fast enough; what SMs are left go to the slowest groups.
+GridPlan grid_plan(const LargeBlock* b, int count, int nsm) {
+  double foot = 0.0;
+  for (int q = 0; q < count; q++) foot += 8.0 * b[q].n * b[q].n;
+  const double gbs = foot > 1e8 ? 30.0 : 75.0;
+  struct Group { int G, cap; double us; std::vector<int> list; };
+  std::vector<Group> gs;
+  double span = grid_us(b[0].n, std::min(nsm, grid_max_ctas(b[0].n)), gbs);
+  for (;; span *= 1.05) {
+    gs.clear();
+    int used = 0;
+    bool ok = true;
+    for (int q = 0; q < count && ok; q++) {
+      const int n = b[q].n, lo = grid_min_ctas(n);
+      Group* to = nullptr;
+      for (Group& g : gs)
+        if (!to && g.G >= lo && g.us + grid_us(n, std::min(g.G, grid_max_ctas(n)), gbs) <= span) to = &g;
+      if (!to) {
+        int G = lo;
+        while (G < grid_max_ctas(n) && grid_us(n, G, gbs) > span) G++;
+        ok = grid_us(n, G, gbs) <= span * 1.0001 && used + G <= nsm;
+        if (!ok) break;
+        used += G;
+        gs.push_back(Group{G, grid_max_ctas(n), 0.0, {}});
+        to = &gs.back();
+      }
+      to->us += grid_us(n, to->G, gbs);
+      to->list.push_back(q);
+    }
+    if (!ok) continue;
+    while (used < nsm) {  // the rest
+      Group* slow = nullptr;
+      for (Group& g : gs)
+        if (g.G < g.cap && (!slow || g.us > slow->us)) slow = &g;
+      if (!slow) break;
+      slow->G++;
+      used++;
+      slow->us = 0.0;
+      for (int q : slow->list) slow->us += grid_us(b[q].n, slow->G, gbs);
+    }
+    break;
+  }
+  GridPlan p;
+  for (const Group& g : gs) {
+    p.groups.push_back(GridGroup{p.ctas, g.G, (int)p.jobs.size(), (int)g.list.size()});
+    p.jobs.insert(p.jobs.end(), g.list.begin(), g.list.end());
+    p.ctas += g.G;
+    p.us = std::max(p.us, g.us);
+    for (int q : g.list)
+      p.smem = std::max(p.smem, sizeof(double) * grid_smem_doubles(b[q].ldp, (b[q].n + g.G - 1) / g.G));
+  }
   return p;
 }
 
@@ -2102,6 +2475,7 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
                    ? reinterpret_cast<char*>(take((kPrepGlobalB * (size_t)nb_ + 7) / 8)) : nullptr;
       L.slot = reinterpret_cast<int2*>(take(nb_));
       L.rot = reinterpret_cast<DcRot*>(take(4 * (size_t)nb_));
+      L.gx = take(grid_scratch_doubles(nb_));
       L.info = info_dev + b;
       L.n = nb_;
       if ((int)(t - pos) < nts) {
@@ -2299,6 +2673,8 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
     const StagedGemm gram_g = stage_gemm(img, gram), vt_g = stage_gemm(img, vt);
     std::vector<StagedGemm> bs_g(bsteps.size());
     for (size_t t = 0; t < bsteps.size(); t++) bs_g[t] = stage_gemm(img, bsteps[t]);
+    // room for the grid reduction's groups, jobs and barrier counters (filled when planned)
+    const size_t grid_off = push(img, std::vector<char>(160 * (sizeof(GridGroup) + 128) + sizeof(int) * (size_t)nb + 1024));
     rc = stage_desc(c, img, s);
     if (rc) return rc;
     char* dbase = static_cast<char*>(c->desc);
@@ -2357,7 +2733,32 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
       const int nb1 = nb - nts;
       int nbig = 0;
       while (nbig < nb1 && b1[nbig].n > std::min(cluster_max_n, dsm_max_order())) nbig++;
-      const DsmPlan dp = dsm_plan(b1, nbig, nb1, mid_max_n, nsm);
+      const int nclu = nb1 - nbig;
+      // The larger blocks: by groups of CTAs, beside the clusters with SMs in proportion to the work,
+      // unless there are so many that the streaming kernel runs several CTAs per SM (below). Measured
+      // on B200, reductions in ms by groups / streamed: 40 blocks of order 650-900 12 / 65, 200 56 / 83, 800
+      // 204 / 276 (one per SM), 1400 357 / 230 (three per SM); 40 of order 900-2000 62 / 577; 12 of
+      // order 800-2000 16, 93 by one cluster of 8 or 16 CTAs each; one of order 7049 263, 623 in two
+      // stages (band_min_n).
+      int per_sm = c->tune.reduction_ctas_per_sm;
+      while (per_sm > 1 && (long long)nbig < 3LL * per_sm * nsm) per_sm--;
+      GridPlan gp;
+      int nsm_clu = nsm;
+      if (nbig > 0 && per_sm == 1) {
+        double wg = 0.0, wc = 0.0;
+        int most = 0;
+        for (int q = 0; q < nbig; q++) wg += grid_min_ctas(b1[q].n) * grid_us(b1[q].n, grid_min_ctas(b1[q].n), 30.0);
+        for (int q = nbig; q < nb1; q++) {
+          int C = 1;
+          while (!dsm_fits(b1[q].n, C)) C *= 2;
+          wc += C * dsm_us(b1[q].n, C);
+          most = std::max(most, C);
+        }
+        if (nclu > 0) nsm_clu = std::min(nsm - grid_min_ctas(b1[0].n), std::max(most, (int)(nsm * wc / (wg + wc))));
+        gp = grid_plan(b1, nbig, nsm - (nclu > 0 ? nsm_clu : 0));
+      }
+      const bool grid = gp.ctas > 0;
+      const DsmPlan dp = dsm_plan(b1, nbig, nb1, mid_max_n, nsm_clu, !grid);
       nbig = dp.first;
       // Launches that can run side by side go to streams of their own: the streaming reduction of
       // the largest blocks on s, each cluster size and the one-CTA kernel beside it, largest first
@@ -2377,7 +2778,35 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
       }
       PhaseScope ps(c, kPhTridiag, s, (nbig ? 2 : 0) + (int)ls.size());
       unsigned used = 0;  // side streams with a launch
-      if (nbig) {
+      if (grid) {
+        pack_full_kernel<<<dim3((b1[0].ldp + 31) / 32, (b1[0].n + 31) / 32, nbig), 256, 0, s>>>(d1);
+        NRG_CK(cudaGetLastError());
+        std::vector<char> gi;
+        const size_t go = push(gi, gp.groups), jo = push(gi, gp.jobs),
+                     co = push(gi, std::vector<unsigned>(32 * gp.groups.size(), 0u));
+        if (grid_off + gi.size() > c->desc_size) return fail(NRG_ERR_ARG, "internal: grid descriptors");
+        char* gb = dbase + grid_off;
+        NRG_CK(cudaMemcpyAsync(gb, gi.data(), gi.size(), cudaMemcpyHostToDevice, s));
+        const void* fn = b1[0].n <= 8 * kGridThreads ? (const void*)tridiag_grid_kernel<8> : (const void*)tridiag_grid_kernel<20>;
+        NRG_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gp.smem));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)gp.ctas);
+        cfg.blockDim = dim3(kGridThreads);
+        cfg.dynamicSmemBytes = gp.smem;
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;  // the groups' barriers need all CTAs resident
+        at[0].val.cooperative = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        const LargeBlock* db = d1;
+        const GridGroup* dg = reinterpret_cast<const GridGroup*>(gb + go);
+        int ng = (int)gp.groups.size();
+        const int* dj = reinterpret_cast<const int*>(gb + jo);
+        unsigned* dc = reinterpret_cast<unsigned*>(gb + co);
+        void* kargs[] = {(void*)&db, (void*)&dg, (void*)&ng, (void*)&dj, (void*)&dc};
+        NRG_CK(cudaLaunchKernelExC(&cfg, fn, kargs));
+      } else if (nbig) {
         auto tri_bytes = [&](int st) {
           return 1024 + sizeof(double) * ((size_t)kTriWarps * st * kSlabD + 2 * (size_t)b1[0].n +
                                           (size_t)kTriWarps * 2 * NB + 2 * NB + 64);
@@ -2385,9 +2814,6 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
         const CUtensorMap* tm = reinterpret_cast<const CUtensorMap*>(dbase + tmap_off) + nts;
         pack_lower_kernel<<<dim3((b1[0].n + 7) / 8, nbig), 256, 0, s>>>(d1);
         NRG_CK(cudaGetLastError());
-        // Few large blocks: one cluster of kTclC CTAs per block, when the clusters fill at most
-        // about two waves of the SMs and the device can hold one such cluster at a time.
-        bool tcl = false;
         // reduction_ctas_per_sm (nrg_tuning) sets how many CTAs of the streaming kernel share an
         // SM: one, when each requests at least half of an SM's shared memory; two, with four
         // slabs in flight per warp; three (the default), with two slabs per warp and at most 168
@@ -2396,58 +2822,10 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
         // leave no room for that many, the next smaller count is used. Several per SM once gave
         // wrong reductions through a race on alpha = v[k+1] in the reflector step (alpha was read
         // after a barrier that a thread overwriting it could pass); alpha is now read before that
-        // barrier, and batches with more of these CTAs than SMs pass every check on B200. The
-        // cluster kernel's ring gets 8, 6 or 4 slabs per warp, the most that fit.
-        int smsm = 0, optin = 0;
+        // barrier, and batches with more of these CTAs than SMs pass every check on B200.
+        int smsm = 0;
         cudaDeviceGetAttribute(&smsm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c->device);
-        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-        // The cluster kernel serves few blocks (latency): its CTAs keep an SM each, whatever
-        // reduction_ctas_per_sm says for the streaming kernel of the throughput regime.
-        auto tcl_bytes = [&](int st) {
-          return std::max(1024 + sizeof(double) * ((size_t)kTriWarps * st * kSlabD + 2 * (size_t)b1[0].n +
-                                                   (size_t)kTriWarps * 2 * NB + 4 * NB + 66),
-                          (size_t)smsm / 2 + 1024);
-        };
-        int stages = 8;
-        while (stages > 4 && tcl_bytes(stages) + 256 > (size_t)optin) stages -= 2;
-        const size_t smem_tcl = tcl_bytes(stages);
-        const void* tcl_fn = stages == 8 ? (const void*)tridiag_tcl_kernel<8>
-                             : stages == 6 ? (const void*)tridiag_tcl_kernel<6> : (const void*)tridiag_tcl_kernel<4>;
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute at[1];
-        if ((long long)nbig * kTclC <= 2LL * nsm && smem_tcl + 256 <= (size_t)optin) {
-          NRG_CK(cudaFuncSetAttribute(tcl_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_tcl));
-          NRG_CK(cudaFuncSetAttribute(tcl_fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-          cfg.blockDim = dim3(kTriThreads);
-          cfg.dynamicSmemBytes = smem_tcl;
-          cfg.stream = s;
-          at[0].id = cudaLaunchAttributeClusterDimension;
-          at[0].val.clusterDim.y = 1;
-          at[0].val.clusterDim.z = 1;
-          cfg.attrs = at;
-          cfg.numAttrs = 1;
-          // 16 CTAs per block when the blocks are few enough for all their clusters to be active
-          // at once, else 8
-          for (int C : {2 * kTclC, kTclC}) {
-            if (C > kTclC && (long long)nbig * C > nsm) continue;
-            cfg.gridDim = dim3((unsigned)(nbig * C));
-            at[0].val.clusterDim.x = (unsigned)C;
-            int ncl = 0;
-            if (cudaOccupancyMaxActiveClusters(&ncl, tcl_fn, &cfg) != cudaSuccess) {
-              cudaGetLastError();
-              ncl = 0;
-            }
-            if (C > kTclC ? ncl >= nbig : ncl > 0) {
-              tcl = true;
-              break;
-            }
-          }
-        }
-        if (tcl) {
-          const LargeBlock* db = d1;
-          void* kargs[] = {(void*)&db, (void*)&tm};
-          NRG_CK(cudaLaunchKernelExC(&cfg, tcl_fn, kargs));
-        } else {
+        {
           // one, two or three CTAs per SM as above (1 KB of shared memory is reserved per CTA);
           // reduction_ctas_per_sm is the most, used when the batch fills at least three waves of
           // that many CTAs per SM. A batch of fewer large blocks is bound by its largest ones,
@@ -2455,8 +2833,6 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
           // 1500 blocks of order 8-2048, about 330 of them streamed, take 873 ms with one CTA
           // per SM, 909 with two, 1015 with three; the benchmark's 10,000 blocks run 6.5% faster
           // with three than with two).
-          int per_sm = c->tune.reduction_ctas_per_sm;
-          while (per_sm > 1 && (long long)nbig < 3LL * per_sm * nsm) per_sm--;
           if (per_sm == 3 && 3 * (tri_bytes(2) + 1024) > (size_t)smsm) per_sm = 2;
           if (per_sm == 2 && 2 * (tri_bytes(4) + 1024) > (size_t)smsm) per_sm = 1;
           if (per_sm == 3) {

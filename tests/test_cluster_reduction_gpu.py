@@ -75,3 +75,14 @@ def test_one_cta_solver_orders(nb, oracle, scale):
             check_eig(h, g.val, g.vec, w, v, oracle)
         else:  # check_eig's norms underflow or overflow; the scaled problem is the same one
             check_eig(h / scale, g.val / scale, g.vec, w / scale, v, oracle)
+
+
+@pytest.mark.parametrize("sizes", [[601], [625, 640, 703], [768, 1025, 1300], [608] * 60 + [801]])
+def test_group_reduction(nb, oracle, sizes):
+    """The reduction by groups of CTAs: one block over the whole chip, several beside one another and
+    beside clusters, more blocks than groups (a queue each); panel remainders, decoupled halves."""
+    blocks = blocks_of(sizes + [300, 70], 5)
+    got = nb.diagonalisations(blocks)
+    for k in {0, 1, len(sizes) // 2, len(sizes) - 1, len(sizes)}:
+        w, v = oracle.diagonalise(blocks[k])
+        check_eig(blocks[k], got[k].val, got[k].vec, w, v, oracle)
