@@ -64,21 +64,21 @@ NRG_API int nrg_trim(nrg_ctx* ctx);
 
 /* Launch parameters of the batched eigensolver, chosen per device by the autotuner
  * (nrgljubljana_b200/autotune.py) from timed sweeps; the defaults are its result on B200.
- *   small_max_n    blocks up to this order are solved whole in the shared memory of one
- *                  CTA (32..96)
- *   mid_max_n      larger blocks up to this order are reduced to tridiagonal form in the
- *                  shared memory of one CTA (small_max_n..236)
+ *   small_max_n    blocks up to this order are solved whole by one CTA (32..96)
+ *   mid_max_n      in batches of many blocks, larger ones up to this order are reduced to
+ *                  tridiagonal form in the shared memory of one CTA (small_max_n..236)
  *   cluster_max_n  larger blocks up to this order are reduced in the distributed shared
- *                  memory of a thread-block cluster when the clusters fit the SMs at once
- *                  (mid_max_n..640); larger blocks stream their trailing matrix from HBM
+ *                  memory of a thread-block cluster of 1 to 16 CTAs (mid_max_n..640);
+ *                  larger ones by groups of CTAs through L2, or, when they are many, by the
+ *                  streaming reduction with several CTAs per SM
  *   reduction_ctas_per_sm  most CTAs of the streaming reduction kernel per SM (1, 2 or 3;
- *                  default 3), used when the batch's streamed blocks fill three waves of them
- *                  (fewer otherwise: a batch of few large blocks is bound by its largest)
+ *                  default 3); it serves batches whose larger blocks fill three waves of at
+ *                  least two of them per SM
  *   band_min_n     blocks of at least this order, when at most band_max_blocks of them are
  *                  in a batch, take the two-stage reduction (dense -> band on the FP64
- *                  tensor cores, band -> tridiagonal by bulge chasing); 0 = never; default 3072
- *   band_max_blocks  see band_min_n (few large blocks: the regime where the one-stage
- *                  reduction's per-column chain bounds the step); default 64 */
+ *                  tensor cores, band -> tridiagonal by bulge chasing); 0 = never, the
+ *                  default: the reduction by groups of CTAs is faster at every order measured
+ *   band_max_blocks  see band_min_n; default 64 */
 typedef struct nrg_tuning {
   int small_max_n;
   int mid_max_n;

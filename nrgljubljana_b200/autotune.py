@@ -1,10 +1,10 @@
 """Autotuner of the batched eigensolver's launch parameters (nrg_tuning, include/nrg_b200.h).
 
 The eigensolver sends each block of a step down one of four paths by its order: the
-one-CTA shared-memory solver (n <= small_max_n), the one-CTA shared-memory tridiagonal
-reduction (n <= mid_max_n), the cluster reduction in distributed shared memory
-(n <= cluster_max_n, when the clusters fit the SMs at once) and the streaming reduction
-from HBM, whose CTAs run one, two or three per SM (reduction_ctas_per_sm). Where the crossovers
+one-CTA solver (n <= small_max_n), the reduction in the shared memory of one CTA or of a
+cluster (n <= cluster_max_n; one CTA up to mid_max_n in large batches), the reduction by groups of
+CTAs through L2 and, for many large blocks, the streaming reduction from HBM, whose CTAs run two or
+three per SM (reduction_ctas_per_sm). Where the crossovers
 lie depends on the device, so they are measured, not assumed: the reference's own
 scheduler (c++/core.hpp:98-107, c++/subspaces.hpp:103-123) only orders the blocks largest
 first; on a GPU the choice of path per block is the equivalent decision.
@@ -47,10 +47,9 @@ GRID = {
     "small_max_n": [32, 48, 64, 80, 96],
     "mid_max_n": [128, 160, 192, 224, 236],
     "cluster_max_n": [400, 480, 560, 600, 640],
-    # The two-stage path's bulge chasing has a critical path of about 3n dependent steps; below
-    # order ~2000 it is as long as the block's one-stage reduction, so lower thresholds only
-    # pay where the other blocks of a batch hide it, and cost 10-15% on keep-4000 Anderson
-    # steps (blocks up to 1622), measured.
+    # The two-stage path's bulge chasing has a critical path of about 3n dependent steps; the
+    # reduction by groups of CTAs overtakes it at every order measured (a step of 24 blocks in
+    # [200, 7049] takes 468 ms, 663 with the blocks from 3072 on in two stages).
     "band_min_n": [0, 2048, 3072, 4096],
     "reduction_ctas_per_sm": [1, 2, 3],
     "band_max_blocks": [4, 8, 16, 32, 64],
