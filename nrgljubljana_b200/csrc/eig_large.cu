@@ -67,7 +67,9 @@ struct LargeBlock {
   double* lam;    // eigenvalues of the current divide-and-conquer nodes
   double* dsort;  // per node: non-deflated poles, ascending
   double* dgrp;   // per node: non-deflated poles, grouped order
-  double* zgrp;   // per node: z in grouped order
+  double* zgrp;   // per node: z in grouped order; then z-hat
+  double* rorg;   // per node: root j is rorg[j] + rtau[j], rorg the pole it was measured from
+  double* rtau;
   double* GT;     // per back-transform panel of nb reflectors: Gram matrix V^T V then T (nb x nb each)
   int* rank;      // per node: sorted position of grouped entry
   int* perm;      // final eigenvalue order
@@ -1890,17 +1892,20 @@ NRG_DEV void dc_move_rows(const LargeBlock& B, const DcNode& nd, const DcState& 
 
 // ---------------------------------------------------------------- divide and conquer: secular equation
 // Root j of 1 + rho sum_i z_i^2 / (d_i - lambda) = 0 with poles d ascending. One warp per
-// root, lanes over i. On exit Dt[j][g] = d_g - lambda_j for every grouped entry g. The CTAs
-// blockIdx.y >= ysec move the node's eigenvector rows beside it (dc_move_rows).
+// root, lanes over i. The root is left as the pole it was measured from and the distance, which
+// give d_g - lambda_j without cancellation wherever it is needed. The CTAs blockIdx.y >= ysec move
+// the node's eigenvector rows beside it (dc_move_rows).
 // The iteration starts from the root of the two-pole model that the midpoint's values give, and
 // the last root, which lies right of every pole, takes the model's root on that side: the other
 // one is outside the bracket, and bisection in its place took 45-100 steps (the longest warp of
 // the launch) where now every root takes at most ten.
-// Measured on B200, 40 blocks up to order 480 (4 levels): 0.59 ms before, 0.14 ms now with the
-// row moves in it.
-__global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __restrict__ blocks,
-                                                         const DcNode* __restrict__ nodes,
-                                                         const DcState* __restrict__ states, int ysec) {
+// The divisions bound it, two per pole and step, so warps in flight count: four CTAs per SM.
+// Measured on B200 with the row moves in it: 40 blocks up to order 480 (4 levels) 0.095 ms, from 0.59
+// with bisections and 0.104 with two CTAs per SM and the K x K matrix of d_g - lambda_j written
+// for the kernels below; 2192 blocks of orders 147-200 21.6 ms, from 37.6 (one CTA per SM: 56).
+__global__ void __launch_bounds__(256, 4) dc_secular_kernel(const LargeBlock* __restrict__ blocks,
+                                                            const DcNode* __restrict__ nodes,
+                                                            const DcState* __restrict__ states, int ysec) {
   const DcNode nd = nodes[blockIdx.x];
   const DcState st = states[blockIdx.x];
   const LargeBlock B = blocks[nd.blk];
@@ -1910,7 +1915,7 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __res
   }
   const int K = st.K;
   if (K == 0) return;
-  const int n = B.n, a = nd.a;
+  const int a = nd.a;
   const double rho = st.rho;
   const int lane = threadIdx.x & 31;
   const int wg = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1919,14 +1924,14 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __res
   const double* dg = B.dgrp + a;
   const double* zg = B.zgrp + a;
   const int* rk = B.rank + a;
-  double* Dt = B.evecs + (size_t)a * n + a;
   for (int j = wg; j < K; j += wstride) {
     double dorg, lo, hi, tau;
     int p1, p2;
     if (K == 1) {
       const double z = zg[0];
       if (lane == 0) {
-        Dt[0] = -rho * z * z;
+        B.rorg[a] = ds[0];
+        B.rtau[a] = rho * z * z;
         B.lam[a] = ds[0] + rho * z * z;
       }
       continue;
@@ -1994,18 +1999,23 @@ __global__ void __launch_bounds__(256) dc_secular_kernel(const LargeBlock* __res
       if (tn == tau) break;
       tau = tn;
     }
-    for (int i = lane; i < K; i += 32) Dt[(size_t)j * n + i] = (dg[i] - dorg) - tau;
-    if (lane == 0) B.lam[a + j] = dorg + tau;
+    if (lane == 0) {
+      B.rorg[a + j] = dorg;
+      B.rtau[a + j] = tau;
+      B.lam[a + j] = dorg + tau;
+    }
   }
 }
 
 // ---------------------------------------------------------------- divide and conquer: vectors
-// z-hat by the Gu-Eisenstat product formula (into dgrp, free after the secular solve), then
-// u_j(g) = zhat_g / (d_g - lambda_j), normalised, written over Dt in place (same grouped
-// column order). Both kernels spread a node over gridDim.y CTAs.
+// z-hat by the Gu-Eisenstat product formula (into zgrp, free after the secular solve), then
+// u_j(g) = zhat_g / (d_g - lambda_j), normalised, in grouped column order. Both kernels spread a
+// node over gridDim.y CTAs, and form d_g - lambda_j from the poles and (rorg, rtau): that they need no
+// matrix of these, and one division per entry, brought 2192 blocks of orders 147-200 from 16.2 to
+// 12.0 ms.
 // A CTA takes 32 columns g and splits the product over the roots between its eight warps (the
 // chain of K dependent multiplications and divisions was the whole time of small batches: 0.52 ms
-// of a step of 40 blocks up to order 480 with one thread per column, both kernels, 0.12 ms now).
+// of a step of 40 blocks up to order 480 with one thread per column, both kernels, 0.077 ms now).
 __global__ void __launch_bounds__(256) dc_zhat_kernel(const LargeBlock* __restrict__ blocks,
                                                       const DcNode* __restrict__ nodes,
                                                       const DcState* __restrict__ states) {
@@ -2016,16 +2026,17 @@ __global__ void __launch_bounds__(256) dc_zhat_kernel(const LargeBlock* __restri
   const int g = blockIdx.y * 32 + lane;
   if ((int)blockIdx.y * 32 >= K) return;  // uniform over the CTA
   const LargeBlock B = blocks[nd.blk];
-  const int n = B.n, a = nd.a;
+  const int a = nd.a;
   const double* ds = B.dsort + a;
-  const double* Dt = B.evecs + (size_t)a * n + a;
+  const double* og = B.rorg + a;
+  const double* rt = B.rtau + a;
   double p = 1.0;
   if (g < K) {
     const int i = B.rank[a + g];
     const double di = ds[i];
 #pragma unroll 4
-    for (int j = warp; j < K - 1; j += 8) p *= -Dt[(size_t)j * n + g] / (ds[j < i ? j : j + 1] - di);
-    if (warp == 0) p *= -Dt[(size_t)(K - 1) * n + g] / st.rho;
+    for (int j = warp; j < K - 1; j += 8) p *= -((di - og[j]) - rt[j]) / (ds[j < i ? j : j + 1] - di);
+    if (warp == 0) p *= -((di - og[K - 1]) - rt[K - 1]) / st.rho;
   }
   part[warp][lane] = p;
   __syncthreads();
@@ -2033,7 +2044,7 @@ __global__ void __launch_bounds__(256) dc_zhat_kernel(const LargeBlock* __restri
     double q = 1.0;
 #pragma unroll
     for (int v = 0; v < 8; v++) q *= part[v][lane];
-    B.dgrp[a + g] = copysign(sqrt(fabs(q)), B.zgrp[a + g]);
+    B.zgrp[a + g] = copysign(sqrt(fabs(q)), B.zgrp[a + g]);
   }
 }
 
@@ -2050,17 +2061,34 @@ __global__ void __launch_bounds__(256) dc_vectors_kernel(const LargeBlock* __res
   // deflated rows are final: grouped copy (W2) back to the node's rows a+K.. (H)
   for (int r = a + K + wg; r < nd.b; r += wstride)
     for (int col = a + lane; col < nd.b; col += 32) B.H[(size_t)r * n + col] = B.W2[(size_t)r * n + col];
-  const double* zh = B.dgrp + a;
-  double* Dt = B.evecs + (size_t)a * n + a;
+  const double* zh = B.zgrp + a;
+  const double* dg = B.dgrp + a;
   for (int j = wg; j < K; j += wstride) {
-    double* row = Dt + (size_t)j * n;
-    double ss = 0.0;
-    for (int g = lane; g < K; g += 32) {
-      const double u = zh[g] / row[g];
-      ss = fma(u, u, ss);
+    double* row = B.evecs + (size_t)(a + j) * n + a;
+    const double og = B.rorg[a + j], rt = B.rtau[a + j];
+    constexpr int U = 16;  // entries a lane keeps between the norm and the scaled store
+    double u[U], ss = 0.0;
+#pragma unroll
+    for (int q = 0; q < U; q++) {
+      if (32 * q >= K) break;
+      const int g = lane + 32 * q;
+      u[q] = g < K ? zh[g] / ((dg[g] - og) - rt) : 0.0;
+      ss = fma(u[q], u[q], ss);
+    }
+#pragma unroll 4
+    for (int g = lane + 32 * U; g < K; g += 32) {
+      const double x = zh[g] / ((dg[g] - og) - rt);
+      ss = fma(x, x, ss);
     }
     const double inv = 1.0 / sqrt(warp_sum(ss));
-    for (int g = lane; g < K; g += 32) row[g] = zh[g] / row[g] * inv;
+#pragma unroll
+    for (int q = 0; q < U; q++) {
+      if (32 * q >= K) break;
+      const int g = lane + 32 * q;
+      if (g < K) row[g] = u[q] * inv;
+    }
+#pragma unroll 4
+    for (int g = lane + 32 * U; g < K; g += 32) row[g] = zh[g] / ((dg[g] - og) - rt) * inv;
   }
 }
 
@@ -2221,7 +2249,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 size_t large_block_doubles(int n, bool two_stage) {
   const size_t ldp = (size_t)(n + 31) / 32 * 32;
-  return (size_t)n * ldp + (size_t)n * n + 8 * (size_t)n + 2 * (size_t)NBT * n + 7 * (size_t)n + 64 * 16 + grid_scratch_doubles(n) +
+  return (size_t)n * ldp + (size_t)n * n + 8 * (size_t)n + 2 * (size_t)NBT * n + 9 * (size_t)n + 64 * 18 + grid_scratch_doubles(n) +
          (prep_layout(n).total > kPrepSmemMax ? (kPrepGlobalB * (size_t)n + 7) / 8 : 0) +
          (two_stage ? band_extra_doubles(n) + 4 * 64 : 0);
 }
@@ -2466,6 +2494,8 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
       L.dsort = take(nb_);
       L.dgrp = take(nb_);
       L.zgrp = take(nb_);
+      L.rorg = take(nb_);
+      L.rtau = take(nb_);
       L.npanel = (nb_ - 2 + NBT - 1) / NBT;
       L.GT = take(2 * (size_t)NBT * nb_);  // >= sum over panels of 2 nb^2
       int* ip = reinterpret_cast<int*>(take(nb_));
