@@ -95,7 +95,8 @@ struct DcNode {
 struct DcState {
   int K, k1, k2, k3;
   double rho;
-  int nrot, pad;
+  int nrot;
+  int ex;  // poles, rho and roots of the merge are divided by 2^ex (about the size of the merged matrix)
 };
 
 // ---------------------------------------------------------------- tridiagonalisation
@@ -1704,6 +1705,9 @@ __global__ void __launch_bounds__(512) dc_prep_kernel(const LargeBlock* __restri
   zmx = block_max(zmx, red);
   const double tol = 8.0 * kEps * fmax(dmx, rho * zmx);  // relative to the merged matrix
   const bool none = rho * zmx <= tol;  // nothing couples the children
+  // the secular equation in units in which squares neither overflow nor underflow
+  const int ex = min(1000, max(-1000, ilogb(fmax(dmx, rho))));
+  const double sc = scalbn(1.0, -ex);
   // 3. deflation of small couplings; the rest in order. Thread t has the positions [s0, s1).
   const int per = (N + nt - 1) / nt, s0 = min(N, tid * per), s1 = min(N, s0 + per);
   unsigned long long total;
@@ -1796,9 +1800,9 @@ __global__ void __launch_bounds__(512) dc_prep_kernel(const LargeBlock* __restri
       const int t = g1 + g2 + g3;  // rank among the non-deflated poles
       g = f == 1 ? g1++ : f == 3 ? k1 + g2++ : k1 + k2 + g3++;
       B.rank[a + g] = t;
-      B.dgrp[a + g] = key[s];
+      B.dgrp[a + g] = key[s] * sc;
       B.zgrp[a + g] = zs[s];
-      B.dsort[a + t] = key[s];
+      B.dsort[a + t] = key[s] * sc;
     }
     B.slot[a + sidx[s]] = make_int2(g, f & 3);
   }
@@ -1808,9 +1812,9 @@ __global__ void __launch_bounds__(512) dc_prep_kernel(const LargeBlock* __restri
     st.k1 = k1;
     st.k2 = k2;
     st.k3 = k3;
-    st.rho = rho;
+    st.rho = rho * sc;
     st.nrot = s_nrot;
-    st.pad = 0;
+    st.ex = ex;
     states[blockIdx.x] = st;
     // the two merge GEMMs: rows of child-1 columns from types 1+2, child-2 columns from 2+3
     gouts[nd.gout].M = K;
@@ -1902,7 +1906,7 @@ NRG_DEV void dc_move_rows(const LargeBlock& B, const DcNode& nd, const DcState& 
 // The divisions bound it, two per pole and step, so warps in flight count: four CTAs per SM.
 // Measured on B200 with the row moves in it: 40 blocks up to order 480 (4 levels) 0.095 ms, from 0.59
 // with bisections and 0.104 with two CTAs per SM and the K x K matrix of d_g - lambda_j written
-// for the kernels below; 2192 blocks of orders 147-200 21.6 ms, from 37.6 (one CTA per SM: 56).
+// for the kernels below; 1400 blocks of order 601-900 21.6 ms, from 37.6 (one CTA per SM: 56).
 __global__ void __launch_bounds__(256, 4) dc_secular_kernel(const LargeBlock* __restrict__ blocks,
                                                             const DcNode* __restrict__ nodes,
                                                             const DcState* __restrict__ states, int ysec) {
@@ -1932,7 +1936,7 @@ __global__ void __launch_bounds__(256, 4) dc_secular_kernel(const LargeBlock* __
       if (lane == 0) {
         B.rorg[a] = ds[0];
         B.rtau[a] = rho * z * z;
-        B.lam[a] = ds[0] + rho * z * z;
+        B.lam[a] = scalbn(ds[0] + rho * z * z, st.ex);
       }
       continue;
     }
@@ -2002,7 +2006,7 @@ __global__ void __launch_bounds__(256, 4) dc_secular_kernel(const LargeBlock* __
     if (lane == 0) {
       B.rorg[a + j] = dorg;
       B.rtau[a + j] = tau;
-      B.lam[a + j] = dorg + tau;
+      B.lam[a + j] = scalbn(dorg + tau, st.ex);
     }
   }
 }
@@ -2011,7 +2015,7 @@ __global__ void __launch_bounds__(256, 4) dc_secular_kernel(const LargeBlock* __
 // z-hat by the Gu-Eisenstat product formula (into zgrp, free after the secular solve), then
 // u_j(g) = zhat_g / (d_g - lambda_j), normalised, in grouped column order. Both kernels spread a
 // node over gridDim.y CTAs, and form d_g - lambda_j from the poles and (rorg, rtau): that they need no
-// matrix of these, and one division per entry, brought 2192 blocks of orders 147-200 from 16.2 to
+// matrix of these, and one division per entry, brought 1400 blocks of order 601-900 from 16.2 to
 // 12.0 ms.
 // A CTA takes 32 columns g and splits the product over the roots between its eight warps (the
 // chain of K dependent multiplications and divisions was the whole time of small batches: 0.52 ms
