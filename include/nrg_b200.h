@@ -69,11 +69,10 @@ NRG_API int nrg_trim(nrg_ctx* ctx);
  *                  tridiagonal form in the shared memory of one CTA (small_max_n..236)
  *   cluster_max_n  larger blocks up to this order are reduced in the distributed shared
  *                  memory of a thread-block cluster of 1 to 16 CTAs (mid_max_n..640);
- *                  larger ones by groups of CTAs through L2, or, when they are many, by the
- *                  streaming reduction with several CTAs per SM
- *   reduction_ctas_per_sm  most CTAs of the streaming reduction kernel per SM (1, 2 or 3;
- *                  default 3); it serves batches whose larger blocks fill three waves of at
- *                  least two of them per SM
+ *                  larger ones by groups of CTAs through L2; in batches of many blocks
+ *                  the streaming reduction, two CTAs per SM, takes those above mid_max_n
+ *                  that it finishes in the time the batch needs
+ *   reduction_ctas_per_sm  1: the streaming reduction is not used; 2 or 3 (default): it is
  *   band_min_n     blocks of at least this order, when at most band_max_blocks of them are
  *                  in a batch, take the two-stage reduction (dense -> band on the FP64
  *                  tensor cores, band -> tridiagonal by bulge chasing); 0 = never, the

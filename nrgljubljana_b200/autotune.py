@@ -3,9 +3,8 @@
 The eigensolver sends each block of a step down one of four paths by its order: the
 one-CTA solver (n <= small_max_n), the reduction in the shared memory of one CTA or of a
 cluster (n <= cluster_max_n; one CTA up to mid_max_n in large batches), the reduction by groups of
-CTAs through L2 and, for many large blocks, the streaming reduction from HBM, whose CTAs run two or
-three per SM (reduction_ctas_per_sm). Where the crossovers
-lie depends on the device, so they are measured, not assumed: the reference's own
+CTAs through L2 and, in batches of many blocks, the streaming reduction from HBM (not used with
+reduction_ctas_per_sm = 1). Where the crossovers lie depends on the device, so they are measured, not assumed: the reference's own
 scheduler (c++/core.hpp:98-107, c++/subspaces.hpp:103-123) only orders the blocks largest
 first; on a GPU the choice of path per block is the equivalent decision.
 

@@ -5,12 +5,10 @@
 // of copy_results (ascending eigenvalues, eigenvectors as rows, c++/diag.hpp:41-58).
 //
 // Pipeline per chunk of blocks (all blocks of the chunk advance together):
-//   1. reduction to tridiagonal form, one of several by order and number of the blocks (in
-//      shared memory, by groups of CTAs through L2, in two stages, or, for many large blocks,)
-//      tridiag_kernel     one CTA per block: blocked Householder reduction A = Q T Q^T
-//                         (panel width NB); the symmetric matrix-vector product streams
-//                         the lower triangle from HBM once per column, the panel update
-//                         is a rank-2NB update of the trailing lower triangle.
+//   1. reduction to tridiagonal form A = Q T Q^T by Householder reflectors, several kernels side by
+//      side by order and number of the blocks (reduction_plan): in the shared memory of a CTA or
+//      a cluster, by groups of CTAs through L2, in two stages (eig_band.cu), or, in batches of many
+//      blocks, one CTA per block streaming the lower triangle once per column (tridiag_kernel).
 //   2. divide and conquer on T: leaves (<= kLeaf) by one in shared memory, merges
 //      by rank-one tearing (Cuppen), deflation (small z and close poles with Givens
 //      rotations), secular-equation roots with a two-pole rational model safeguarded by
@@ -101,36 +99,28 @@ struct DcState {
 
 // ---------------------------------------------------------------- tridiagonalisation
 
-// Column sums of an 8-column slab: lane l holds x[c] = A(i_l, j0+c) * v[i_l]; returns, in
-// every lane, the sum over all 32 lanes of x[c] for c = (l >> 2) & 7 (9 shuffles).
-NRG_DEV double slab_colsum8(double (&x)[8], int lane) {
-  {
-    const bool up = (lane & 16) != 0;
+// block_sum_1b with warp_sum_mma for both levels (at most 32 warps).
+NRG_DEV double block_sum_mma(double x, double* red, int& phase) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  x = warp_sum_mma(x);
+  double* b = red + 32 * (phase & 1);
+  phase++;
+  if (lane == 0) b[wid] = x;
+  __syncthreads();
+  return warp_sum_mma(lane < nw ? b[lane] : 0.0);
+}
+
+// The sum over all lanes of x[c] for c = lane / 4, by DMMAs: a matrix with a one in row c and its product
+// with the lanes' x[c] put the sums over the lanes of equal l/4 into row c; a last one sums each row.
+NRG_DEV double colsum8_mma(const double (&x)[8], int lane) {
+  double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0, e0 = 0.0, e1 = 0.0;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const double send = up ? x[q] : x[q + 4];
-      const double keep = up ? x[q + 4] : x[q];
-      x[q] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-    }
+  for (int c = 0; c < 8; c += 2) {
+    dmma884(a0, a1, lane >> 2 == c ? 1.0 : 0.0, x[c]);
+    dmma884(b0, b1, lane >> 2 == c + 1 ? 1.0 : 0.0, x[c + 1]);
   }
-  {
-    const bool up = (lane & 8) != 0;
-#pragma unroll
-    for (int q = 0; q < 2; q++) {
-      const double send = up ? x[q] : x[q + 2];
-      const double keep = up ? x[q + 2] : x[q];
-      x[q] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-    }
-  }
-  {
-    const bool up = (lane & 4) != 0;
-    const double send = up ? x[0] : x[1];
-    const double keep = up ? x[1] : x[0];
-    x[0] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-  }
-  x[0] += __shfl_xor_sync(0xffffffffu, x[0], 2);
-  x[0] += __shfl_xor_sync(0xffffffffu, x[0], 1);
-  return x[0];
+  dmma884(e0, e1, (a0 + a1) + (b0 + b1), 1.0);
+  return e0;
 }
 
 // ---- bulk asynchronous copies (TMA, non-multicast) into the CTA's own shared memory
@@ -147,6 +137,9 @@ NRG_DEV void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
 // Orders this thread's earlier generic-proxy global writes before later bulk (async-proxy)
 // reads of the same memory.
 NRG_DEV void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+
+// Orders this thread's earlier generic-proxy accesses of shared memory before later bulk copies into it.
+NRG_DEV void fence_proxy_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 NRG_DEV void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 
@@ -174,18 +167,9 @@ NRG_DEV bool mbar_wait(uint64_t* bar, unsigned parity, int bound = (1 << 26)) {
 }
 
 // 2-D bulk tensor copy (TMA, non-multicast) of one box at coordinates (x, y) into this
-// CTA's shared memory, completing on an mbarrier.
-NRG_DEV void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-          smem_u32(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// The same with an L2 eviction-priority hint (an access policy from createpolicy): the slabs of
-// a trailing triangle that is streamed once per column and does not fit in L2 go first, so
-// that the panel's vectors (read three times per column) stay.
+// CTA's shared memory, completing on an mbarrier, with an L2 eviction-priority hint (an access policy
+// from createpolicy): the slabs of a trailing triangle that is streamed once per column and does not
+// fit in L2 go first, so that the panel's vectors (read twice per column) stay.
 NRG_DEV void tma_load_2d_hint(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar, uint64_t policy) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, "
@@ -200,7 +184,7 @@ NRG_DEV uint64_t l2_evict_first_policy() {
   return p;
 }
 
-// Loads and stores of the panel's vectors (V and W columns, re-read three times per column of
+// Loads and stores of the panel's vectors (V and W columns, re-read twice per column of
 // the panel) with an evict-last L2 hint, so that the streamed slabs do not push them out.
 NRG_DEV uint64_t l2_evict_last_policy() {
   uint64_t p;
@@ -216,128 +200,147 @@ NRG_DEV void st_keep(double* a, double v, uint64_t pol) {
   asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(a), "d"(v), "l"(pol) : "memory");
 }
 
-constexpr int kStages = 4;                 // slabs in flight per warp
+constexpr int kTriStages = 3;              // slabs in flight per warp
 constexpr int kSlabRows = 64;              // rows of a slab (two per lane)
 constexpr int kSlabD = kSlabRows * 8;      // doubles per slab: 64 rows x 8 columns
 constexpr int kTriWarps = kTriThreads / 32;
 
-// y[i] += sum_{j >= s0} A(i, j) v[j] for s0 <= i < n. A is the packed lower triangle
-// (A(i, j) = P[j*ld + i] for i >= j, zero above the diagonal and in the padding) behind the
-// 2-D tensor map `tmap` (inner extent ld rows, outer extent n columns, box 64 x 8). The
-// triangle is cut into 64-row x 8-column slabs; the slabs, in tile-row order, are split
-// evenly between the warps, and each warp streams its slabs through a ring of kStages
-// shared-memory buffers, one TMA box copy per slab completing on the buffer's mbarrier.
-// A lane owns rows l and l+32 of the slab: row sums stay in registers until the tile row
-// changes, column sums are transposed across the warp; both are added to y (shared memory).
-// `parity` holds the warp's mbarrier phase bits across calls.
-// gwarp / gnwarps: this warp's index among the warps that share the product (the warps of
-// one CTA, or of every CTA of a cluster), and their number; y receives this warp's part.
-template <int STAGES = kStages, bool EVICT_FIRST = false>
-NRG_DEV void symv_lower(const CUtensorMap* tmap, int n, int s0, const double* v, double* y, double* ring,
-                        uint64_t* bars, unsigned& parity, int* err, int gwarp, int gnwarps) {
+// Length of a vector of the product: the last slab of a column group may end this far below row n-1.
+__host__ __device__ inline int tri_pad(int n) { return (n + 7) / 8 * 8 + kSlabRows; }
+
+// y += A(s0:n, s0:n) v, with v(s0) replaced by vs. A is the packed lower triangle (A(i, j) =
+// P[j*ld + i] for i >= j, zero above the diagonal and in the padding) behind the 2-D tensor map `tmap`
+// (inner extent ld rows, outer extent n columns, box 64 x 8). The triangle is cut into slabs of 64 rows
+// x 8 columns, those of a column group from its diagonal down (slabs of aligned rows read a tenth more at
+// order 900); the slabs, column group by column group, are split evenly between the warps, and each warp
+// streams its slabs through a ring of kTriStages shared-memory buffers, one TMA box copy per slab
+// completing on the buffer's mbarrier. A lane owns rows l and l+32 of the slab. A column group's sums stay
+// in registers down the group and cross the lanes once at its end; the row sums are added in
+// each slab to the warp's own copy of y, which takes no shuffles (walking along the rows instead costs a
+// transposed sum of 8 columns and shared-memory atomics in every slab). y has ny copies of vp numbers,
+// one per warp or else (large orders) shared by pairs of warps with atomics; v is zero in n .. vp-1.
+// Rows of y before s0 take sums that nothing reads.
+// `parity` holds the warp's mbarrier phase bits across calls. `between` is called while the first
+// copies are under way.
+template <typename F>
+NRG_DEV void symv_lower(const CUtensorMap* tmap, int n, int s0, const double* v, double vs, double* y, int ny, int vp,
+                        double* ring, uint64_t* bars, unsigned& parity, int* err, uint64_t policy, const F& between) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int T0 = s0 >> 6, Tn = (n - 1) >> 6, sl0 = s0 >> 3, slmax = (n - 1) >> 3;
-  auto rowlen = [&](int I) { return min(8 * I + 7, slmax) - sl0 + 1; };
-  long long S = 0;
-  for (int I = T0; I <= Tn; I++) S += rowlen(I);
-  const long long f0 = S * gwarp / gnwarps, f1 = S * (gwarp + 1) / gnwarps;
-  if (f0 >= f1) return;
-  double* myring = ring + (size_t)warp * STAGES * kSlabD;
-  uint64_t* mybar = bars + warp * STAGES;
-  auto advance = [&](int& I_, int& sl_) {
-    if (sl_ < min(8 * I_ + 7, slmax)) {
-      sl_++;
+  // column groups u = gl - j/8 from the last one (u = 0) to the one of s0; u/8 + 1 slabs each, so that
+  // 4 a (a + 1) slabs belong to the 8 a last groups
+  const int gl = (n - 1) >> 3, U1 = gl - (s0 >> 3) + 1;
+  const int S = 4 * (U1 >> 3) * ((U1 >> 3) + 1) + (U1 & 7) * ((U1 >> 3) + 1);
+  const int f0 = (int)((long long)S * warp / kTriWarps), f1 = (int)((long long)S * (warp + 1) / kTriWarps);
+  int a8 = 0;
+  while (4 * (a8 + 1) * (a8 + 2) < S - f0) a8++;
+  const int rem = S - f0 - 4 * a8 * (a8 + 1);  // slabs left in the octet of groups, this one included
+  int u = 8 * a8 + (rem - 1) / (a8 + 1), m = (u - 8 * a8 + 1) * (a8 + 1) - rem;
+  double* myring = ring + (size_t)warp * kTriStages * kSlabD;
+  uint64_t* mybar = bars + warp * kTriStages;
+  auto advance = [](int& m_, int& u_) {
+    if (m_ < u_ >> 3) {
+      m_++;
     } else {
-      I_++;
-      sl_ = sl0;
+      u_--;
+      m_ = 0;
     }
   };
-  const uint64_t policy = EVICT_FIRST ? l2_evict_first_policy() : 0;
-  auto issue = [&](int I_, int sl_, int st) {
+  auto issue = [&](int m_, int u_, int st) {
     if (lane == 0) {
       mbar_expect_tx(mybar + st, (unsigned)(kSlabD * sizeof(double)));
-      if (EVICT_FIRST)
-        tma_load_2d_hint(myring + st * kSlabD, tmap, I_ * kSlabRows, sl_ * 8, mybar + st, policy);
-      else
-        tma_load_2d(myring + st * kSlabD, tmap, I_ * kSlabRows, sl_ * 8, mybar + st);
+      tma_load_2d_hint(myring + st * kSlabD, tmap, 8 * (gl - u_) + m_ * kSlabRows, 8 * (gl - u_), mybar + st, policy);
     }
   };
-  int I = T0;
-  long long acc = 0;
-  while (acc + rowlen(I) <= f0) {
-    acc += rowlen(I);
-    I++;
+  int pm = m, pu = u;
+  for (int t = 0; t < min(kTriStages, f1 - f0); t++) {
+    issue(pm, pu, t);
+    advance(pm, pu);
   }
-  int sl = sl0 + (int)(f0 - acc);
-  int pI = I, psl = sl;
-  const int npre = (int)((f1 - f0) < (long long)STAGES ? (f1 - f0) : (long long)STAGES);
-  for (int t = 0; t < npre; t++) {
-    issue(pI, psl, t);
-    advance(pI, psl);
-  }
-  double r0 = 0.0, r1 = 0.0;
-  int cI = I, csl = sl;
-  for (long long f = f0; f < f1; f++) {
-    const int st = (int)((f - f0) % STAGES);
+  between();
+  double* yw = y + (size_t)(warp % ny) * vp;
+  const bool own = ny == kTriWarps;
+  auto value = [&](int i) { return i > s0 ? v[i] : (i == s0 ? vs : 0.0); };
+  double vj[8], cp[8];
+  bool first = true;
+  int st = 0;
+  for (int f = f0; f < f1; f++) {
+    const int j0 = 8 * (gl - u);
+    if (first) {
+#pragma unroll
+      for (int c = 0; c < 8; c++) {
+        vj[c] = value(j0 + c);
+        cp[c] = 0.0;
+      }
+      first = false;
+    }
+    const int ia = j0 + m * kSlabRows + lane, ib = ia + 32;
+    const double va = value(ia), vb = value(ib);
     if (!mbar_wait(mybar + st, (parity >> st) & 1u)) {
       // a copy never completed: flag the block, wait (bounded) for the copies still in
       // flight so that none lands after this call, and stop streaming
       if (lane == 0) atomicExch(err, -5);
-      const long long last = (f + STAGES < f1) ? f + STAGES : f1;
-      for (long long g = f + 1; g < last; g++) {
-        const int sg = (int)((g - f0) % STAGES);
-        mbar_wait(mybar + sg, (parity >> sg) & 1u, 1 << 22);
-        parity ^= 1u << sg;
-      }
       parity ^= 1u << st;
+      for (int g = f + 1; g < min(f + kTriStages, f1); g++) {
+        st = st + 1 == kTriStages ? 0 : st + 1;
+        mbar_wait(mybar + st, (parity >> st) & 1u, 1 << 22);
+        parity ^= 1u << st;
+      }
       return;
     }
     parity ^= 1u << st;
     const double* buf = myring + st * kSlabD;
-    const int ia = cI * kSlabRows + lane, ib = ia + 32, j0 = csl << 3;
-    const double va = (ia >= s0 && ia < n) ? v[ia] : 0.0;
-    const double vb = (ib >= s0 && ib < n) ? v[ib] : 0.0;
-    double cp[8];
-    if (j0 >= s0 && j0 + 8 <= cI * kSlabRows && j0 + 8 <= n) {
-      // strictly left of the tile row's diagonal and inside the trailing block: no masks
+    double a0[8], a1[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      a0[c] = buf[c * kSlabRows + lane];
+      a1[c] = buf[c * kSlabRows + 32 + lane];
+    }
+    double r0 = 0.0, r1 = 0.0, q0 = 0.0, q1 = 0.0;
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      r0 = fma(a0[c], vj[c], r0);
+      r1 = fma(a1[c], vj[c], r1);
+      q0 = fma(a0[c + 1], vj[c + 1], q0);
+      q1 = fma(a1[c + 1], vj[c + 1], q1);
+    }
+    if (m > 0) {
+#pragma unroll
+      for (int c = 0; c < 8; c++) cp[c] = fma(a0[c], va, fma(a1[c], vb, cp[c]));
+    } else {  // on the diagonal: its elements count in the row sums only
 #pragma unroll
       for (int c = 0; c < 8; c++) {
-        const double a0 = buf[c * kSlabRows + lane], a1 = buf[c * kSlabRows + 32 + lane];
-        const double vj = v[j0 + c];
-        r0 = fma(a0, vj, r0);
-        r1 = fma(a1, vj, r1);
-        cp[c] = fma(a0, va, a1 * vb);
-      }
-    } else {
-#pragma unroll
-      for (int c = 0; c < 8; c++) {
-        const int jj = j0 + c;
-        const bool cok = jj >= s0 && jj < n;  // reduced columns hold Householder vectors
-        const double a0 = cok ? buf[c * kSlabRows + lane] : 0.0;
-        const double a1 = cok ? buf[c * kSlabRows + 32 + lane] : 0.0;
-        const double vj = cok ? v[jj] : 0.0;
-        r0 = fma(a0, vj, r0);
-        r1 = fma(a1, vj, r1);
-        cp[c] = (jj < ia ? a0 * va : 0.0) + (jj < ib ? a1 * vb : 0.0);  // diagonal: row sum only
+        cp[c] = fma(a0[c], c == lane ? 0.0 : va, fma(a1[c], vb, cp[c]));
       }
     }
+    r0 += q0;
+    r1 += q1;
+    // the slab's reads by all lanes come before the copy that overwrites it
+    fence_proxy_async_shared();
     __syncwarp();
-    if (f + STAGES < f1) {  // refill this stage with the slab STAGES ahead
-      issue(pI, psl, st);
-      advance(pI, psl);
+    if (f + kTriStages < f1) {  // refill this stage with the slab kTriStages ahead
+      issue(pm, pu, st);
+      advance(pm, pu);
     }
-    const double cs = slab_colsum8(cp, lane);
-    const int jc = j0 + ((lane >> 2) & 7);
-    if ((lane & 3) == 0 && jc >= s0 && jc < n && cs != 0.0) atomicAdd(&y[jc], cs);
-    int nI = cI, nsl = csl;
-    advance(nI, nsl);
-    if (f + 1 == f1 || nI != cI) {
-      if (ia >= s0 && ia < n && r0 != 0.0) atomicAdd(&y[ia], r0);
-      if (ib >= s0 && ib < n && r1 != 0.0) atomicAdd(&y[ib], r1);
-      r0 = r1 = 0.0;
+    if (own) {
+      yw[ia] += r0;
+      yw[ib] += r1;
+    } else {
+      atomicAdd(yw + ia, r0);
+      atomicAdd(yw + ib, r1);
     }
-    cI = nI;
-    csl = nsl;
+    st = st + 1 == kTriStages ? 0 : st + 1;
+    if (m == u >> 3 || f + 1 == f1) {  // the end of the group's part here
+      const double cs = colsum8_mma(cp, lane);
+      __syncwarp();
+      if ((lane & 3) == 0) {
+        double* yj = yw + j0 + (lane >> 2);
+        if (own) *yj += cs;
+        else atomicAdd(yj, cs);
+      }
+      __syncwarp();
+      first = true;
+    }
+    advance(m, u);
   }
 }
 
@@ -349,15 +352,6 @@ NRG_DEV void symv_lower(const CUtensorMap* tmap, int n, int s0, const double* v,
 // is 8 consecutive doubles per quarter-warp. The row operands Y of a tile row stay in
 // registers while the warp walks the columns. The tiles of the trailing lower triangle,
 // in tile-row order, are split evenly between the warps.
-// CG: read P and W past the L1 cache (ld.global.cg); needed when other CTAs wrote them,
-// since an SM's L1 may still hold lines it read before those writes.
-template <bool CG>
-NRG_DEV double ldp(const double* p) {
-  if constexpr (CG) return __ldcg(p);
-  else return *p;
-}
-
-template <bool CG>
 NRG_DEV void panel_update(double* __restrict__ P, const double* __restrict__ W, int n, int ld, int p0, int nbp,
                           int s0, int gwarp, int gnwarps) {
   const int lane = threadIdx.x & 31;
@@ -389,7 +383,7 @@ NRG_DEV void panel_update(double* __restrict__ P, const double* __restrict__ W, 
 #pragma unroll
         for (int mi = 0; mi < 4; mi++) {
           const int ii = i0 + 8 * mi + r;
-          ya[mi][ks] = (qq < nbp && ii < n) ? -ldp<CG>(row + ii) : 0.0;
+          ya[mi][ks] = (qq < nbp && ii < n) ? -row[ii] : 0.0;
         }
       }
     }
@@ -402,7 +396,7 @@ NRG_DEV void panel_update(double* __restrict__ P, const double* __restrict__ W, 
         for (int h = 0; h < 2; h++) {
           const int ii = i0 + 8 * mi + r, jj = j0 + 8 * ni + 2 * c4 + h;
           const bool ok = jj >= s0 && ii < n && ii >= jj;
-          acc[mi][ni][h] = ok ? ldp<CG>(P + (size_t)jj * ld + ii) : 0.0;
+          acc[mi][ni][h] = ok ? P[(size_t)jj * ld + ii] : 0.0;
         }
 #pragma unroll
     for (int ks = 0; ks < 2 * NB / 4; ks++) {
@@ -414,7 +408,7 @@ NRG_DEV void panel_update(double* __restrict__ P, const double* __restrict__ W, 
 #pragma unroll
       for (int ni = 0; ni < 4; ni++) {
         const int jj = j0 + 8 * ni + r;
-        b[ni] = (qq < nbp && jj < n) ? ldp<CG>(row + jj) : 0.0;
+        b[ni] = (qq < nbp && jj < n) ? row[jj] : 0.0;
       }
 #pragma unroll
       for (int mi = 0; mi < 4; mi++)
@@ -456,149 +450,188 @@ __global__ void __launch_bounds__(256) pack_lower_kernel(const LargeBlock* __res
 // One CTA per block: blocked (NB) Householder reduction of the packed lower triangle in W1
 // (leading dimension ldp) to tridiagonal form; d, e, tau out; Householder vector k is left
 // in column k (W1[k*ldp + k+1 ..], with a unit at k+1).
-// STAGES slabs in flight per warp; MINB CTAs per SM for the register budget: <4, 2> (two per
-// SM, 255 registers) and <2, 3> (three per SM, 168 registers and a smaller ring).
-template <int STAGES, int MINB>
-__global__ void __launch_bounds__(kTriThreads, MINB) tridiag_kernel(const LargeBlock* __restrict__ blocks,
-                                                                    const CUtensorMap* __restrict__ tmaps) {
+// Two CTAs per SM (255 registers, three slabs in flight per warp; three CTAs at 168 registers and two
+// slabs took 9% longer). ny: copies of y.
+// Many blocks are bound by HBM: 4/3 n^3 bytes of the triangle and a third more for the panel's vectors and
+// updates, about 5.5 TB/s over 1400 blocks of order 601-900: 189 ms, from 241 with slabs of aligned
+// rows, sums across lanes in every slab and three passes over V and W; 900 of order 380-420 (in L2) 24 ms,
+// from 66.
+// What bounds it is the chain of a column: its product, then sums that need the whole of a vector. The
+// reflector stays unscaled in v (u = v / scale, u(k+1) = u1), so that the product starts right after its
+// norm; the sums with the panel's V and W run while the product's first slabs are under way, one warp
+// per vector; and one pass over V and W gives both t = tau (A v - V (W^T v) - W (V^T v)) and the next
+// column without the terms in t, which follow once K = tau/2 t^T v is known: c -= v w(k+1) + w.
+__global__ void __launch_bounds__(kTriThreads, 2) tridiag_kernel(const LargeBlock* __restrict__ blocks,
+                                                                 const CUtensorMap* __restrict__ tmaps, int ny) {
   extern __shared__ __align__(16) double sm[];
-  __shared__ __align__(8) uint64_t bars[kTriWarps * STAGES];
+  __shared__ __align__(8) uint64_t bars[kTriWarps * kTriStages];
+  __shared__ double t1;  // t(k+1)
   const LargeBlock B = blocks[blockIdx.x];
-  const int n = B.n, ld = B.ldp, tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
+  const int n = B.n, ld = B.ldp, tid = threadIdx.x, nt = kTriThreads, vp = tri_pad(n);
+  const int lane = tid & 31, warp = tid >> 5;
   double* A = B.W1;
   double* W = B.W2;
-  const uint64_t keep = l2_evict_last_policy();
-  // TMA destinations: 1024-byte aligned ring of STAGES slabs per warp
+  const uint64_t keep = l2_evict_last_policy(), once = l2_evict_first_policy();
+  // TMA destinations: 1024-byte aligned ring of kTriStages slabs per warp
   double* ring = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(sm) + 1023) & ~(uintptr_t)1023);
-  double* v = ring + kTriWarps * STAGES * kSlabD;      // n
-  double* y = v + n;                                   // n
-  double* part = y + n;                                // nwarps * 2NB
-  double* cwv = part + nwarps * 2 * NB;                // 2NB
-  double* red = cwv + 2 * NB;                          // 64 (two halves for block_sum_1b)
+  double* v = ring + kTriWarps * kTriStages * kSlabD;      // vp
+  double* y = v + vp;                                  // ny x vp, ny >= 2
+  double4* coef = reinterpret_cast<double4*>(y + (size_t)ny * vp);  // NB: W^T u, V^T u, row k+1 of W and V
+  double* red = reinterpret_cast<double*>(coef + NB);  // 64 (two halves for block_sum_mma)
+  double* vb = y + vp;  // the next column, in the second copy of y between two products
   int phase = 0;
   unsigned parity = 0;
   if (lane == 0) {
-    for (int st = 0; st < STAGES; st++) mbar_init(bars + warp * STAGES + st, 1);
+    for (int st = 0; st < kTriStages; st++) mbar_init(bars + warp * kTriStages + st, 1);
     fence_mbar_init();
     tmap_acquire(tmaps + blockIdx.x);  // lane 0 issues this warp's bulk copies
+  }
+  for (int i = tid; i < vp; i += nt) {
+    v[i] = 0.0;
+    for (int c = 0; c < ny; c++) y[(size_t)c * vp + i] = 0.0;
   }
   __syncthreads();
 
   for (int p0 = 0; p0 < n - 2; p0 += NB) {
     const int pe = min(p0 + NB, n - 2);
+    double ps = 0.0;
+    for (int i = p0 + tid; i < n; i += nt) {
+      const double a = A[(size_t)p0 * ld + i];
+      v[i] = a;
+      if (i >= p0 + 2) ps = fma(a, a, ps);
+    }
+    if (tid < 4 * NB) reinterpret_cast<double*>(coef)[tid] = 0.0;
+    double sigma = block_sum_mma(ps, red, phase);  // its barrier also publishes v
     for (int k = p0; k < pe; k++) {
       const int j = k - p0;
-      // (1) current column k (rows k..n-1) = stored column minus the pending panel terms
-      {
-        double wk[NB], vk[NB];
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-          wk[q] = (q < j) ? W[(size_t)q * n + k] : 0.0;
-          vk[q] = (q < j) ? A[(size_t)(p0 + q) * ld + k] : 0.0;
-        }
-        for (int i = k + tid; i < n; i += nt) {
-          double a = A[(size_t)k * ld + i];
-#pragma unroll
-          for (int q = 0; q < NB; q++)
-            if (q < j) a -= ld_keep(A + (size_t)(p0 + q) * ld + i, keep) * wk[q] + ld_keep(W + (size_t)q * n + i, keep) * vk[q];
-          v[i] = a;
-          y[i] = 0.0;
-        }
-      }
-      __syncthreads();
-      // (2) Householder reflector for rows k+1..n-1 (dlarfg convention, v[k+1] = 1)
-      double ps = 0.0;
-      for (int i = k + 2 + tid; i < n; i += nt) ps += v[i] * v[i];
-      // alpha is read before the barrier inside block_sum_1b: thread 0 overwrites v[k+1] with
-      // the unit below, with no barrier between, and a warp that read it late would scale its
-      // part of the reflector with a wrong beta (and disagree with the others on tau)
+      // (1) Householder reflector for rows k+1..n-1 (dlarfg convention, v[k+1] = 1)
       const double alpha = v[k + 1];
-      const double sigma = block_sum_1b(ps, red, phase);
-      double tau = 0.0, beta = alpha, scale = 1.0;
+      double tau = 0.0, beta = alpha, scale = 1.0, u1 = 1.0;
       if (sigma > 0.0) {
         beta = -copysign(sqrt(alpha * alpha + sigma), alpha);
+        u1 = alpha - beta;
         tau = (beta - alpha) / beta;
-        scale = 1.0 / (alpha - beta);
+        scale = 1.0 / u1;
       }
       if (tid == 0) {
         B.d[k] = v[k];
         B.e[k] = beta;
         B.tau[k] = tau;
       }
-      for (int i = k + 2 + tid; i < n; i += nt) {
-        const double vi = v[i] * scale;
-        v[i] = vi;
-        st_keep(A + (size_t)k * ld + i, vi, keep);
+      // (2) W^T u and V^T u, four vectors q = warp + 4 c of each per warp; row k+1 of W and V
+      auto dots = [&](auto nq) {
+        constexpr int Q = decltype(nq)::value;
+        double x[8] = {};
+        const double *pw[Q], *pv[Q];
+#pragma unroll
+        for (int c = 0; c < Q; c++) {
+          const int q = min(warp + 4 * c, j - 1);
+          pw[c] = W + (size_t)q * n;
+          pv[c] = A + (size_t)(p0 + q) * ld;
+        }
+        for (int i = k + 1 + lane; i < n; i += 64) {
+          const int i2 = min(i + 32, n - 1);
+          double a[Q], b[Q], a2[Q], b2[Q];
+#pragma unroll
+          for (int c = 0; c < Q; c++) {
+            a[c] = ld_keep(pw[c] + i, keep);
+            b[c] = ld_keep(pv[c] + i, keep);
+            a2[c] = ld_keep(pw[c] + i2, keep);
+            b2[c] = ld_keep(pv[c] + i2, keep);
+          }
+          const double ui = i == k + 1 ? u1 : v[i], ui2 = i + 32 < n ? v[i2] : 0.0;
+#pragma unroll
+          for (int c = 0; c < Q; c++) {
+            x[c] = fma(a[c], ui, fma(a2[c], ui2, x[c]));
+            x[4 + c] = fma(b[c], ui, fma(b2[c], ui2, x[4 + c]));
+          }
+        }
+        const double s = colsum8_mma(x, lane);
+        const int q = warp + 4 * ((lane >> 2) & 3);
+        double* cq = reinterpret_cast<double*>(coef + q);
+        if ((lane & 3) == 0 && q < j) cq[lane >> 4] = s;
+        if ((lane & 3) == 1 && q < j) cq[2 + (lane >> 4)] = lane < 16 ? W[(size_t)q * n + k + 1] : A[(size_t)(p0 + q) * ld + k + 1];
+      };
+      auto between = [&] {
+        if (j > 12) dots(std::integral_constant<int, 4>{});
+        else if (j > 8) dots(std::integral_constant<int, 3>{});
+        else if (j > 4) dots(std::integral_constant<int, 2>{});
+        else if (j > 0) dots(std::integral_constant<int, 1>{});
+      };
+      // (3) y = A u, A as it was at the panel's start
+      if (tau != 0.0)
+        symv_lower(tmaps + blockIdx.x, n, k + 1, v, u1, y, ny, vp, ring, bars, parity, B.info, once, between);
+      else
+        between();
+      __syncthreads();
+      // (4) t, the part of K, the next column but for its terms in t; the reflector scaled
+      const double f = tau * scale;
+      const bool next = k + 1 < pe;
+      double pp = 0.0;
+      for (int i0 = k + 1 + tid; i0 < n; i0 += 4 * nt) {
+        int ii[4];
+        double t[4], b[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          ii[r] = min(i0 + r * nt, n - 1);
+          b[r] = next ? A[(size_t)(k + 1) * ld + ii[r]] : 0.0;
+          t[r] = y[ii[r]] + vb[ii[r]];
+        }
+        for (int c = 2; c < ny; c++)
+#pragma unroll
+          for (int r = 0; r < 4; r++) t[r] += y[(size_t)c * vp + ii[r]];
+        for (int q = 0; q < j; q += 4) {  // coefficients beyond j are zero
+          double a[4][4], w[4][4];
+#pragma unroll
+          for (int h = 0; h < 4; h++) {
+            const int qq = min(q + h, j - 1);
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+              a[h][r] = ld_keep(A + (size_t)(p0 + qq) * ld + ii[r], keep);
+              w[h][r] = ld_keep(W + (size_t)qq * n + ii[r], keep);
+            }
+          }
+#pragma unroll
+          for (int h = 0; h < 4; h++) {
+            const double4 cf = coef[q + h];
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+              t[r] = fma(-a[h][r], cf.x, fma(-w[h][r], cf.y, t[r]));
+              b[r] = fma(-a[h][r], cf.z, fma(-w[h][r], cf.w, b[r]));
+            }
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+          if (i0 + r * nt < n) {
+            const int i = ii[r];
+            const double vi = i == k + 1 ? 1.0 : scale * v[i], ti = f * t[r];
+            pp = fma(ti, vi, pp);
+            v[i] = vi;
+            y[i] = ti;
+            vb[i] = b[r];
+            if (i == k + 1) t1 = ti;
+            st_keep(A + (size_t)k * ld + i, vi, keep);
+          }
       }
       // column k of W1 now holds v_k below the diagonal; clear its entries above, inside
       // the back-transform panel, so that the panel's V block is exactly unit lower trapezoidal
-      const int kb0 = (k / NBT) * NBT;
-      for (int i = kb0 + 1 + tid; i <= k; i += nt) A[(size_t)k * ld + i] = 0.0;
-      if (tid == 0) {
-        v[k + 1] = 1.0;
-        A[(size_t)k * ld + k + 1] = 1.0;
+      for (int i = (k / NBT) * NBT + 1 + tid; i <= k; i += nt) A[(size_t)k * ld + i] = 0.0;
+      const double Kc = 0.5 * tau * block_sum_mma(pp, red, phase);  // its barrier also publishes t1
+      // (5) w, the next column and its norm
+      const double w1 = t1 - Kc;
+      ps = 0.0;
+      for (int i = k + 1 + tid; i < n; i += nt) {
+        const double vi = v[i], wi = y[i] - Kc * vi, ci = vb[i] - vi * w1 - wi;
+        st_keep(W + (size_t)j * n + i, wi, keep);
+        v[i] = ci;
+        for (int c = 0; c < ny; c++) y[(size_t)c * vp + i] = 0.0;
+        if (i >= k + 3) ps = fma(ci, ci, ps);
       }
-      __syncthreads();
-      if (tau != 0.0) {
-        // (3) y = A_panel_start(k+1:, k+1:) v - V (W^T v) - W (V^T v), W[:, j] = tau y - K v
-        symv_lower<STAGES, true>(tmaps + blockIdx.x, n, k + 1, v, y, ring, bars, parity, B.info, warp, nwarps);
-        if (j > 0) {
-          double pw[NB], pv[NB];
-#pragma unroll
-          for (int q = 0; q < NB; q++) pw[q] = pv[q] = 0.0;
-          for (int i = k + 1 + tid; i < n; i += nt) {
-            const double vi = v[i];
-#pragma unroll
-            for (int q = 0; q < NB; q++)
-              if (q < j) {
-                pw[q] = fma(ld_keep(W + (size_t)q * n + i, keep), vi, pw[q]);
-                pv[q] = fma(ld_keep(A + (size_t)(p0 + q) * ld + i, keep), vi, pv[q]);
-              }
-          }
-#pragma unroll
-          for (int q = 0; q < NB; q++) {
-            if (q < j) {
-              const double a = warp_sum(pw[q]);
-              const double b = warp_sum(pv[q]);
-              if (lane == 0) {
-                part[warp * 2 * NB + q] = a;
-                part[warp * 2 * NB + NB + q] = b;
-              }
-            }
-          }
-          __syncthreads();
-          if (tid < 2 * NB) {
-            double s = 0.0;
-            for (int w = 0; w < nwarps; w++) s += part[w * 2 * NB + tid];
-            cwv[tid] = s;
-          }
-        }
-        __syncthreads();
-        double cw[NB], cv[NB];
-#pragma unroll
-        for (int q = 0; q < NB; q++) {
-          cw[q] = (q < j) ? cwv[q] : 0.0;
-          cv[q] = (q < j) ? cwv[NB + q] : 0.0;
-        }
-        double pp = 0.0;
-        for (int i = k + 1 + tid; i < n; i += nt) {
-          double yi = y[i];
-#pragma unroll
-          for (int q = 0; q < NB; q++)
-            if (q < j) yi -= ld_keep(A + (size_t)(p0 + q) * ld + i, keep) * cw[q] + ld_keep(W + (size_t)q * n + i, keep) * cv[q];
-          yi *= tau;
-          y[i] = yi;
-          pp = fma(yi, v[i], pp);
-        }
-        const double Kc = 0.5 * tau * block_sum_1b(pp, red, phase);
-        for (int i = k + 1 + tid; i < n; i += nt) st_keep(W + (size_t)j * n + i, y[i] - Kc * v[i], keep);
-      } else {
-        for (int i = k + 1 + tid; i < n; i += nt) W[(size_t)j * n + i] = 0.0;
-      }
-      __syncthreads();
+      if (next) sigma = block_sum_mma(ps, red, phase);  // its barrier also publishes v, w and y
     }
-    panel_update<false>(A, W, n, ld, p0, pe - p0, pe, warp, nwarps);
+    __syncthreads();
+    panel_update(A, W, n, ld, p0, pe - p0, pe, warp, kTriWarps);
     fence_proxy_async_global();  // the next symv reads the updated trailing block by bulk copies
     __syncthreads();
   }
@@ -797,30 +830,6 @@ NRG_DEV bool mbar_wait_cluster(uint64_t* bar, unsigned parity, int bound = (1 <<
     if (done) return true;
   }
   return false;
-}
-
-// block_sum_1b with warp_sum_mma for both levels (at most 32 warps).
-NRG_DEV double block_sum_mma(double x, double* red, int& phase) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  x = warp_sum_mma(x);
-  double* b = red + 32 * (phase & 1);
-  phase++;
-  if (lane == 0) b[wid] = x;
-  __syncthreads();
-  return warp_sum_mma(lane < nw ? b[lane] : 0.0);
-}
-
-// slab_colsum8 by DMMAs: a matrix with a one in row c and its product with the lanes' x[c] put the
-// sums over the lanes of equal l/4 into row c; a last one sums each row.
-NRG_DEV double colsum8_mma(const double (&x)[8], int lane) {
-  double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0, e0 = 0.0, e1 = 0.0;
-#pragma unroll
-  for (int c = 0; c < 8; c += 2) {
-    dmma884(a0, a1, lane >> 2 == c ? 1.0 : 0.0, x[c]);
-    dmma884(b0, b1, lane >> 2 == c + 1 ? 1.0 : 0.0, x[c + 1]);
-  }
-  dmma884(e0, e1, (a0 + a1) + (b0 + b1), 1.0);
-  return e0;
 }
 
 template <int C>
@@ -2271,64 +2280,128 @@ int dsm_max_order() {
 // Microseconds of a block's reduction in a C-cluster (B200, see tridiag_dsm_kernel).
 double dsm_us(int n, int C) { return n * (1.42 + 7.5e-5 * n * n / C); }
 
-// How the blocks [lo, hi) (sorted by falling order, the first within dsm_max_order) are reduced:
-// C[q] CTAs for block q, 0 for the one-CTA kernel over the packed triangle (tridiag_smem_kernel);
-// blocks before `first` go to the streaming reduction.
-struct DsmPlan {
-  int first;
-  std::vector<int> C;
-};
-
-DsmPlan dsm_plan(const LargeBlock* b, int lo, int hi, int mid_max_n, int nsm, bool may_stream) {
-  DsmPlan p{lo, std::vector<int>(hi, 0)};
-  int sum = 0;
-  for (int q = lo; q < hi; q++) {
-    int C = 1;
-    while (!dsm_fits(b[q].n, C)) C *= 2;
-    p.C[q] = C;
-    sum += C;
-  }
-  if (sum <= nsm) {
-    // Few blocks: bound by the longest chain, so the block whose reduction takes longest gets
-    // twice the CTAs as long as the clusters fit the SMs at once.
-    for (;;) {
-      int best = -1;
-      double tb = 0.0;
-      for (int q = lo; q < hi; q++)
-        if (dsm_us(b[q].n, p.C[q]) > tb) tb = dsm_us(b[q].n, p.C[best = q]);
-      if (best < 0 || p.C[best] == 16 || sum + p.C[best] > nsm) return p;
-      sum += p.C[best];
-      p.C[best] *= 2;
-    }
-  }
-  // Many: bound by the SMs' time. Blocks that fit one CTA's packed triangle stay in one CTA (two
-  // would take 1.3 times the SM time of that kernel from order 160 on, and it half as much again
-  // as the full square below). Of the larger ones a C-cluster holds C SMs for dsm_us; the
-  // streaming reduction takes the chip's bandwidth for their bytes, but its largest block has one
-  // SM (15 GB/s, 4/3 n^3 bytes). Measured on B200, 300 blocks up to order 1024 (60 of them of order
-  // 225-600): the reductions 91 ms with all streamed, 55 with those in clusters (the 37 larger
-  // ones).
-  int mid = lo;
-  while (mid < hi && b[mid].n > mid_max_n) mid++;
-  double clu = 0.0, bytes = 0.0;
-  for (int q = lo; q < mid; q++) {
-    clu += p.C[q] * dsm_us(b[q].n, p.C[q]) / nsm;
-    bytes += 4.0 / 3.0 * b[q].n * (double)b[q].n * b[q].n;
-  }
-  if (mid > lo && may_stream) {
-    const double n0 = b[lo].n, stream = std::max(bytes / 4.4e6, 4.0 / 3.0 * n0 * n0 * n0 / 1.5e4);
-    if (stream < clu + dsm_us(b[lo].n, p.C[lo])) p.first = mid;
-  }
-  for (int q = mid; q < hi; q++)
-    if (p.C[q] > 1) p.C[q] = 0;
-  return p;
-}
-
 // Microseconds of a block's reduction by a group of G CTAs (B200, see tridiag_grid_kernel): the chain of
-// columns and the bytes an SM streams, 75 GB/s from L2 and 30 when the chip streams from HBM.
+// columns and the bytes an SM streams, 75 GB/s from L2; 45 when the chip streams from HBM, and 30 where it is
+// the largest blocks that count.
+constexpr double kGroupL2 = 75.0, kGroupHbm = 45.0, kGroupHbmLow = 30.0;
 double grid_us(int n, int G, double gbs) { return n * (5.2 + 8.0 / 3.0 * n * n / (1e3 * gbs * G)); }
 int grid_min_ctas(int n) { return (n + kGridMaxT - 1) / kGridMaxT; }
 int grid_max_ctas(int n) { return std::min(kGridMaxG, std::max(grid_min_ctas(n), n / 16)); }
+
+// Shared memory of a CTA of tridiag_kernel for blocks up to order n with ny copies of the product.
+size_t tri_smem(int n, int ny) {
+  return 1024 + sizeof(double) * ((size_t)kTriWarps * kTriStages * kSlabD + (size_t)(1 + ny) * tri_pad(n) +
+                                  4 * NB + 64);
+}
+// Copies of the product: one per warp, or two where that leaves no room for two CTAs in an SM's smsm
+// bytes (1 KB is reserved per CTA), or 0 if two do not fit either.
+int tri_copies(int n, int smsm) {
+  for (int ny : {kTriWarps, 2})
+    if (2 * (tri_smem(n, ny) + 1024 + 256) <= (size_t)smsm) return ny;
+  return 0;
+}
+
+// ... in a CTA of tridiag_kernel, two per SM (alone on the chip 10 n + 5e-5 n^3), and in
+// tridiag_smem_kernel.
+double stream_us(int n) { return n * (10.0 + 7.2e-5 * n * n); }
+double smem_us(int n) { return n * (2.0 + 1.4e-4 * n * n); }
+
+// How blocks sorted by falling order are reduced: [0, ngrid) by groups of CTAs, [ngrid, cut) and
+// [mid, nb) by clusters of C[q] (C = 0: tridiag_smem_kernel), [cut, mid) by the streaming kernel.
+// While the least clusters and groups of all blocks fit the SMs at once the longest chain bounds the
+// call: no block streams, and clusters double, the slowest block first, as long as they fit. Otherwise
+// the SMs' time does. Of that the streaming kernel takes least from order mid_max_n on (SM ms of a block
+// of order 250 / 500 / 850: 1.9 / 7 / 26; clusters 2.7 / 21, groups - / 9 / 45), but its blocks take longest: so
+// the shortest span is sought, in steps of 5%, in which the blocks that stream within it do, groups take
+// the larger ones, and the SMs (85% of them) have time for all. It has to be 7% below what clusters
+// and groups alone take. (Clusters beside streamed blocks starve: those take each SM that falls free.)
+// Measured on B200, reductions in ms by clusters and groups alone / all streamed / this plan: 300 blocks
+// of order 225-300 6.9 / 4.3 / 4.3, 100 of 400-600 17 / 16.5 / 9.7, 300 of 400-600 50 / 19 / 17, 1400 of 601-900
+// 489 / 189 / 189, 300 of 225-1000 46 / 66 / 33, 1500 of 8-2048 569 / 656 / 384, 500 of 1200-1500 667 / 363 / 377, 160
+// of 1800-2200 670 / 770 / 683, 300 of 8-1024 13.9 / 74 / 13.9; 12 of order 800-2000 16 by groups, 93 by one
+// cluster of 8 or 16 CTAs each; one of order 7049 263 by a group, 623 in two stages (band_min_n).
+struct ReductionPlan {
+  int ngrid = 0, cut = 0, mid = 0;
+  int nsm_grid = 0;  // SMs for the groups
+  std::vector<int> C;
+};
+
+ReductionPlan reduction_plan(const LargeBlock* b, int nb, int cluster_max_n, int mid_max_n, int nsm, int smsm,
+                             bool may_stream) {
+  ReductionPlan p;
+  p.C.assign(nb, 0);
+  // SM time of the first q blocks: by clusters or groups; by groups; streamed
+  std::vector<double> wl(nb + 1, 0.0), wg(nb + 1, 0.0), ws(nb + 1, 0.0);
+  double foot = 0.0;
+  for (; p.ngrid < nb && b[p.ngrid].n > cluster_max_n; p.ngrid++) foot += 8.0 * b[p.ngrid].n * b[p.ngrid].n;
+  const double gbs = foot > 1e8 ? kGroupHbm : kGroupL2;
+  int sum = 0;
+  for (int q = 0; q < nb; q++) {
+    const int n = b[q].n, G = grid_min_ctas(n);
+    const double group = G * grid_us(n, G, gbs);
+    if (q < p.ngrid) {
+      sum += G;
+      wl[q + 1] = wl[q] + group;
+    } else {
+      int C = 1;
+      while (!dsm_fits(n, C)) C *= 2;
+      p.C[q] = C;
+      sum += C;
+      wl[q + 1] = wl[q] + (n > mid_max_n ? C * dsm_us(n, C) : smem_us(n));
+    }
+    if (n > mid_max_n) p.mid = q + 1;
+    wg[q + 1] = wg[q] + group;
+    ws[q + 1] = ws[q] + 0.5 * stream_us(n);
+  }
+  p.cut = p.mid;
+  const double wmid = wl[nb] - wl[p.mid];
+  if (sum > nsm && p.mid > 0 && may_stream) {
+    const double chain = p.ngrid > 0 ? grid_us(b[0].n, grid_max_ctas(b[0].n), gbs) : dsm_us(b[0].n, 16);
+    const double most = 0.93 * std::max(chain, wl[nb] / (0.95 * nsm));
+    for (double span = chain; span < most; span *= 1.05) {
+      const int cut = (int)(std::partition_point(b, b + p.mid, [&](const LargeBlock& x) {
+                              return stream_us(x.n) > span || !tri_copies(x.n, smsm);
+                            }) - b);
+      if (wg[cut] + (ws[p.mid] - ws[cut]) + wmid > 0.85 * nsm * span) continue;
+      if (cut < p.mid) p.ngrid = p.cut = cut;
+      break;
+    }
+  }
+  int most = 1, clusters = 0;
+  double wrest = ws[p.mid] - ws[p.cut], wgrid = 0.0;
+  foot = 0.0;
+  for (int q = 0; q < p.ngrid; q++) foot += 8.0 * b[q].n * b[q].n;
+  for (int q = 0; q < nb; q++) {
+    const int n = b[q].n, G = grid_min_ctas(n);
+    if (q < p.ngrid) {
+      wgrid += G * grid_us(n, G, foot < 1e8 ? kGroupL2 : p.cut < p.mid ? kGroupHbm : kGroupHbmLow);
+    } else if (q < p.cut || q >= p.mid) {
+      most = std::max(most, p.C[q]);
+      clusters += p.C[q];
+      wrest += p.C[q] * dsm_us(n, p.C[q]);
+    }
+  }
+  if (p.ngrid > 0)  // SMs in proportion to the work
+    p.nsm_grid = p.ngrid == nb ? nsm
+                               : nsm - std::min(nsm - grid_min_ctas(b[0].n),
+                                                std::max(most, (int)(nsm * wrest / (wgrid + wrest))));
+  if (p.cut == p.mid && clusters <= nsm - p.nsm_grid) {
+    for (;;) {
+      int best = -1;
+      double tb = 0.0;
+      for (int q = p.ngrid; q < nb; q++)
+        if (dsm_us(b[q].n, p.C[q]) > tb) tb = dsm_us(b[q].n, p.C[best = q]);
+      if (best < 0 || p.C[best] == 16 || clusters + p.C[best] > nsm - p.nsm_grid) return p;
+      clusters += p.C[best];
+      p.C[best] *= 2;
+    }
+  }
+  // Blocks that fit one CTA's packed triangle stay in one CTA (two would take 1.3 times the SM time of
+  // that kernel from order 160 on, and it half as much again as the full square below).
+  for (int q = p.mid; q < nb; q++)
+    if (p.C[q] > 1) p.C[q] = 0;
+  return p;
+}
 
 struct GridPlan {
   std::vector<GridGroup> groups;
@@ -2344,7 +2417,7 @@ struct GridPlan {
 GridPlan grid_plan(const LargeBlock* b, int count, int nsm) {
   double foot = 0.0;
   for (int q = 0; q < count; q++) foot += 8.0 * b[q].n * b[q].n;
-  const double gbs = foot > 1e8 ? 30.0 : 75.0;
+  const double gbs = foot > 1e8 ? kGroupHbmLow : kGroupL2;
   struct Group { int G, cap; double us; std::vector<int> list; };
   std::vector<Group> gs;
   double span = grid_us(b[0].n, std::min(nsm, grid_max_ctas(b[0].n)), gbs);
@@ -2765,55 +2838,38 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
       const LargeBlock* b1 = blk.data() + nts;
       const LargeBlock* d1 = dblk + nts;
       const int nb1 = nb - nts;
-      int nbig = 0;
-      while (nbig < nb1 && b1[nbig].n > std::min(cluster_max_n, dsm_max_order())) nbig++;
-      const int nclu = nb1 - nbig;
-      // The larger blocks: by groups of CTAs, beside the clusters with SMs in proportion to the work,
-      // unless there are so many that the streaming kernel runs several CTAs per SM (below). Measured
-      // on B200, reductions in ms by groups / streamed: 40 blocks of order 650-900 12 / 65, 200 56 / 83, 800
-      // 204 / 276 (one per SM), 1400 357 / 230 (three per SM); 40 of order 900-2000 62 / 577; 12 of
-      // order 800-2000 16, 93 by one cluster of 8 or 16 CTAs each; one of order 7049 263, 623 in two
-      // stages (band_min_n).
-      int per_sm = c->tune.reduction_ctas_per_sm;
-      while (per_sm > 1 && (long long)nbig < 3LL * per_sm * nsm) per_sm--;
-      GridPlan gp;
-      int nsm_clu = nsm;
-      if (nbig > 0 && per_sm == 1) {
-        double wg = 0.0, wc = 0.0;
-        int most = 0;
-        for (int q = 0; q < nbig; q++) wg += grid_min_ctas(b1[q].n) * grid_us(b1[q].n, grid_min_ctas(b1[q].n), 30.0);
-        for (int q = nbig; q < nb1; q++) {
-          int C = 1;
-          while (!dsm_fits(b1[q].n, C)) C *= 2;
-          wc += C * dsm_us(b1[q].n, C);
-          most = std::max(most, C);
-        }
-        if (nclu > 0) nsm_clu = std::min(nsm - grid_min_ctas(b1[0].n), std::max(most, (int)(nsm * wc / (wg + wc))));
-        gp = grid_plan(b1, nbig, nsm - (nclu > 0 ? nsm_clu : 0));
-      }
-      const bool grid = gp.ctas > 0;
-      const DsmPlan dp = dsm_plan(b1, nbig, nb1, mid_max_n, nsm_clu, !grid);
-      nbig = dp.first;
-      // Launches that can run side by side go to streams of their own: the streaming reduction of
-      // the largest blocks on s, each cluster size and the one-CTA kernel beside it, largest first
-      // (clusters need SMs of one GPC free at once).
-      struct Launch { int C, q0, q1; };  // C = 0: tridiag_smem_kernel
+      int smsm = 0;
+      NRG_CK(cudaDeviceGetAttribute(&smsm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c->device));
+      const ReductionPlan rp = reduction_plan(b1, nb1, std::min(cluster_max_n, dsm_max_order()), mid_max_n, nsm, smsm,
+                                              c->tune.reduction_ctas_per_sm > 1);
+      const int ngrid = rp.ngrid, nstream = rp.mid - rp.cut;
+      // Launches that can run side by side go to streams of their own: the groups of the largest blocks on
+      // s, then each cluster size, the streaming kernel and the one-CTA kernels beside them,
+      // largest first (clusters need SMs of one GPC free at once).
+      struct Launch { int C, q0, q1; };  // C = 0: tridiag_smem_kernel, -1: tridiag_kernel
       std::vector<Launch> ls;
-      for (int C = 16; C >= 0; C = C > 1 ? C / 2 : C - 1)
-        for (int q0 = nbig, q1; q0 < nb1; q0 = q1) {
-          for (q1 = q0 + 1; q1 < nb1 && dp.C[q1] == dp.C[q0]; q1++) {}
-          if (dp.C[q0] == C) ls.push_back({C, q0, q1});
+      for (int C = 16; C >= 0; C = C > 1 ? C / 2 : C - 1) {
+        if (C == 1 && nstream > 0) ls.push_back({-1, rp.cut, rp.mid});
+        for (int q0 = ngrid, q1; q0 < nb1; q0 = q1) {
+          if (q0 >= rp.cut && q0 < rp.mid) {
+            q1 = rp.mid;
+            continue;
+          }
+          for (q1 = q0 + 1; q1 < nb1 && q1 != rp.cut && rp.C[q1] == rp.C[q0]; q1++) {}
+          if (rp.C[q0] == C) ls.push_back({C, q0, q1});
         }
-      const bool fork = ls.size() + (nbig > 0) > 1;
+      }
+      const bool fork = ls.size() + (ngrid > 0) > 1;
       if (fork) {
         rc = tri_streams(c);
         if (rc) return rc;
         NRG_CK(cudaEventRecord(c->tri_fork, s));
       }
-      PhaseScope ps(c, kPhTridiag, s, (nbig ? 2 : 0) + (int)ls.size());
+      PhaseScope ps(c, kPhTridiag, s, (ngrid > 0 ? 2 : 0) + (nstream > 0 ? 1 : 0) + (int)ls.size());
       unsigned used = 0;  // side streams with a launch
-      if (grid) {
-        pack_full_kernel<<<dim3((b1[0].ldp + 31) / 32, (b1[0].n + 31) / 32, nbig), 256, 0, s>>>(d1);
+      if (ngrid > 0) {
+        const GridPlan gp = grid_plan(b1, ngrid, rp.nsm_grid);
+        pack_full_kernel<<<dim3((b1[0].ldp + 31) / 32, (b1[0].n + 31) / 32, ngrid), 256, 0, s>>>(d1);
         NRG_CK(cudaGetLastError());
         std::vector<char> gi;
         const size_t go = push(gi, gp.groups), jo = push(gi, gp.jobs),
@@ -2840,59 +2896,30 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
         unsigned* dc = reinterpret_cast<unsigned*>(gb + co);
         void* kargs[] = {(void*)&db, (void*)&dg, (void*)&ng, (void*)&dj, (void*)&dc};
         NRG_CK(cudaLaunchKernelExC(&cfg, fn, kargs));
-      } else if (nbig) {
-        auto tri_bytes = [&](int st) {
-          return 1024 + sizeof(double) * ((size_t)kTriWarps * st * kSlabD + 2 * (size_t)b1[0].n +
-                                          (size_t)kTriWarps * 2 * NB + 2 * NB + 64);
-        };
-        const CUtensorMap* tm = reinterpret_cast<const CUtensorMap*>(dbase + tmap_off) + nts;
-        pack_lower_kernel<<<dim3((b1[0].n + 7) / 8, nbig), 256, 0, s>>>(d1);
-        NRG_CK(cudaGetLastError());
-        // reduction_ctas_per_sm (nrg_tuning) sets how many CTAs of the streaming kernel share an
-        // SM: one, when each requests at least half of an SM's shared memory; two, with four
-        // slabs in flight per warp; three (the default), with two slabs per warp and at most 168
-        // registers per thread. More CTAs per SM keep the SM's HBM stream going while a CTA is
-        // in the serial part of a column (norm, reflector, block sums); where the blocks' vectors
-        // leave no room for that many, the next smaller count is used. Several per SM once gave
-        // wrong reductions through a race on alpha = v[k+1] in the reflector step (alpha was read
-        // after a barrier that a thread overwriting it could pass); alpha is now read before that
-        // barrier, and batches with more of these CTAs than SMs pass every check on B200.
-        int smsm = 0;
-        cudaDeviceGetAttribute(&smsm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c->device);
-        {
-          // one, two or three CTAs per SM as above (1 KB of shared memory is reserved per CTA);
-          // reduction_ctas_per_sm is the most, used when the batch fills at least three waves of
-          // that many CTAs per SM. A batch of fewer large blocks is bound by its largest ones,
-          // which finish sooner with an SM's bandwidth shared by fewer CTAs (measured on B200:
-          // 1500 blocks of order 8-2048, about 330 of them streamed, take 873 ms with one CTA
-          // per SM, 909 with two, 1015 with three; the benchmark's 10,000 blocks run 6.5% faster
-          // with three than with two).
-          if (per_sm == 3 && 3 * (tri_bytes(2) + 1024) > (size_t)smsm) per_sm = 2;
-          if (per_sm == 2 && 2 * (tri_bytes(4) + 1024) > (size_t)smsm) per_sm = 1;
-          if (per_sm == 3) {
-            const size_t smem3 = tri_bytes(2);
-            NRG_CK(cudaFuncSetAttribute(tridiag_kernel<2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem3));
-            tridiag_kernel<2, 3><<<nbig, kTriThreads, smem3, s>>>(d1, tm);
-          } else {
-            const size_t smem1 = std::max(tri_bytes(4), (per_sm == 1 ? (size_t)smsm / 2 + 1024 : (size_t)0));
-            NRG_CK(cudaFuncSetAttribute(tridiag_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem1));
-            tridiag_kernel<4, 2><<<nbig, kTriThreads, smem1, s>>>(d1, tm);
-          }
-          NRG_CK(cudaGetLastError());
-        }
       }
       for (size_t q = 0; q < ls.size(); q++) {
         cudaStream_t ss = s;
-        const size_t side = q + (nbig > 0);  // 0: stream s
+        const size_t side = q + (ngrid > 0);  // 0: stream s
         if (side > 0) {
           const int i = (int)(side - 1) % nrg_ctx::kTriStreams;
           ss = c->tri[i];
           if (!(used >> i & 1)) NRG_CK(cudaStreamWaitEvent(ss, c->tri_fork, 0));
           used |= 1u << i;
         }
-        NRG_CK(reduce_in_smem_launch(d1 + ls[q].q0, b1[ls[q].q0].n, ls[q].q1 - ls[q].q0, ls[q].C, ss));
+        const LargeBlock* dq = d1 + ls[q].q0;
+        const int nq = b1[ls[q].q0].n, count = ls[q].q1 - ls[q].q0;
+        if (ls[q].C < 0) {
+          const int ny = tri_copies(nq, smsm);
+          const size_t smem = tri_smem(nq, ny);
+          pack_lower_kernel<<<dim3((nq + 7) / 8, count), 256, 0, ss>>>(dq);
+          NRG_CK(cudaGetLastError());
+          NRG_CK(cudaFuncSetAttribute(tridiag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+          tridiag_kernel<<<count, kTriThreads, smem, ss>>>(
+              dq, reinterpret_cast<const CUtensorMap*>(dbase + tmap_off) + nts + ls[q].q0, ny);
+          NRG_CK(cudaGetLastError());
+        } else {
+          NRG_CK(reduce_in_smem_launch(dq, nq, count, ls[q].C, ss));
+        }
       }
       for (int i = 0; i < nrg_ctx::kTriStreams; i++)
         if (used >> i & 1) NRG_CK(cudaEventRecord(c->tri_join[i], c->tri[i]));
