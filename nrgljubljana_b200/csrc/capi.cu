@@ -978,7 +978,7 @@ int nrg_spec_accumulate(nrg_ctx* c, int npair, const nrg_spec_pair* pairs, const
   const char* base = static_cast<const char*>(c->desc);
   nrg::PhaseScope ps(c, nrg::kPhSpecBin, s);
   CK(nrg::spec_bin_launch(reinterpret_cast<const nrg::SpecRegion*>(base + ro), (int)regs.size(), tiles, rows, bp, pos,
-                          neg, s));
+                          neg, !regs.empty() && regs[0].kind == nrg::kSpecDMNRG, s));
   return NRG_OK;
 }
 

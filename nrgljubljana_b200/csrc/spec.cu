@@ -14,7 +14,6 @@ namespace nrg {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kUnroll = 4;  // rows whose operands a lane loads together
 
 struct Hist {
   double* pos;
@@ -81,8 +80,8 @@ NRG_DEV void bin_add(Run& a, const Hist& h, const BinParams& bp, double energy, 
 }
 
 // One warp tile: columns i0 + 32 ti .., `rows` rows from j0 + rows tj. A lane keeps one column
-// and walks down the rows.
-template <int KIND>
+// and walks down the rows, U of whose operands it loads together.
+template <int KIND, int U>
 NRG_DEV void bin_tile(const SpecRegion& r, const Hist& h, const BinParams& bp, int ib, int jb, int jn) {
   const int lane = threadIdx.x & 31;
   const int i = ib + lane;
@@ -90,29 +89,36 @@ NRG_DEV void bin_tile(const SpecRegion& r, const Hist& h, const BinParams& bp, i
   const double ei = act ? r.Ei[i] : 0.0;
   const double xi = (KIND == kSpecExpI && act) ? exp(-ei / r.T) : 0.0;
   Run run;
+  const bool XY = KIND == kSpecDMNRG || KIND == kSpecGemmX;
+  const double* p1 = r.op1 + (int64_t)jb * r.ld1 + i;
+  const double* p2 = KIND != kSpecGemmX ? r.op2 + (int64_t)jb * r.ld2 + i : nullptr;
+  const double* px = XY ? r.X + (int64_t)(jb - r.j0) * r.ldx + (i - r.i0) : nullptr;
+  const double* py = KIND == kSpecDMNRG ? r.Y + (int64_t)(jb - r.j0) * r.ldy + (i - r.i0) : nullptr;
   for (int g = 0; g < jn; g += 32) {
     const int cnt = min(32, jn - g);
     const double ejl = lane < cnt ? r.Ej[jb + g + lane] : 0.0;
     const double xjl = (KIND == kSpecExpJ && lane < cnt) ? exp(-ejl / r.T) : 0.0;
-    for (int q = 0; q < cnt; q += kUnroll) {
-      double en[kUnroll], o1[kUnroll], o2[kUnroll], x[kUnroll], y[kUnroll], xj[kUnroll];
-      bool ok[kUnroll];
+    for (int q = 0; q < cnt; q += U) {
+      double en[U], o1[U], o2[U], x[U], y[U], xj[U];
+      bool ok[U];
 #pragma unroll
-      for (int u = 0; u < kUnroll; u++) {
+      for (int u = 0; u < U; u++) {
         const int row = min(q + u, 31);
         en[u] = __shfl_sync(0xffffffffu, ejl, row) - ei;
         xj[u] = KIND == kSpecExpJ ? __shfl_sync(0xffffffffu, xjl, row) : 0.0;
         ok[u] = act && q + u < cnt;
         if (KIND == kSpecDMNRG) ok[u] = ok[u] && !(fabs(en[u]) < r.Emin || fabs(en[u]) > r.Emax);
-        const int64_t j = jb + g + q + u;
-        o1[u] = ok[u] ? r.op1[j * r.ld1 + i] : 0.0;
-        o2[u] = (KIND != kSpecGemmX && ok[u]) ? r.op2[j * r.ld2 + i] : 0.0;
-        if (KIND == kSpecDMNRG || KIND == kSpecGemmX)
-          x[u] = ok[u] ? r.X[(j - r.j0) * r.ldx + (i - r.i0)] : 0.0;
-        if (KIND == kSpecDMNRG) y[u] = ok[u] ? r.Y[(j - r.j0) * r.ldy + (i - r.i0)] : 0.0;
+        o1[u] = ok[u] ? p1[u * r.ld1] : 0.0;
+        o2[u] = (KIND != kSpecGemmX && ok[u]) ? p2[u * r.ld2] : 0.0;
+        if (XY) x[u] = ok[u] ? px[u * r.ldx] : 0.0;
+        if (KIND == kSpecDMNRG) y[u] = ok[u] ? py[u * r.ldy] : 0.0;
       }
+      p1 += U * r.ld1;
+      if (KIND != kSpecGemmX) p2 += U * r.ld2;
+      if (XY) px += U * r.ldx;
+      if (KIND == kSpecDMNRG) py += U * r.ldy;
 #pragma unroll
-      for (int u = 0; u < kUnroll; u++) {
+      for (int u = 0; u < U; u++) {
         if (!ok[u]) continue;
         double w;
         if (KIND == kSpecDMNRG) w = x[u] * o1[u] + (double)(-r.sign) * (y[u] * o2[u]);
@@ -154,11 +160,15 @@ NRG_DEV void bin_tile(const SpecRegion& r, const Hist& h, const BinParams& bp, i
 // (one flush of its non-zero bins at the end); larger grids take FP64 atomics in L2.
 // Measured on B200, both FDM parts of 12 subspaces of order 800-2000 (36 million terms, 10 bins a
 // decade, whole call with its GEMMs): 2643 us with one atomic pair per term and a 64-bit division
-// for the indices, 815 us so; a DM-NRG call of 40 subspaces up to order 192 on 1000 bins a decade
-// 76 and 55 us.
-__global__ void __launch_bounds__(kThreads) spec_bin_kernel(const SpecRegion* __restrict__ regs, int nreg,
-                                                            int64_t ntiles, int rows, BinParams bp, double* gpos,
-                                                            double* gneg, int use_smem) {
+// for the indices, 628 us so; a DM-NRG call of 40 subspaces up to order 192 on 1000 bins a decade
+// 76 and 36 us. What is left is the latency of a term's chain (a logarithm, 200 instructions): the FDM
+// kernel runs at four CTAs per SM with two rows loaded together (its launches 0.38 ms, 0.50 at two
+// CTAs and four rows, 0.42 at four and four), DM-NRG's short launch at two and four (16 us, 19).
+// DM: all regions are of DM-NRG (kSpecDMNRG), otherwise none is.
+template <bool DM>
+__global__ void __launch_bounds__(kThreads, DM ? 2 : 4) spec_bin_kernel(const SpecRegion* __restrict__ regs, int nreg,
+                                                                        int64_t ntiles, int rows, BinParams bp,
+                                                                        double* gpos, double* gneg, int use_smem) {
   extern __shared__ __align__(16) double sh[];
   Hist h{gpos, gneg};
   if (use_smem) {
@@ -172,11 +182,14 @@ __global__ void __launch_bounds__(kThreads) spec_bin_kernel(const SpecRegion* __
     const SpecRegion r = regs[find_region(regs, nreg, t)];
     const int lt = (int)(t - r.tile0), ti = (r.i1 - r.i0 + 31) / 32;
     const int ib = r.i0 + 32 * (lt % ti), jb = r.j0 + rows * (lt / ti), jn = min(rows, r.j1 - jb);
-    switch (r.kind) {
-      case kSpecDMNRG: bin_tile<kSpecDMNRG>(r, h, bp, ib, jb, jn); break;
-      case kSpecExpI: bin_tile<kSpecExpI>(r, h, bp, ib, jb, jn); break;
-      case kSpecExpJ: bin_tile<kSpecExpJ>(r, h, bp, ib, jb, jn); break;
-      default: bin_tile<kSpecGemmX>(r, h, bp, ib, jb, jn); break;
+    if (DM) {
+      bin_tile<kSpecDMNRG, 4>(r, h, bp, ib, jb, jn);
+    } else {
+      switch (r.kind) {
+        case kSpecExpI: bin_tile<kSpecExpI, 2>(r, h, bp, ib, jb, jn); break;
+        case kSpecExpJ: bin_tile<kSpecExpJ, 2>(r, h, bp, ib, jb, jn); break;
+        default: bin_tile<kSpecGemmX, 2>(r, h, bp, ib, jb, jn); break;
+      }
     }
     __syncwarp();
   }
@@ -348,18 +361,18 @@ int spec_tile_rows(int64_t terms) {
 }
 
 cudaError_t spec_bin_launch(const SpecRegion* d_regs, int nreg, int64_t ntiles, int rows, const BinParams& bp,
-                            double* pos, double* neg, cudaStream_t stream) {
+                            double* pos, double* neg, bool dmnrg, cudaStream_t stream) {
   if (nreg <= 0 || ntiles <= 0) return cudaSuccess;
   const size_t smem = 2 * sizeof(double) * (size_t)bp.nbins;
   const int use_smem = smem <= kSpecSmemMax ? 1 : 0;
+  const auto kernel = dmnrg ? spec_bin_kernel<true> : spec_bin_kernel<false>;
   if (use_smem) {
     cudaError_t err =
-        cudaFuncSetAttribute(spec_bin_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpecSmemMax);
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpecSmemMax);
     if (err != cudaSuccess) return err;
   }
   const int64_t grid = std::min<int64_t>((ntiles + kThreads / 32 - 1) / (kThreads / 32), 148 * 6);
-  spec_bin_kernel<<<(unsigned)grid, kThreads, use_smem ? smem : 0, stream>>>(d_regs, nreg, ntiles, rows, bp, pos, neg,
-                                                                            use_smem);
+  kernel<<<(unsigned)grid, kThreads, use_smem ? smem : 0, stream>>>(d_regs, nreg, ntiles, rows, bp, pos, neg, use_smem);
   return cudaGetLastError();
 }
 

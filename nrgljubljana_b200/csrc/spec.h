@@ -65,7 +65,7 @@ inline int64_t spec_tiles(int i0, int i1, int j0, int j1, int rows) {
 // Rows of a warp tile for a call of `terms` terms.
 int spec_tile_rows(int64_t terms);
 cudaError_t spec_bin_launch(const SpecRegion* d_regs, int nreg, int64_t ntiles, int rows, const BinParams& bp,
-                            double* pos, double* neg, cudaStream_t stream);
+                            double* pos, double* neg, bool dmnrg, cudaStream_t stream);
 
 constexpr int kMatsChunk = 2048;  // terms of one CTA's pass of the Matsubara kernel
 inline int64_t mats_chunks(int i0, int i1, int j0, int j1) {
