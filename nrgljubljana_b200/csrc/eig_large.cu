@@ -778,9 +778,13 @@ __global__ void __launch_bounds__(kMidThreads) tridiag_smem_kernel(const LargeBl
 // after it received all of column k+1's, which each other CTA sends after reading column k's.
 // The reflector is kept unscaled (u = v / scale, so that the product does not wait for the
 // scaling). The rows of a column are summed in the same order whatever C is.
-// Measured on B200 (one block, us per column): n = 456 in 16 CTAs 2.4 (5.4 with two cluster barriers
-// per column over one triangle), n = 300 1.9 in 16 and 2.3 in 8, n = 224 1.6 in 16, 1.9 in 8, 2.5 in
-// 4, 3.7 in 2, n = 128 1.5 in 16, 1.8 in 4, 3.1 in 1; 256 threads are 8% faster than 512.
+// Pairs are stored by their sender, so that a warp's stores go to consecutive slots of one CTA at a time
+// (to 32 slots C apart in as many CTAs they cost a further 0.25 us per column).
+// Measured on B200 (one block, us per column): n = 456 in 16 CTAs 2.2 (5.4 with two cluster barriers
+// per column over one triangle), n = 300 1.8 in 16, n = 224 1.55 and n = 128 1.4; with the stores apart
+// n = 300 2.3 in 8, n = 224 1.6 in 16, 1.9 in 8, 2.5 in 4, 3.7 in 2, n = 128 1.5 in 16, 1.8 in 4, 3.1
+// in 1. 256 threads are 8% faster than 512. At n = 456 the products take 1900 cycles of a column, the
+// two sums 740, the reflector 250, the exchange the rest.
 // Output as tridiag_kernel: d, e, tau, and v_k in row k of W1 (unit at k+1, zeros from the start
 // of its back-transform panel up to k).
 constexpr int kDsmThreads = 256;
@@ -791,11 +795,14 @@ constexpr int kRowSplit = 4, kColSplit = kDsmWarps / kRowSplit;
 
 __host__ __device__ inline int dsm_cols(int n, int C) { return (n + C - 1) / C; }
 
+// Pairs of a CTA's columns in a pair buffer, odd: neighbouring rows of it lie on different banks.
+__host__ __device__ inline int dsm_slot(int n, int C) { return dsm_cols(n, C) | 1; }
+
 // Doubles of shared memory of one CTA of a C-cluster for a block of order n: pairs (2 buffers), v,
 // w, u, partial products, row k+1, reduction scratch, columns.
 __host__ __device__ inline size_t dsm_smem_doubles(int n, int C) {
   const size_t T = dsm_cols(n, C), Tp = (T + 7) / 8 * 8;
-  return 4 * (size_t)n + 3 * (size_t)n + (kRowSplit + 1) * Tp + 64 + T * n;
+  return 4 * (size_t)C * dsm_slot(n, C) + 3 * (size_t)n + (kRowSplit + 1) * Tp + 64 + T * n;
 }
 
 inline bool dsm_fits(int n, int C) {
@@ -841,9 +848,10 @@ __global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const Large
   const int r = blockIdx.x % C;  // rank in the cluster
   const LargeBlock B = blocks[blockIdx.x / C];
   const int n = B.n, ld = B.ldp, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int T = (n - r + C - 1) / C, Tp = (dsm_cols(n, C) + 7) / 8 * 8;  // owned columns
-  double2* buf = reinterpret_cast<double2*>(sm);  // 2 x n pairs (product, column element)
-  double* v = sm + 4 * (size_t)n;                 // previous reflector
+  const int T = (n - r + C - 1) / C, Tp = (dsm_cols(n, C) + 7) / 8 * 8, Tm = dsm_slot(n, C);  // owned columns
+  double2* buf = reinterpret_cast<double2*>(sm);  // 2 x C x Tm pairs (product, column element), by sender
+  auto slot = [Tm](int i) { return (i % C) * Tm + i / C; };
+  double* v = sm + 4 * C * Tm;                    // previous reflector
   double* w = v + n;                              // and its w
   double* u = w + n;                              // new reflector, unscaled, before the shift of u[k+1]
   double* part = u + n;                           // kRowSplit x Tp
@@ -863,7 +871,7 @@ __global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const Large
     for (int t = lane; t < T; t += 32)
       if (r + t * C > i) M[(size_t)t * n + i] = B.H[(size_t)i * n + r + t * C];
   for (int i = tid; i < n; i += kDsmThreads) {
-    buf[i] = make_double2(0.0, B.H[i]);
+    buf[slot(i)] = make_double2(0.0, B.H[i]);
     v[i] = w[i] = 0.0;
   }
   if (tid == 0) {
@@ -884,7 +892,7 @@ __global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const Large
   double ur[kDsmRows] = {};             // u of this thread's rows (of the previous column)
   double alpha = 0.0, beta = 0.0;       // previous reflector
   for (int k = 0; k < n - 1; k++) {
-    const double2* pb = buf + (size_t)(k & 1) * n;
+    const double2* pb = buf + (k & 1) * C * Tm;
     const double tau = sc[2 * (k & 1)], scale = sc[2 * (k & 1) + 1], f = tau * scale;
     double vr[kDsmRows];
 #pragma unroll
@@ -917,13 +925,13 @@ __global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const Large
       const int i = tid + q * kDsmThreads;
       y[q] = cc[q] = 0.0;
       if (i >= k && i < n) {
-        const double2 p = pb[i];
+        const double2 p = pb[slot(i)];
         y[q] = f * p.x;
         cc[q] = p.y;
         pd = fma(y[q], vr[q], pd);
       }
     }
-    const double yk = f * pb[k].x;
+    const double yk = f * pb[slot(k)].x;
     const double Kc = 0.5 * tau * block_sum_mma(pd, red, phase);
     // (2) column k after that update; reflector for rows k+1..n-1 (dlarfg convention)
     const double wk = k > 0 ? yk - Kc : 0.0;
@@ -1018,16 +1026,18 @@ __global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const Large
     }
     __syncthreads();
     // (4) each owned column's product and element of row k+1 to every CTA
-    double2* nb = buf + (size_t)((k + 1) & 1) * n;
+    double2* nb = buf + ((k + 1) & 1) * C * Tm;
     if constexpr (C > 1) {
       uint64_t* bar = bars + ((k + 1) & 1);
       if (tid == 0) mbar_expect_tx(bar, 16u * (unsigned)(n - k - 1));
-      const int items = (T - t0) * C;
-      for (int it = tid; it < items; it += kDsmThreads) {
-        const int t = t0 + it / C, dst = it % C;
-        static_assert(kRowSplit == 4, "pairwise sum of the row parts");
-        const double yj = (part[t] + part[Tp + t]) + (part[2 * Tp + t] + part[3 * Tp + t]);
-        st_async_pair(cluster_addr(smem_u32(nb + r + t * C), dst), yj, rowk[t], cluster_addr(smem_u32(bar), dst));
+      // a warp sends its columns' pairs to one CTA at a time, to consecutive slots there
+      constexpr int kPer = C < kDsmWarps ? kDsmWarps / C : 1;  // warps per destination
+      static_assert(kRowSplit == 4, "pairwise sum of the row parts");
+      for (int t = t0 + lane + 32 * (warp / C); t < T; t += 32 * kPer) {
+        const double yj = (part[t] + part[Tp + t]) + (part[2 * Tp + t] + part[3 * Tp + t]), xj = rowk[t];
+#pragma unroll
+        for (int dst = warp % C; dst < C; dst += kDsmWarps)
+          st_async_pair(cluster_addr(smem_u32(nb + r * Tm + t), dst), yj, xj, cluster_addr(smem_u32(bar), dst));
       }
     } else {
       for (int t = t0 + tid; t < T; t += kDsmThreads)
