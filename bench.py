@@ -345,7 +345,7 @@ def main():
         pk = peaks.get("hbm_gbs", 6650.0)
         roof = {"kernel": "tridiag_kernel", "bound": "hbm", "achieved": ach, "peak": pk, "unit": "GB/s",
                 "frac": ach / pk, "traffic": per_launch_bytes * tridiag_traffic_ratio,
-                "traffic_source": "ncu dram bytes of tridiag_kernel (three CTAs per SM) on 1400 x n=608 (profiles/tridiag_kernel_1400x608.md), scaled by algorithmic bytes",
+                "traffic_source": "ncu dram bytes of an earlier tridiag_kernel (three CTAs per SM) on 1400 x n=608 (profiles/tridiag_kernel_1400x608.md), scaled by algorithmic bytes",
                 "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
                 "bytes_per_launch": per_launch_bytes, "avg_launch_ms": avg * 1e3}
     else:
