@@ -38,7 +38,7 @@ constexpr int kTriThreads = 128;
 constexpr int NB = 16;     // tridiagonalisation panel width
 constexpr int NBT = 128;   // back-transform panel width
 constexpr int kLeaf = 64;  // divide-and-conquer leaves have at most this order
-constexpr int kMaxLargeN = 10240;  // the tridiagonalisation's shared memory (68 KB + 16 n bytes) fits to here
+constexpr int kMaxLargeN = 10240;  // the rows that the threads of tridiag_grid_kernel<20> hold
 // Merge nodes whose prep arrays exceed this many bytes keep them in global scratch (kPrepGlobalB
 // bytes per row of the block) instead of shared memory.
 constexpr size_t kPrepSmemMax = 200 * 1024;
