@@ -14,13 +14,15 @@ namespace nrg {
 constexpr int kCtaEigThreads = 256;
 constexpr int kCtaEigWarps = kCtaEigThreads / 32;
 
-// Scratch of smem_dc for order N: eleven doubles and five ints per row.
-__host__ __device__ inline size_t dc_scratch_bytes(int N) { return (11 * sizeof(double) + 5 * sizeof(int)) * (size_t)N; }
+// Scratch of smem_dc for order N: ten doubles and five ints per row.
+__host__ __device__ inline size_t dc_scratch_bytes(int N) { return (10 * sizeof(double) + 5 * sizeof(int)) * (size_t)N; }
 
 // Eigenvalues a[i][i] and eigenvectors (rows of v) of a symmetric matrix of order 4 by cyclic Jacobi
 // rotations, one thread; of smaller orders with zero rows and columns (zero couplings are
-// skipped). False if 30 sweeps did not converge (five or so do).
-NRG_DEV bool jacobi4(double (&a)[4][4], double (&v)[4][4]) {
+// skipped). False if 30 sweeps did not converge (five or so do). Couplings between equal diagonals may be
+// of any size, down to the smallest denormal: the tangent is formed in units in which its squares
+// stay in range.
+__host__ __device__ __forceinline__ bool jacobi4(double (&a)[4][4], double (&v)[4][4]) {
 #pragma unroll
   for (int i = 0; i < 4; i++)
 #pragma unroll
@@ -36,7 +38,8 @@ NRG_DEV bool jacobi4(double (&a)[4][4], double (&v)[4][4]) {
       const bool act = fabs(apq) > 0.5 * kEps * (fabs(a[p][p]) + fabs(a[q][q]));
       any |= act;
       // tan of the angle, the smaller root: 2 a_pq / (df + sgn(df) sqrt(df^2 + 4 a_pq^2))
-      const double tn = copysign(2.0 * apq, copysign(1.0, df) * apq) / (fabs(df) + sqrt(fma(df, df, 4.0 * apq * apq)));
+      const double up = fmax(fabs(df), fabs(apq)) < 1e-150 ? 0x1p1000 : 1.0, x = up * df, y = 2.0 * (up * apq);
+      const double tn = copysign(y, copysign(1.0, df) * apq) / (fabs(x) + sqrt(fma(x, x, y * y)));
       const double t = act ? tn : 0.0, c = act ? rsqrt(fma(t, t, 1.0)) : 1.0, s = t * c;
       a[p][p] = fma(-t, apq, a[p][p]);
       a[q][q] = fma(t, apq, a[q][q]);
@@ -170,8 +173,7 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
   double* zh = lamn + N;
   double* rc = zh + N;                      // deflation rotations
   double* rs = rc + N;
-  double* red = rs + N;                     // N >= 1
-  int* sidx = reinterpret_cast<int*>(red + N);
+  int* sidx = reinterpret_cast<int*>(rs + N);
   int* srow = sidx + N;                     // row of Z behind entry t (deflated ones from K on)
   int* flag = srow + N;                     // deflated
   int* rp = flag + N;
@@ -179,25 +181,22 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
   int* nrot = ctl;       // per node, 8
   int* status = ctl + 8;
 
-  // scale
+  // scale (by scalbn: 2^-ex itself is out of range for the smallest and the largest norms)
   if (warp == 0) {
     double m = 0.0;
     for (int i = lane; i < N; i += 32) m = fmax(m, fmax(fabs(d[i]), i < N - 1 ? fabs(e[i]) : 0.0));
     m = warp_max(m);
     if (lane == 0) {
-      red[0] = m > 0.0 ? scalbn(1.0, -ilogb(m)) : 1.0;
+      ctl[9] = m > 0.0 ? ilogb(m) : 0;
       *status = 0;
     }
   }
   for (int i = tid; i < N * ld; i += kCtaEigThreads) Z[i] = 0.0;
   __syncthreads();
-  const double sc = red[0];
-  const bool scaled = sc < 1e300 && sc > 1e-300;  // beyond that the scaled values would not be exact
+  const int ex = ctl[9];
   if (tid < N) {
-    if (scaled) {
-      d[tid] *= sc;
-      if (tid < N - 1) e[tid] *= sc;
-    }
+    d[tid] = scalbn(d[tid], -ex);
+    if (tid < N - 1) e[tid] = scalbn(e[tid], -ex);
     Z[tid * ld + tid] = 1.0;
   }
   const int L = N > 64 ? 5 : N > 32 ? 4 : N > 16 ? 3 : N > 8 ? 2 : N > 4 ? 1 : 0;  // leaves of order 2..4
@@ -485,7 +484,7 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
     if (gt < n) d[lo + gt] = lamn[lo + gt];
     __syncthreads();
   }
-  if (scaled && tid < N) d[tid] /= sc;  // a power of two
+  if (tid < N) d[tid] = scalbn(d[tid], ex);
   __syncthreads();
   return *status;
 }

@@ -1,0 +1,86 @@
+"""The one-CTA eigensolver's device code run on the CPU (tests/cpp/cta_emulator.h), on matrices whose
+small numbers leave the range in which squares can be formed: tridiagonal matrices with degenerate
+pairs that are coupled by next to nothing, blocks of denormal norm."""
+import ctypes
+import os
+import re
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "nrgljubljana_b200", "csrc")
+PTR = ctypes.POINTER(ctypes.c_double)
+
+
+def _replace(text, pattern, new):
+    out, count = re.subn(pattern, lambda m: new, text, flags=re.S)
+    assert count == 1, (count, pattern)
+    return out
+
+
+@pytest.fixture(scope="module")
+def solver(tmp_path_factory):
+    tmp = tmp_path_factory.mktemp("small_solver")
+    read = lambda f: open(os.path.join(CSRC, f)).read()  # noqa: E731
+    common = _replace(read("common.cuh"), r"NRG_DEV void dmma884\(.*?\n}\n",
+                      "NRG_DEV void dmma884(double& d0, double& d1, double a, double b) { emu_dmma884(d0, d1, a, b); }\n")
+    common = _replace(common, r"// FP64 tensor-core MMA: D\(16x8\).*\Z", "}\n")
+    small = _replace(read("eig_small.cu"), r'#include "kernels.h"\n', "")
+    small = _replace(small, r"extern __shared__ __align__\(16\) double sm\[\];", "double* sm = emu_smem;")
+    small = _replace(small, r"}  // namespace\s+cudaError_t eig_small_launch.*\Z", "}\n}\n")
+    for name, text in (("cuda_runtime.h", '#include "cta_emulator.h"\n'), ("common.cuh", common),
+                       ("eig_small.cuh", read("eig_small.cuh")), ("eig_small.cu", small)):
+        (tmp / name).write_text(text)
+    lib = tmp / "small_solver.so"
+    r = subprocess.run(["g++", "-std=c++17", "-O2", "-march=native", "-U_FORTIFY_SOURCE", "-fPIC", "-shared", "-w", "-I", str(tmp),
+                        "-I", os.path.join(HERE, "cpp"), os.path.join(HERE, "cpp", "small_solver_cpu.cpp"), "-o", str(lib)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    return ctypes.CDLL(str(lib))
+
+
+def solve(lib, h):
+    """Status, eigenvalues and eigenvector rows of the symmetric matrix with h's upper triangle."""
+    H = np.ascontiguousarray(np.triu(h) + np.triu(h, 1).T)
+    n = len(H)
+    w, v = np.full(n, np.nan), np.full((n, n), np.nan)
+    st = lib.solve(n, *(x.ctypes.data_as(PTR) for x in (H, w, v)), ctypes.c_double(np.nan))
+    return st, w, v
+
+
+def check(lib, h, unit=1.0):
+    """`unit`: a power of two that brings the matrix to order one. Tolerances: 2 n roundings of relative size
+    2^-53 per entry of a vector, in norm."""
+    st, w, v = solve(lib, h)
+    n = len(w)
+    assert st == 0 and np.isfinite(w).all() and np.isfinite(v).all()
+    H = (np.triu(h) + np.triu(h, 1).T) * unit
+    w = w * unit
+    ref = np.linalg.eigvalsh(H)
+    nrm, tol = np.abs(ref).max(), 4 * n * 2.0 ** -52
+    assert (np.diff(w) >= 0).all() and np.abs(w - ref).max() <= tol * nrm
+    assert np.abs(v @ v.T - np.eye(n)).max() <= tol
+    assert np.abs(v @ H - w[:, None] * v).max() <= tol * nrm
+    return w
+
+
+@pytest.mark.parametrize("n", [3, 9, 40, 96])
+@pytest.mark.parametrize("t", [1e-150, 1e-160, 1e-163, 1e-200, 1e-300, 5e-324])
+def test_degenerate_pair(solver, n, t):
+    """Two states of energy zero, coupled by t: the pair's eigenvalues are -t and t."""
+    h = np.diag(np.r_[1.0 / np.arange(1, n - 1), 0.0, 0.0])
+    h[-2, -1] = t
+    w = check(solver, h)
+    assert abs(w[0] + t) <= 1e-15 * t and abs(w[1] - t) <= 1e-15 * t
+
+
+@pytest.mark.parametrize("norm", [2.0 ** -1000, 2.0 ** -1022, 2.0 ** -1060, 2.0 ** 1020])
+def test_norms_without_room_for_the_scale(solver, norm):
+    """Norms whose reciprocal, or the power of two that scales them, is out of range."""
+    for h in (np.array([[1.0, 0.5], [0.0, 1.0]]), np.array([[0.0, 1.0], [0.0, 0.0]])):
+        st, w, v = solve(solver, h * norm)
+        ref = np.linalg.eigvalsh(np.triu(h) + np.triu(h, 1).T)
+        assert st == 0 and np.abs(v @ v.T - np.eye(2)).max() <= 1e-15
+        assert np.abs(w / norm - ref).max() <= 1e-15 + 2 * 5e-324 / norm
