@@ -64,13 +64,13 @@ NRG_DEV void solve_block(const EigBlock& b, double* sm) {
     if (tid < n) bad = !isfinite(d[tid]) || (tid < n - 1 && !isfinite(e[tid]));  // overflow on the way
     if (__syncthreads_or(bad)) st = -2;
   }
+  if (!st) st = smem_dc<R>(d, e, n, Z, U, ld, scr, ctl);
   if (st) {
     if (tid == 0) *b.info = st;
     for (int r = tid; r < n; r += kCtaEigThreads) b.evals[r] = nan("");
     for (int idx = tid; idx < n * n; idx += kCtaEigThreads) b.evecs[idx] = nan("");
     return;
   }
-  st = smem_dc<R>(d, e, n, Z, U, ld, scr, ctl);
   cta_apply_q<R>(Z, ld, n, taus, V);
   if (tid < n) {  // ascending order
     const double di = d[tid];
@@ -79,7 +79,7 @@ NRG_DEV void solve_block(const EigBlock& b, double* sm) {
     perm[rank] = tid;
     b.evals[rank] = di;
   }
-  if (tid == 0) *b.info = st;
+  if (tid == 0) *b.info = 0;
   __syncthreads();
   for (int idx = tid; idx < n * n; idx += kCtaEigThreads) {
     const int r = idx / n, j = idx - r * n;

@@ -141,6 +141,13 @@ NRG_DEV void dc_rows(const double* U, double* Z, int ld, const int* srow, int n,
   }
 }
 
+// x, or zero and ok = false if it is not finite: poles are compared with one another to index memory.
+NRG_DEV double finite_or_zero(double x, bool& ok) {
+  if (isfinite(x)) return x;
+  ok = false;
+  return 0.0;
+}
+
 // Bounds of node p of the 2^depth nodes that halving [0, N) `depth` times gives.
 NRG_DEV void dc_bounds(int p, int depth, int N, int& lo, int& hi) {
   lo = 0;
@@ -154,7 +161,8 @@ NRG_DEV void dc_bounds(int p, int depth, int N, int& lo, int& hi) {
 // Eigenvalues (into d, unsorted) and eigenvectors (rows of Z, row stride ld) of the symmetric
 // tridiagonal matrix (d, e) of order N <= 32 R by divide and conquer in shared memory, 256 threads.
 // U: N x ld doubles, scr: dc_scratch_bytes(N), ctl: 10 ints. Returns 0, or > 0 if a leaf did not
-// converge. d and e must be finite.
+// converge or something came out that is not finite (d and Z then hold no solution, but d no NaN).
+// d and e must be finite.
 // Up to 32 leaves of order <= 4 are solved by one thread each; up to eight nodes of a level are
 // merged at once, 256 / nodes threads each, with the method of the large merges (eig_large.cu:
 // rank-one tearing, deflation, secular roots, Gu-Eisenstat vectors): an order-64 problem takes
@@ -214,15 +222,16 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
         if (i == j && i == 0 && lo > 0) a[i][i] -= fabs(e[lo - 1]);
         if (i == j && lo + i == hi - 1 && hi < N) a[i][i] -= fabs(e[hi - 1]);
       }
-    if (!jacobi4(a, v)) atomicMax(status, lo + 1);
+    bool ok = jacobi4(a, v);
 #pragma unroll
     for (int i = 0; i < 4; i++)
       if (lo + i < hi) {
-        d[lo + i] = a[i][i];
+        d[lo + i] = finite_or_zero(a[i][i], ok);
 #pragma unroll
         for (int j = 0; j < 4; j++)
           if (lo + j < hi) Z[(lo + i) * ld + lo + j] = v[i][j];
       }
+    if (!ok) atomicMax(status, lo + 1);
   }
   __syncthreads();
 
@@ -464,6 +473,7 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
         }
       ss = wsum(ss);
       if (j < K) {
+        if (wl == 0 && !(ss > 0.0 && isfinite(ss))) atomicMax(status, lo + j + 1);
         const double inv = 1.0 / sqrt(ss);
         for (int i = wl; i < K; i += W) row[i] *= inv;
       }
@@ -481,7 +491,11 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
       else if (tn <= 8) dc_rows<8, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);
       else if constexpr (R == 3) dc_rows<12, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);
     }
-    if (gt < n) d[lo + gt] = lamn[lo + gt];
+    if (gt < n) {
+      bool ok = true;
+      d[lo + gt] = finite_or_zero(lamn[lo + gt], ok);
+      if (!ok) atomicMax(status, lo + gt + 1);
+    }
     __syncthreads();
   }
   if (tid < N) d[tid] = scalbn(d[tid], ex);

@@ -1,6 +1,7 @@
 """The one-CTA eigensolver's device code run on the CPU (tests/cpp/cta_emulator.h), on matrices whose
 small numbers leave the range in which squares can be formed: tridiagonal matrices with degenerate
-pairs that are coupled by next to nothing, blocks of denormal norm."""
+pairs that are coupled by next to nothing, blocks of denormal norm; and what it does with numbers that are
+not finite."""
 import ctypes
 import os
 import re
@@ -84,3 +85,15 @@ def test_norms_without_room_for_the_scale(solver, norm):
         ref = np.linalg.eigvalsh(np.triu(h) + np.triu(h, 1).T)
         assert st == 0 and np.abs(v @ v.T - np.eye(2)).max() <= 1e-15
         assert np.abs(w / norm - ref).max() <= 1e-15 + 2 * 5e-324 / norm
+
+
+@pytest.mark.parametrize("n", [4, 9, 33, 64, 67, 96])
+@pytest.mark.parametrize("x", [np.nan, np.inf])
+def test_not_finite_is_flagged_and_indexes_nothing(solver, n, x):
+    """Poles that are not finite (planted here; the kernels check their input) end in a status, and the
+    order of the poles stays a permutation: rows are looked up by it."""
+    for at in (0, n // 2, n - 1):
+        d, e, z = np.arange(1.0, n + 1), np.full(n, 0.1), np.empty((n, n))
+        d[at] = x
+        st = solver.divide_and_conquer(n, *(a.ctypes.data_as(PTR) for a in (d, e, z)), ctypes.c_double(np.nan))
+        assert 0 < st <= n and not np.isnan(d).any()
