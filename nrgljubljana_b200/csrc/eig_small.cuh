@@ -167,7 +167,8 @@ NRG_DEV void dc_bounds(int p, int depth, int N, int& lo, int& hi) {
 // merged at once, 256 / nodes threads each, with the method of the large merges (eig_large.cu:
 // rank-one tearing, deflation, secular roots, Gu-Eisenstat vectors): an order-64 problem takes
 // four levels of some ten thousand cycles where its QL chain is 3500 rotations of 350 cycles.
-// The problem is scaled by a power of two to order one, so the tolerances are relative.
+// The problem is scaled by a power of two to order one, and each merge again, so the tolerances are
+// relative.
 template <int R>
 NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, void* scr, int* ctl) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -242,7 +243,7 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
     int lo, hi;
     dc_bounds(node + 8 * rnd, lev, N, lo, hi);
     const int mid = lo + (hi - lo) / 2, n = hi - lo;
-    const double beta = e[mid - 1], rho = 2.0 * fabs(beta), sg = beta >= 0.0 ? 1.0 : -1.0;
+    const double beta = e[mid - 1], rho0 = 2.0 * fabs(beta), sg = beta >= 0.0 ? 1.0 : -1.0;
     // poles in order (each thread counts the smaller ones), z beside them
     if (gt < n) {
       const double di = d[lo + gt];
@@ -266,11 +267,11 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
       zmx = fmax(zmx, fabs(zv[q]));
     }
     zmx = warp_max(zmx);
-    const double tol = 8.0 * kEps * fmax(fmax(fabs(key[lo]), fabs(key[hi - 1])), rho * zmx);
+    const double tol = 8.0 * kEps * fmax(fmax(fabs(key[lo]), fabs(key[hi - 1])), rho0 * zmx);
     unsigned live[R];
 #pragma unroll
     for (int q = 0; q < R; q++)
-      live[q] = __ballot_sync(0xffffffffu, lane + 32 * q < n && !(rho * fabs(zv[q]) <= tol));
+      live[q] = __ballot_sync(0xffffffffu, lane + 32 * q < n && !(rho0 * fabs(zv[q]) <= tol));
     bool close = false;
 #pragma unroll
     for (int q = 0; q < R; q++) {
@@ -330,6 +331,11 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
         *zj = sn * a + c * b;
       }
     }
+    // The merge in units of 2^ex, in which poles and rho are at most of order one: a node far down a graded
+    // problem (a matrix of low rank leaves remainders of 1e-16, 1e-32, ... of its norm) has poles whose
+    // squares and reciprocal squares the problem's own units do not hold.
+    const int ex = min(1000, max(-1000, ilogb(fmax(fmax(fabs(key[lo]), fabs(key[hi - 1])), rho0))));
+    const double unit = scalbn(1.0, -ex), rho = rho0 * unit;
     int K = 0;
     {
       int before[R];
@@ -349,7 +355,7 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
           const int t = al[q] ? before[q] : K + (s - before[q]);
           srow[lo + t] = sidx[lo + s];
           if (al[q]) {
-            pole[lo + t] = key[lo + s];
+            pole[lo + t] = key[lo + s] * unit;
             zz[lo + t] = zs[lo + s];
           } else {
             lamn[lo + t] = key[lo + s];
@@ -441,7 +447,7 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
       if (act && wl == 0) {
         org[lo + j] = dorg;
         tau[lo + j] = t;
-        lamn[lo + j] = dorg + t;
+        lamn[lo + j] = scalbn(dorg + t, ex);
       }
     }
     __syncthreads();

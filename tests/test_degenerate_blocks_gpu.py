@@ -1,5 +1,5 @@
 """Blocks in which numbers far below the block's norm matter: degenerate states coupled by next to
-nothing, against the oracle's dsyev."""
+nothing, parts that are tiny beside the rest, against the oracle's dsyev."""
 import numpy as np
 import pytest
 
@@ -46,3 +46,14 @@ def test_smallest_norms(nb):
         got = nb.diagonalisations([norm * np.array([[1.0, 0.5], [0.0, 1.0]])])[0]
         assert np.abs(got.val / norm - [0.5, 1.5]).max() <= 1e-15 + 5e-324 / norm
         assert np.abs(got.vec @ got.vec.T - np.eye(2)).max() <= 1e-15
+
+
+def test_tiny_tails(nb, oracle):
+    """Blocks of order one whose last two thirds are a tridiagonal matrix of size x."""
+    blocks = []
+    for x in (1e-100, 1e-155, 1e-163, 1e-300):
+        for n in (12, 20, 40, 64, 96, 300, 700):
+            d, e = np.full(n, x), np.full(n, x)
+            d[: n // 3], e[: n // 3] = 1.0 + np.arange(n // 3), 0.5
+            blocks.append(np.diag(d) + np.diag(e[:-1], 1))
+    check_all(nb, oracle, blocks, small_max_n=96)

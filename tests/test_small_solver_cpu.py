@@ -1,6 +1,6 @@
 """The one-CTA eigensolver's device code run on the CPU (tests/cpp/cta_emulator.h), on matrices whose
 small numbers leave the range in which squares can be formed: tridiagonal matrices with degenerate
-pairs that are coupled by next to nothing, blocks of denormal norm; and what it does with numbers that are
+pairs that are coupled by next to nothing, parts that are tiny beside the rest, blocks of denormal norm; and what it does with numbers that are
 not finite."""
 import ctypes
 import os
@@ -97,3 +97,14 @@ def test_not_finite_is_flagged_and_indexes_nothing(solver, n, x):
         d[at] = x
         st = solver.divide_and_conquer(n, *(a.ctypes.data_as(PTR) for a in (d, e, z)), ctypes.c_double(np.nan))
         assert 0 < st <= n and not np.isnan(d).any()
+
+
+@pytest.mark.parametrize("n", [12, 20, 40, 96])
+@pytest.mark.parametrize("x", [1e-100, 1e-155, 1e-163, 1e-250, 1e-300])
+def test_tiny_tail(solver, n, x):
+    """A tridiagonal matrix of order one whose last two thirds are x: the merges there have poles and couplings of
+    size x. (The reduction leaves such tails of matrices of low rank.)"""
+    d, e = np.full(n, x), np.full(n, x)
+    d[: n // 3], e[: n // 3] = 1.0 + np.arange(n // 3), 0.5
+    h = np.diag(d) + np.diag(e[:-1], 1)
+    check(solver, h)
