@@ -505,7 +505,17 @@ __global__ void __launch_bounds__(kTriThreads, 2) tridiag_kernel(const LargeBloc
     for (int k = p0; k < pe; k++) {
       const int j = k - p0;
       // (1) Householder reflector for rows k+1..n-1 (dlarfg convention, v[k+1] = 1)
-      const double alpha = v[k + 1];
+      double alpha = v[k + 1], unit = 1.0;
+      if (tiny_column(alpha, sigma)) {  // the same in every thread
+        alpha *= kTinyUp;
+        ps = 0.0;
+        for (int i = k + 2 + tid; i < n; i += nt) {
+          v[i] *= kTinyUp;
+          ps = fma(v[i], v[i], ps);
+        }
+        sigma = tiny_squares(block_sum_mma(ps, red, phase));
+        unit = 1.0 / kTinyUp;
+      }
       double tau = 0.0, beta = alpha, scale = 1.0, u1 = 1.0;
       if (sigma > 0.0) {
         beta = -copysign(sqrt(alpha * alpha + sigma), alpha);
@@ -515,7 +525,7 @@ __global__ void __launch_bounds__(kTriThreads, 2) tridiag_kernel(const LargeBloc
       }
       if (tid == 0) {
         B.d[k] = v[k];
-        B.e[k] = beta;
+        B.e[k] = beta * unit;
         B.tau[k] = tau;
       }
       // (2) W^T u and V^T u, four vectors q = warp + 4 c of each per warp; row k+1 of W and V
@@ -685,13 +695,19 @@ __global__ void __launch_bounds__(kMidThreads) tridiag_smem_kernel(const LargeBl
       const double x = P[ck + i];
       ps = fma(x, x, ps);
     }
-    const double sigma = block_sum_1b(ps, red, phase);
-    const double alpha = P[ck + k + 1];
+    double sigma = block_sum_1b(ps, red, phase), alpha = P[ck + k + 1], up = 1.0;
+    if (tiny_column(alpha, sigma)) {  // the same in every thread
+      up = kTinyUp;
+      alpha *= up;
+      ps = 0.0;
+      for (int i = k + 2 + tid; i < n; i += nt) ps = fma(up * P[ck + i], up * P[ck + i], ps);
+      sigma = tiny_squares(block_sum_1b(ps, red, phase));
+    }
     double tau = 0.0, beta = alpha, scale = 1.0;
     if (sigma > 0.0) {
       beta = -copysign(sqrt(alpha * alpha + sigma), alpha);
       tau = (beta - alpha) / beta;
-      scale = 1.0 / (alpha - beta);
+      scale = up / (alpha - beta);
     }
     for (int i = k + 1 + tid; i < n; i += nt) {
       const double vi = (i == k + 1) ? 1.0 : P[ck + i] * scale;
@@ -702,7 +718,7 @@ __global__ void __launch_bounds__(kMidThreads) tridiag_smem_kernel(const LargeBl
     for (int i = kb0 + 1 + tid; i <= k; i += nt) A[(size_t)k * ld + i] = 0.0;
     if (tid == 0) {
       B.d[k] = P[ck + k];
-      B.e[k] = beta;
+      B.e[k] = beta / up;
       B.tau[k] = tau;
     }
     __syncthreads();
@@ -890,7 +906,7 @@ __global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const Large
   }
 
   double ur[kDsmRows] = {};             // u of this thread's rows (of the previous column)
-  double alpha = 0.0, beta = 0.0;       // previous reflector
+  double ek = 0.0;                      // e of the previous column
   for (int k = 0; k < n - 1; k++) {
     const double2* pb = buf + (k & 1) * C * Tm;
     const double tau = sc[2 * (k & 1)], scale = sc[2 * (k & 1) + 1], f = tau * scale;
@@ -908,7 +924,7 @@ __global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const Large
       if (r == k % C)
         for (int i = ((k - 1) / NBT) * NBT + 1 + tid; i < k; i += kDsmThreads) A[(size_t)(k - 1) * ld + i] = 0.0;
       if (tid == 0 && r == 0) {
-        B.e[k - 1] = beta;
+        B.e[k - 1] = ek;
         B.tau[k - 1] = tau;
       }
     }
@@ -949,8 +965,8 @@ __global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const Large
         if (i >= k + 2) ps = fma(ai, ai, ps);
       }
     }
-    const double sigma = block_sum_mma(ps, red, phase);  // its barrier also publishes v, w and u
-    alpha = u[k + 1];
+    double sigma = block_sum_mma(ps, red, phase);  // its barrier also publishes v, w and u
+    double alpha = u[k + 1], unit = 1.0;
     if (tid == 0 && r == 0) B.d[k] = u[k];
     if (k == n - 2) {
       if (tid == 0 && r == 0) {
@@ -964,8 +980,24 @@ __global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const Large
       }
       break;
     }
-    beta = sigma > 0.0 ? -copysign(sqrt(alpha * alpha + sigma), alpha) : alpha;
+    if (tiny_column(alpha, sigma)) {  // the same in every thread of the cluster
+      alpha *= kTinyUp;
+      ps = 0.0;
+#pragma unroll
+      for (int q = 0; q < kDsmRows; q++) {
+        const int i = tid + q * kDsmThreads;
+        if (i >= k + 2 && i < n) {  // u[k+1] may still be read for alpha
+          ur[q] *= kTinyUp;
+          u[i] = ur[q];
+          ps = fma(ur[q], ur[q], ps);
+        }
+      }
+      sigma = tiny_squares(block_sum_mma(ps, red, phase));
+      unit = 1.0 / kTinyUp;
+    }
+    const double beta = sigma > 0.0 ? -copysign(sqrt(alpha * alpha + sigma), alpha) : alpha;
     const double u1 = alpha - beta;  // u[k+1]
+    ek = beta * unit;
 #pragma unroll
     for (int q = 0; q < kDsmRows; q++)
       if (tid + q * kDsmThreads == k + 1) ur[q] = u1;
@@ -1382,8 +1414,18 @@ __global__ void __launch_bounds__(kGridThreads, 1) tridiag_grid_kernel(const Lar
           if (i >= k + 2) ps = fma(a, a, ps);
         }
       }
-      const double sigma = block_sum_mma(ps, red, phase);
-      const double dk = vf[k], alpha = vf[k + 1];
+      double sigma = block_sum_mma(ps, red, phase), alpha = vf[k + 1], unit = 1.0;
+      const double dk = vf[k];
+      if (tiny_column(alpha, sigma)) {  // the same in every thread of the group
+        alpha *= kTinyUp;
+        ps = 0.0;
+        for (int i = k + 2 + tid; i < n; i += kGridThreads) {
+          vf[i] *= kTinyUp;
+          ps = fma(vf[i], vf[i], ps);
+        }
+        sigma = tiny_squares(block_sum_mma(ps, red, phase));
+        unit = 1.0 / kTinyUp;
+      }
       const double beta = sigma > 0.0 ? -copysign(sqrt(alpha * alpha + sigma), alpha) : alpha;
       const double u1 = alpha - beta;
       if (j > 0)
@@ -1436,7 +1478,7 @@ __global__ void __launch_bounds__(kGridThreads, 1) tridiag_grid_kernel(const Lar
       }
       if (tid == 0 && r == 0) {
         B.d[k] = dk;
-        B.e[k] = beta;
+        B.e[k] = beta * unit;
         B.tau[k] = tau;
       }
       if (t0 + tid < T) co[t0 + tid] = ck1;

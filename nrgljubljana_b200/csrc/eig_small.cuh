@@ -536,6 +536,16 @@ NRG_DEV double warp_sum_mma(double x) {
   return e0;
 }
 
+// Householder reflectors of columns (alpha, x) whose squares leave the range of doubles. Where alpha^2 + |x|^2
+// is below 1e-270 (0 for a column that is reduced already), |x|^2 is not known well enough for tau and x
+// to give an orthogonal reflector, nor is A x for its update: the column is multiplied by kTinyUp, its squares
+// are summed again, and the reflector is formed in these units. A column with |x| below 1e-290 counts
+// as reduced. (Such columns come in blocks of norm one: each column of a matrix of low rank leaves a
+// remainder of 1e-16 times the last.)
+constexpr double kTinyUp = 0x1p700;
+NRG_DEV bool tiny_column(double alpha, double sigma) { return fma(alpha, alpha, sigma) < 1e-270; }
+NRG_DEV double tiny_squares(double sum) { return sum > 1e-160 ? sum : 0.0; }
+
 // Householder reduction A = Q T Q^T of the symmetric matrix A of order n <= 32 R (2 <= n) in shared memory
 // (row stride ld, both triangles), 256 threads. On exit d, e, taus and the reflectors v_k packed
 // one after another in V (v_k's n-k-1 entries from row k+1 on, the first one 1).
@@ -591,8 +601,7 @@ NRG_DEV void cta_tridiagonalise(const double* A, int ld, int n, double* d, doubl
       if (warp == 0 && k > 0 && i >= k && i < n) V[vo + i] = v[s];
       if (warp == 1 && i == k) d[k] = u[s];
     }
-    const double sigma = warp_sum_mma(ps);
-    double alpha = 0.0;
+    double sigma = warp_sum_mma(ps), alpha = 0.0, unit = 1.0;
 #pragma unroll
     for (int s = 0; s < R; s++) {
       const double a = __shfl_sync(0xffffffffu, u[s], (k + 1) & 31);
@@ -611,6 +620,17 @@ NRG_DEV void cta_tridiagonalise(const double* A, int ld, int n, double* d, doubl
         taus[k] = taus[n - 1] = 0.0;
       }
       break;
+    }
+    if (tiny_column(alpha, sigma)) {  // the same in every thread
+      alpha *= kTinyUp;
+      ps = 0.0;
+#pragma unroll
+      for (int s = 0; s < R; s++) {
+        u[s] *= kTinyUp;
+        if (lane + 32 * s >= k + 2) ps = fma(u[s], u[s], ps);
+      }
+      sigma = tiny_squares(warp_sum_mma(ps));
+      unit = 1.0 / kTinyUp;
     }
     const double beta = sigma > 0.0 ? -copysign(sqrt(alpha * alpha + sigma), alpha) : alpha;
     const double u1 = alpha - beta;
@@ -642,7 +662,7 @@ NRG_DEV void cta_tridiagonalise(const double* A, int ld, int n, double* d, doubl
       scale = 1.0 / u1;
     }
     if (tid == 0) {
-      e[k] = beta;
+      e[k] = beta * unit;
       taus[k] = tau;
     }
     double* ny = yb + ((k + 1) & 1) * n;

@@ -1,5 +1,5 @@
 """Blocks in which numbers far below the block's norm matter: degenerate states coupled by next to
-nothing, parts that are tiny beside the rest, against the oracle's dsyev."""
+nothing, parts that are tiny beside the rest, matrices of low rank, against the oracle's dsyev."""
 import numpy as np
 import pytest
 
@@ -57,3 +57,46 @@ def test_tiny_tails(nb, oracle):
             d[: n // 3], e[: n // 3] = 1.0 + np.arange(n // 3), 0.5
             blocks.append(np.diag(d) + np.diag(e[:-1], 1))
     check_all(nb, oracle, blocks, small_max_n=96)
+
+
+def low_rank(n, kind, t=0.0):
+    rng = np.random.default_rng(n)
+    if kind == "constant":
+        return np.triu(np.full((n, n), 0.3))
+    if kind == "rank two":
+        a = rng.standard_normal((n, 2))
+        return np.triu(a @ a.T)
+    h = np.triu(rng.standard_normal((n, n)))  # the first row's squares underflow
+    h[0, 1:] *= t
+    return h
+
+
+def test_low_rank_one_cta(nb, oracle):
+    blocks = [low_rank(n, kind) for n in range(2, 97) for kind in ("constant", "rank two")]
+    blocks += [low_rank(n, "tiny column", t) for n in (3, 30, 64, 96) for t in (1e-135, 1e-157, 1e-160, 1e-250)]
+    check_all(nb, oracle, blocks, small_max_n=96)
+
+
+# one block: 16 CTAs in a cluster or a group of many; many: single CTAs, clusters of few
+@pytest.mark.parametrize("n", [70, 128, 230, 449, 601, 900])
+def test_low_rank_larger(nb, oracle, n):
+    for kind, t in (("constant", 0.0), ("rank two", 0.0), ("tiny column", 1e-157), ("tiny column", 1e-161)):
+        check_all(nb, oracle, [low_rank(n, kind, t)])
+    check_all(nb, oracle, [low_rank(m, "constant") for m in (225, 226, 230, 301, 402, 300, 171, 165)])
+
+
+@pytest.mark.parametrize("n,count", [(170, 400), (240, 528), (601, 410)])
+def test_low_rank_in_large_batches(nb, n, count):
+    """The kernels of large batches: one CTA's packed triangle (up to mid_max_n), the streaming reduction."""
+    import torch
+    H0 = [torch.tensor(low_rank(n + i % 3, kind, t), device="cuda")
+          for i in range(3) for kind, t in (("constant", 0.0), ("rank two", 0.0), ("tiny column", 1e-157))]
+    H = [H0[i % len(H0)].clone() for i in range(count)]
+    E = [torch.empty(h.shape[0], dtype=torch.float64, device="cuda") for h in H]
+    V = [torch.empty_like(h) for h in H]
+    assert (nb.diag_batch_device(H, E, V) == 0).all()
+    for i in list(range(len(H0))) + [count - 1]:
+        h, e, v = H0[i % len(H0)], E[i], V[i]
+        Hf, m = h + torch.triu(h, 1).T, h.shape[0]
+        assert torch.linalg.norm(v @ Hf - e[:, None] * v, dim=1).max().item() <= 1e-12 * e.abs().max().item() * m ** 0.5
+        assert (v @ v.T - torch.eye(m, dtype=torch.float64, device="cuda")).abs().max().item() < 1e-10

@@ -1,6 +1,6 @@
 """The one-CTA eigensolver's device code run on the CPU (tests/cpp/cta_emulator.h), on matrices whose
 small numbers leave the range in which squares can be formed: tridiagonal matrices with degenerate
-pairs that are coupled by next to nothing, parts that are tiny beside the rest, blocks of denormal norm; and what it does with numbers that are
+pairs that are coupled by next to nothing, parts that are tiny beside the rest, matrices of low rank, blocks of denormal norm; and what it does with numbers that are
 not finite."""
 import ctypes
 import os
@@ -108,3 +108,28 @@ def test_tiny_tail(solver, n, x):
     d[: n // 3], e[: n // 3] = 1.0 + np.arange(n // 3), 0.5
     h = np.diag(d) + np.diag(e[:-1], 1)
     check(solver, h)
+
+
+@pytest.mark.parametrize("t", [1e-100, 1e-135, 1e-150, 1e-157, 1e-160, 1e-162, 1e-170, 1e-250, 1e-300])
+@pytest.mark.parametrize("n", [3, 17, 64, 96])
+def test_tiny_column(solver, n, t):
+    """The first row couples to the rest by numbers whose squares underflow, wholly or in part."""
+    h = np.random.default_rng(n).standard_normal((n, n))
+    h[0, 1:] *= t
+    check(solver, h)
+
+
+@pytest.mark.parametrize("c", [1.0, 0.3, 0.7, 1 / 3, np.pi])
+def test_constant(solver, c):
+    """Rank one: column after column the reduction leaves 1e-16 of the last."""
+    for n in range(2, 97):
+        check(solver, np.full((n, n), c))
+
+
+@pytest.mark.parametrize("norm", [2.0 ** -500, 2.0 ** -400, 2.0 ** 450])
+def test_graded_in_small_and_large_norms(solver, norm):
+    """Rows of sizes 1 to 1e-150 of the norm, as far down as the doubles go."""
+    for n in (5, 40, 96):
+        rng = np.random.default_rng(n)
+        s = 10.0 ** rng.uniform(-75.0, 0.0, n)
+        check(solver, rng.standard_normal((n, n)) * np.outer(s, s) * norm, unit=1.0 / norm)
