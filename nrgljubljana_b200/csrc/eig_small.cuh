@@ -490,7 +490,8 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
       const double* Un = U + lo * ld + lo;
       double* Zn = Z + lo * ld + lo;
       constexpr int NU = R == 3 ? 2 : 1;  // n <= 12 / 2^level tile rows over 8 / 2^level warps
-      const int tn = (n + 7) / 8;
+      // dc_rows has a barrier, so every node of the level takes the instance of its largest
+      const int tn = ((N + (1 << lev) - 1 >> lev) + 7) / 8;
       if (tn <= 1) dc_rows<1, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);
       else if (tn <= 2) dc_rows<2, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);
       else if (tn <= 4) dc_rows<4, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);

@@ -11,6 +11,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <string>
 #include <vector>
 
 #define __device__
@@ -45,6 +46,8 @@ struct EmuCta {
   std::vector<EmuThread> t;
   std::vector<EmuWarp> w;
   int here = 0, round = 0, any[2] = {0, 0};
+  std::string at;      // where the first thread came to the barrier
+  bool apart = false;  // threads met at different barriers
   jmp_buf sched;
   std::function<void()> body;
 };
@@ -75,9 +78,14 @@ inline uint64_t emu_get(int lane) {
 inline uint64_t emu_bits(double d) { uint64_t u; memcpy(&u, &d, 8); return u; }
 inline double emu_double(uint64_t u) { double d; memcpy(&d, &u, 8); return d; }
 
-inline int __syncthreads_or(int p) {
+inline int emu_barrier(int p, const char* function, int line) {
   const int me = threadIdx.x, r = emu->t[me].bround++;
-  if (emu->here == 0) emu->any[r & 1] = 0;
+  const std::string at = std::string(function) + std::to_string(line);
+  if (emu->here == 0) {
+    emu->any[r & 1] = 0;
+    emu->at = at;
+  }
+  emu->apart |= at != emu->at;
   emu->any[r & 1] |= p != 0;
   if (++emu->here == (int)emu->t.size()) {
     emu->here = 0;
@@ -86,7 +94,8 @@ inline int __syncthreads_or(int p) {
   while (emu->round <= r) emu_yield();
   return emu->any[r & 1];
 }
-inline void __syncthreads() { __syncthreads_or(0); }
+#define __syncthreads_or(p) emu_barrier(p, __PRETTY_FUNCTION__, __LINE__)  // with its template arguments
+#define __syncthreads() emu_barrier(0, __PRETTY_FUNCTION__, __LINE__)
 inline void __syncwarp() { emu_put(0); }
 inline double __shfl_sync(unsigned, double v, int src) {
   emu_put(emu_bits(v));
@@ -131,9 +140,9 @@ inline void emu_entry() {
   emu->t[me].done = true;
   _longjmp(emu->sched, 1);
 }
-// Runs `body` as a CTA of `threads` with `smem` doubles of shared memory, each set to `fill`; false if
-// it wrote outside them.
-inline bool emu_run(int threads, size_t smem, double fill, const std::function<void()>& body) {
+// Runs `body` as a CTA of `threads` with `smem` doubles of shared memory, each set to `fill`: 0, or 1000 if it
+// wrote outside them, or 1001 if threads met at different barriers.
+inline int emu_run(int threads, size_t smem, double fill, const std::function<void()>& body) {
   constexpr size_t kGuard = 4096;
   std::vector<double> mem(smem + 2 * kGuard, 0.5);
   std::fill(mem.begin() + kGuard, mem.end() - kGuard, fill);
@@ -168,6 +177,6 @@ inline bool emu_run(int threads, size_t smem, double fill, const std::function<v
     }
   }
   for (size_t i = 0; i < kGuard; i++)
-    if (mem[i] != 0.5 || mem[mem.size() - 1 - i] != 0.5) return false;
-  return true;
+    if (mem[i] != 0.5 || mem[mem.size() - 1 - i] != 0.5) return 1000;
+  return cta.apart ? 1001 : 0;
 }

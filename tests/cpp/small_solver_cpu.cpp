@@ -13,12 +13,12 @@ struct EigBlock {
 
 using namespace nrg;
 
-// Status of the block (or 1000 if shared memory was overrun); H is n x n, both triangles set.
+// Status of the block (or of emu_run); H is n x n, both triangles set.
 extern "C" int solve(int n, double* H, double* evals, double* evecs, double fill) {
   int info = 0;
   EigBlock b{H, evals, evecs, &info, n};
-  const bool in = emu_run(kCtaEigThreads, small_smem_bytes(n) / 8, fill, [&] { eig_small_kernel(&b); });
-  return in ? info : 1000;
+  const int run = emu_run(kCtaEigThreads, small_smem_bytes(n) / 8, fill, [&] { eig_small_kernel(&b); });
+  return run ? run : info;
 }
 
 // Divide and conquer alone: (d, e) -> eigenvalues (unsorted) in d, eigenvectors as rows of Z.
@@ -27,7 +27,7 @@ extern "C" int divide_and_conquer(int n, double* d, double* e, double* Z, double
   int st = 0;
   int* ctl = static_cast<int*>(calloc(64, sizeof(int)));
   std::vector<double> scr(dc_scratch_bytes(n) / 8 + 1, fill);
-  const bool in = emu_run(kCtaEigThreads, 2 * (size_t)n * ld, fill, [&] {
+  const int run = emu_run(kCtaEigThreads, 2 * (size_t)n * ld, fill, [&] {
     double *z = emu_smem, *u = z + n * ld;
     const int s = n <= 32   ? smem_dc<1>(d, e, n, z, u, ld, scr.data(), ctl)
                   : n <= 64 ? smem_dc<2>(d, e, n, z, u, ld, scr.data(), ctl)
@@ -38,5 +38,5 @@ extern "C" int divide_and_conquer(int n, double* d, double* e, double* Z, double
     }
   });
   free(ctl);
-  return in ? st : 1000;
+  return run ? run : st;
 }

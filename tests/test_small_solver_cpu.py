@@ -133,3 +133,10 @@ def test_graded_in_small_and_large_norms(solver, norm):
         rng = np.random.default_rng(n)
         s = 10.0 ** rng.uniform(-75.0, 0.0, n)
         check(solver, rng.standard_normal((n, n)) * np.outer(s, s) * norm, unit=1.0 / norm)
+
+
+def test_every_order(solver):
+    """All orders, and that all threads of the CTA come to the same barriers (nodes of a level differ in
+    size: of order 67, eighths are of 8 and 9 rows)."""
+    for n in range(1, 97):
+        check(solver, np.random.default_rng(n).standard_normal((n, n)))
