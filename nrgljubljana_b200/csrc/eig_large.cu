@@ -789,9 +789,11 @@ __global__ void __launch_bounds__(kMidThreads) tridiag_smem_kernel(const LargeBl
 //   products with the new reflector -- with both triangles stored a column's product is complete
 //   in its CTA, so no partial sums cross the cluster, at 1.5 times the arithmetic of one triangle;
 //   for each of its columns it sends the product and the element of row k+1 (the next column,
-//   by symmetry) to every CTA by st.async, and waits on its own mbarrier for n-k-1 such pairs.
+//   by symmetry) to every CTA by st.async, and waits on its own mbarrier for these pairs.
 // Pair buffers alternate between consecutive columns: a CTA can send pairs of column k+2 only
-// after it received all of column k+1's, which each other CTA sends after reading column k's.
+// after it received all of column k+1's, which each other CTA sends after reading column k's. For this
+// every CTA has to send something: in the last C columns those that own none of the rest send an empty
+// pair to a slot that nobody reads any more.
 // The reflector is kept unscaled (u = v / scale, so that the product does not wait for the
 // scaling). The rows of a column are summed in the same order whatever C is.
 // Pairs are stored by their sender, so that a warp's stores go to consecutive slots of one CTA at a time
@@ -824,6 +826,10 @@ __host__ __device__ inline size_t dsm_smem_doubles(int n, int C) {
 inline bool dsm_fits(int n, int C) {
   return n <= kDsmMaxN && sizeof(double) * dsm_smem_doubles(n, C) + 512 <= 232448;
 }
+
+// Pairs that each CTA receives after column k: one for each of the n-k-1 columns left, whose owners are
+// min(C, n-k-1) of the CTAs, and an empty one from each other CTA.
+__host__ __device__ inline int dsm_pairs(int n, int C, int k) { return n - k - 1 > C ? n - k - 1 : C; }
 
 NRG_DEV unsigned cluster_addr(unsigned smem_addr, unsigned rank) {
   unsigned a;
@@ -1061,12 +1067,16 @@ __global__ void __launch_bounds__(kDsmThreads, 1) tridiag_dsm_kernel(const Large
     double2* nb = buf + ((k + 1) & 1) * C * Tm;
     if constexpr (C > 1) {
       uint64_t* bar = bars + ((k + 1) & 1);
-      if (tid == 0) mbar_expect_tx(bar, 16u * (unsigned)(n - k - 1));
+      if (tid == 0) mbar_expect_tx(bar, 16u * (unsigned)dsm_pairs(n, C, k));
       // a warp sends its columns' pairs to one CTA at a time, to consecutive slots there
       constexpr int kPer = C < kDsmWarps ? kDsmWarps / C : 1;  // warps per destination
       static_assert(kRowSplit == 4, "pairwise sum of the row parts");
-      for (int t = t0 + lane + 32 * (warp / C); t < T; t += 32 * kPer) {
-        const double yj = (part[t] + part[Tp + t]) + (part[2 * Tp + t] + part[3 * Tp + t]), xj = rowk[t];
+      // (without a column left: an empty pair to the slot of its first one, which is reduced)
+      const bool some = t0 < T;
+      const int end = some ? T : 1;
+      for (int t = (some ? t0 : 0) + lane + 32 * (warp / C); t < end; t += 32 * kPer) {
+        const double yj = some ? (part[t] + part[Tp + t]) + (part[2 * Tp + t] + part[3 * Tp + t]) : 0.0;
+        const double xj = some ? rowk[t] : 0.0;
 #pragma unroll
         for (int dst = warp % C; dst < C; dst += kDsmWarps)
           st_async_pair(cluster_addr(smem_u32(nb + r * Tm + t), dst), yj, xj, cluster_addr(smem_u32(bar), dst));

@@ -17,7 +17,7 @@ using namespace nrg;
 extern "C" int solve(int n, double* H, double* evals, double* evecs, double fill) {
   int info = 0;
   EigBlock b{H, evals, evecs, &info, n};
-  const int run = emu_run(kCtaEigThreads, small_smem_bytes(n) / 8, fill, [&] { eig_small_kernel(&b); });
+  const int run = emu_run(1, kCtaEigThreads, small_smem_bytes(n) / 8, fill, [&] { eig_small_kernel(&b); });
   return run ? run : info;
 }
 
@@ -27,8 +27,8 @@ extern "C" int divide_and_conquer(int n, double* d, double* e, double* Z, double
   int st = 0;
   int* ctl = static_cast<int*>(calloc(64, sizeof(int)));
   std::vector<double> scr(dc_scratch_bytes(n) / 8 + 1, fill);
-  const int run = emu_run(kCtaEigThreads, 2 * (size_t)n * ld, fill, [&] {
-    double *z = emu_smem, *u = z + n * ld;
+  const int run = emu_run(1, kCtaEigThreads, 2 * (size_t)n * ld, fill, [&] {
+    double *z = emu_smem(), *u = z + n * ld;
     const int s = n <= 32   ? smem_dc<1>(d, e, n, z, u, ld, scr.data(), ctl)
                   : n <= 64 ? smem_dc<2>(d, e, n, z, u, ld, scr.data(), ctl)
                             : smem_dc<3>(d, e, n, z, u, ld, scr.data(), ctl);

@@ -29,7 +29,7 @@ def solver(tmp_path_factory):
                       "NRG_DEV void dmma884(double& d0, double& d1, double a, double b) { emu_dmma884(d0, d1, a, b); }\n")
     common = _replace(common, r"// FP64 tensor-core MMA: D\(16x8\).*\Z", "}\n")
     small = _replace(read("eig_small.cu"), r'#include "kernels.h"\n', "")
-    small = _replace(small, r"extern __shared__ __align__\(16\) double sm\[\];", "double* sm = emu_smem;")
+    small = _replace(small, r"extern __shared__ __align__\(16\) double sm\[\];", "double* sm = emu_smem();")
     small = _replace(small, r"}  // namespace\s+cudaError_t eig_small_launch.*\Z", "}\n}\n")
     for name, text in (("cuda_runtime.h", '#include "cta_emulator.h"\n'), ("common.cuh", common),
                        ("eig_small.cuh", read("eig_small.cuh")), ("eig_small.cu", small)):
