@@ -5,6 +5,7 @@
 
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "nrg_b200.h"
@@ -126,6 +127,28 @@ struct CallOrder {
     } else {
       cudaGetLastError();
     }
+  }
+};
+
+// Streams that work beside stream s for a while: s waits for all of them at join(), or when the
+// call is left before that -- the caller may free what they still use once s is through.
+struct SideStreams {
+  cudaStream_t s;
+  std::vector<std::pair<cudaStream_t, cudaEvent_t>> sides;
+  explicit SideStreams(cudaStream_t s_) : s(s_) {}
+  void add(cudaStream_t side, cudaEvent_t ev) { sides.emplace_back(side, ev); }
+  cudaError_t join() {
+    cudaError_t first = cudaSuccess;
+    for (auto& q : sides) {
+      cudaError_t e = cudaEventRecord(q.second, q.first);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(s, q.second, 0);
+      if (first == cudaSuccess) first = e;
+    }
+    sides.clear();
+    return first;
+  }
+  ~SideStreams() {
+    if (join() != cudaSuccess) cudaGetLastError();
   }
 };
 

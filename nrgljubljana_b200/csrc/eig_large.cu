@@ -2856,6 +2856,7 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
     //          that the one-stage reductions fill the SMs its clusters leave idle.
     const bool fork3 = nts > 0 && nts < nb;
     cudaStream_t s3 = s;
+    SideStreams two_stage(s);
     if (fork3) {
       if (!c->side3) {
         NRG_CK(cudaStreamCreateWithFlags(&c->side3, cudaStreamNonBlocking));
@@ -2865,6 +2866,7 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
       NRG_CK(cudaEventRecord(c->fork3_ev, s));
       NRG_CK(cudaStreamWaitEvent(c->side3, c->fork3_ev, 0));
       s3 = c->side3;
+      two_stage.add(s3, c->join3_ev);
     }
     if (nts > 0) {
       for (const BandBlock& Bb : bblk)
@@ -2888,7 +2890,6 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
         NRG_CK(band_chase_launch(dbb, nts, s3));
         NRG_CK(band_q2_tfactor_launch(dbb, nts, blk[0].n, s3));
       }
-      if (fork3) NRG_CK(cudaEventRecord(c->join3_ev, s3));
     }
 
     // ---- 1. tridiagonalisation: blocks beyond cluster_max_n (sorted first) stream through
@@ -2929,6 +2930,7 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
       }
       PhaseScope ps(c, kPhTridiag, s, (ngrid > 0 ? 2 : 0) + (nstream > 0 ? 1 : 0) + (int)ls.size());
       unsigned used = 0;  // side streams with a launch
+      SideStreams sides(s);
       if (ngrid > 0) {
         const GridPlan gp = grid_plan(b1, ngrid, rp.nsm_grid);
         pack_full_kernel<<<dim3((b1[0].ldp + 31) / 32, (b1[0].n + 31) / 32, ngrid), 256, 0, s>>>(d1);
@@ -2965,7 +2967,10 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
         if (side > 0) {
           const int i = (int)(side - 1) % nrg_ctx::kTriStreams;
           ss = c->tri[i];
-          if (!(used >> i & 1)) NRG_CK(cudaStreamWaitEvent(ss, c->tri_fork, 0));
+          if (!(used >> i & 1)) {
+            NRG_CK(cudaStreamWaitEvent(ss, c->tri_fork, 0));
+            sides.add(ss, c->tri_join[i]);
+          }
           used |= 1u << i;
         }
         const LargeBlock* dq = d1 + ls[q].q0;
@@ -2983,16 +2988,13 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
           NRG_CK(reduce_in_smem_launch(dq, nq, count, ls[q].C, ss));
         }
       }
-      for (int i = 0; i < nrg_ctx::kTriStreams; i++)
-        if (used >> i & 1) NRG_CK(cudaEventRecord(c->tri_join[i], c->tri[i]));
       if (beside && pos == 0) {  // the small-block solver takes what SMs are left
         rc = beside();
         if (rc) return rc;
       }
-      for (int i = 0; i < nrg_ctx::kTriStreams; i++)
-        if (used >> i & 1) NRG_CK(cudaStreamWaitEvent(s, c->tri_join[i], 0));
+      NRG_CK(sides.join());
     }
-    if (fork3) NRG_CK(cudaStreamWaitEvent(s, c->join3_ev, 0));  // the two-stage blocks are tridiagonal
+    NRG_CK(two_stage.join());  // all blocks are tridiagonal
     // ---- 2. divide and conquer
     {
       PhaseScope ps(c, kPhDcLeaf, s);
