@@ -304,15 +304,15 @@ __global__ void __launch_bounds__(kThreads) spec_mats_kernel(const SpecRegion* _
         const int n = n0 + q;
         const double wn = pt * (double)(mp.bosonic ? 2 * n : 2 * n + 1);
         double sr = 0.0, si = 0.0;
-        if (n == 0 && mp.bosonic && r.mspecial != kMatsPlain) {
+        if (n == 0 && mp.bosonic) {  // w_0 = 0: the denominator is E^2, whose reciprocal E may put out of range
 #pragma unroll
           for (int k = 0; k < kMatsTerms; k++) {
-            if (fabs(e[k]) <= 1e-8) {
+            if (r.mspecial != kMatsPlain && fabs(e[k]) <= 1e-8) {
               sr += v0[k];
             } else {
-              const double t = w[k] * (1.0 / fma(e[k], e[k], wn * wn));
-              sr = fma(-t, e[k], sr);
-              si = fma(-t, wn, si);
+              const double d = e[k] * e[k];
+              sr -= w[k] * e[k] / d;
+              si -= w[k] * wn / d;
             }
           }
         } else {

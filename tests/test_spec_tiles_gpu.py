@@ -107,3 +107,25 @@ def test_matsubara(nb, oracle, mats, sign):
         spec_accumulate_mats_array({"fdm": 3, "ft": 4, "dmnrg": 0}[algo], rows_of(pairs), mats, re, im, sign, T, wnf)
         got = re.cpu().numpy() + 1j * im.cpu().numpy()
         assert np.abs(got - ref).max() <= TOL * np.abs(ref).max(), algo
+
+
+@pytest.mark.parametrize("E", [5e-155, 1e-155, 1e-120, 1e-9])
+def test_matsubara_small_energy_at_zero_frequency(nb, E):
+    """A discarded x kept term of energy E at the bosonic w_0 = 0 is -w / E, also where 1 / E^2 is out of range
+    (E^2 is then a denormal number, whose spacing is the tolerance)."""
+    import torch
+    from nrgljubljana_b200.api import spec_accumulate_mats_array
+    rng = np.random.default_rng(3)
+    p, d = pair(rng, (1, 0, 1, 1))
+    d["Ei"].zero_()
+    d["Ej"].fill_(E)
+    T, wnf = 0.05, 0.21
+    re = torch.zeros(3, dtype=torch.float64, device="cuda")
+    im = torch.zeros_like(re)
+    spec_accumulate_mats_array(3, rows_of([(p, d)]), 3, re, im, 1, T, wnf)
+    w = p["factor"] * p["op1"][0, 0] * p["op2"][0, 0] * (wnf - p["rj"][0, 0])
+    assert abs(re[0].item() + w / E) <= abs(w / E) * (2.0 ** -48 + 2.0 ** -1074 / (E * E))
+    assert im[0].item() == 0.0
+    for n in (1, 2):
+        wn = 2 * n * math.pi * T
+        assert abs(re[n].item() + w * E / wn ** 2) <= 1e-14 * abs(w / wn) and abs(im[n].item() + w / wn) <= 1e-14 * abs(w / wn)
