@@ -397,10 +397,17 @@ int nrg_diag_batch(nrg_ctx* c, int nblk, const int* n, double* const* H, double*
         base = static_cast<char*>(c->desc);
       }
       if (r) return r;
+      int nsm = 148;
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
+      std::vector<int> orders;
+      for (int b : small) orders.push_back(n[b]);
+      std::vector<int> first = nrg::eig_small_split(orders, nsm);
       {
-        nrg::PhaseScope ps(c, nrg::kPhEigSmall, ss);
-        CK(nrg::eig_small_launch(reinterpret_cast<const nrg::EigBlock*>(base + off), (int)small.size(),
-                                 n[small[0]], ss));
+        nrg::PhaseScope ps(c, nrg::kPhEigSmall, ss, (int)first.size());
+        first.push_back((int)small.size());
+        const nrg::EigBlock* d = reinterpret_cast<const nrg::EigBlock*>(base + off);
+        for (size_t q = 0; q + 1 < first.size(); q++)
+          CK(nrg::eig_small_launch(d + first[q], first[q + 1] - first[q], orders[first[q]], nsm, ss));
       }
       if (fork) CK(cudaEventRecord(c->join_ev, ss));
       return NRG_OK;

@@ -11,35 +11,43 @@
 
 namespace nrg {
 
-constexpr int kCtaEigThreads = 256;
-constexpr int kCtaEigWarps = kCtaEigThreads / 32;
+// Threads T of a CTA, a template parameter: 256 for orders up to 96, or 64 for orders up to 16, in whose merges at
+// most two nodes share a CTA (a node has whole warps).
+constexpr int kCtaEigThreads = 256, kTinyEigThreads = 64, kTinyEigN = 16;
+// The largest order for R and T.
+__host__ __device__ constexpr int cta_eig_max(int R, int T) { return T == kTinyEigThreads ? kTinyEigN : 32 * R; }
 
 // Scratch of smem_dc for order N: ten doubles and five ints per row.
 __host__ __device__ inline size_t dc_scratch_bytes(int N) { return (10 * sizeof(double) + 5 * sizeof(int)) * (size_t)N; }
 
+// Tangent of the rotation that zeroes the coupling apq of two diagonals whose difference is df, the smaller root:
+// 2 a_pq / (df + sgn(df) sqrt(df^2 + 4 a_pq^2)). Couplings between equal diagonals may be of any size, down to
+// the smallest denormal: the squares are formed in units in which they stay in range.
+__host__ __device__ __forceinline__ double jacobi_tangent(double df, double apq) {
+  const double up = fmax(fabs(df), fabs(apq)) < 1e-150 ? 0x1p1000 : 1.0, x = up * df, y = 2.0 * (up * apq);
+  return copysign(y, copysign(1.0, df) * apq) / (fabs(x) + sqrt(fma(x, x, y * y)));
+}
+
 // Eigenvalues a[i][i] and eigenvectors (rows of v) of a symmetric matrix of order 4 by cyclic Jacobi
 // rotations, one thread; of smaller orders with zero rows and columns (zero couplings are
-// skipped). False if 30 sweeps did not converge (five or so do). Couplings between equal diagonals may be
-// of any size, down to the smallest denormal: the tangent is formed in units in which its squares
-// stay in range.
+// skipped). False if 30 sweeps did not converge (five or so do). A sweep begins with whether it has anything to
+// do: the last one does not.
 __host__ __device__ __forceinline__ bool jacobi4(double (&a)[4][4], double (&v)[4][4]) {
 #pragma unroll
   for (int i = 0; i < 4; i++)
 #pragma unroll
     for (int j = 0; j < 4; j++) v[i][j] = i == j ? 1.0 : 0.0;
+  auto active = [&](int p, int q) { return fabs(a[p][q]) > 0.5 * kEps * (fabs(a[p][p]) + fabs(a[q][q])); };
 #pragma unroll 1
-  for (int sweep = 0; sweep < 30; sweep++) {
-    bool any = false;
+  for (int sweep = 0; sweep <= 30; sweep++) {
+    if (!(active(0, 1) || active(2, 3) || active(0, 2) || active(1, 3) || active(0, 3) || active(1, 2))) return true;
 #pragma unroll
     for (int g = 0; g < 6; g++) {  // (0,1) (2,3) (0,2) (1,3) (0,3) (1,2): pairs that overlap, without branches
       constexpr int P[6] = {0, 2, 0, 1, 0, 1}, Q[6] = {1, 3, 2, 3, 3, 2};
       const int p = P[g], q = Q[g];
       const double apq = a[p][q], df = a[q][q] - a[p][p];
-      const bool act = fabs(apq) > 0.5 * kEps * (fabs(a[p][p]) + fabs(a[q][q]));
-      any |= act;
-      // tan of the angle, the smaller root: 2 a_pq / (df + sgn(df) sqrt(df^2 + 4 a_pq^2))
-      const double up = fmax(fabs(df), fabs(apq)) < 1e-150 ? 0x1p1000 : 1.0, x = up * df, y = 2.0 * (up * apq);
-      const double tn = copysign(y, copysign(1.0, df) * apq) / (fabs(x) + sqrt(fma(x, x, y * y)));
+      const bool act = active(p, q);
+      const double tn = jacobi_tangent(df, apq);
       const double t = act ? tn : 0.0, c = act ? rsqrt(fma(t, t, 1.0)) : 1.0, s = t * c;
       a[p][p] = fma(-t, apq, a[p][p]);
       a[q][q] = fma(t, apq, a[q][q]);
@@ -58,7 +66,6 @@ __host__ __device__ __forceinline__ bool jacobi4(double (&a)[4][4], double (&v)[
         v[q][r] = s * xv + c * yv;
       }
     }
-    if (!any) return true;
   }
   return false;
 }
@@ -159,7 +166,7 @@ NRG_DEV void dc_bounds(int p, int depth, int N, int& lo, int& hi) {
 }
 
 // Eigenvalues (into d, unsorted) and eigenvectors (rows of Z, row stride ld) of the symmetric
-// tridiagonal matrix (d, e) of order N <= 32 R by divide and conquer in shared memory, 256 threads.
+// tridiagonal matrix (d, e) of order N <= 32 R by divide and conquer in shared memory, T threads.
 // U: N x ld doubles, scr: dc_scratch_bytes(N), ctl: 10 ints. Returns 0, or > 0 if a leaf did not
 // converge or something came out that is not finite (d and Z then hold no solution, but d no NaN).
 // d and e must be finite.
@@ -169,7 +176,7 @@ NRG_DEV void dc_bounds(int p, int depth, int N, int& lo, int& hi) {
 // four levels of some ten thousand cycles where its QL chain is 3500 rotations of 350 cycles.
 // The problem is scaled by a power of two to order one, and each merge again, so the tolerances are
 // relative.
-template <int R>
+template <int R, int T = kCtaEigThreads>
 NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, void* scr, int* ctl) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   double* key = static_cast<double*>(scr);  // poles, sorted
@@ -200,7 +207,7 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
       *status = 0;
     }
   }
-  for (int i = tid; i < N * ld; i += kCtaEigThreads) Z[i] = 0.0;
+  for (int i = tid; i < N * ld; i += T) Z[i] = 0.0;
   __syncthreads();
   const int ex = ctl[9];
   if (tid < N) {
@@ -210,7 +217,16 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
   }
   const int L = N > 64 ? 5 : N > 32 ? 4 : N > 16 ? 3 : N > 8 ? 2 : N > 4 ? 1 : 0;  // leaves of order 2..4
   __syncthreads();
-  if (tid < 1 << L) {  // leaf `tid`: rank-one tearing at its cuts, then Jacobi
+  if (N == 2) {  // one rotation
+    if (tid == 0 && e[0] != 0.0) {
+      const double t = jacobi_tangent(d[1] - d[0], e[0]), c = rsqrt(fma(t, t, 1.0)), s = t * c;
+      d[0] = fma(-t, e[0], d[0]);
+      d[1] = fma(t, e[0], d[1]);
+      Z[0] = Z[ld + 1] = c;
+      Z[1] = -s;
+      Z[ld] = s;
+    }
+  } else if (tid < 1 << L) {  // leaf `tid`: rank-one tearing at its cuts, then Jacobi
     int lo, hi;
     dc_bounds(tid, L, N, lo, hi);
     double a[4][4], v[4][4];
@@ -239,7 +255,7 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
   // (a level of 16 nodes takes two rounds of eight)
   for (int lev = L - 1, rnd = 0; lev >= 0; rnd == 0 && lev == 4 ? rnd++ : (rnd = 0, lev--)) {
     const int nodes = lev > 3 ? 8 : 1 << lev;
-    const int G = kCtaEigThreads / nodes, node = tid / G, gt = tid % G, wn = gt >> 5, nw = G >> 5;
+    const int G = T / nodes, node = tid / G, gt = tid % G, wn = gt >> 5, nw = G >> 5;
     int lo, hi;
     dc_bounds(node + 8 * rnd, lev, N, lo, hi);
     const int mid = lo + (hi - lo) / 2, n = hi - lo;
@@ -492,11 +508,12 @@ NRG_DEV int smem_dc(double* d, double* e, int N, double* Z, double* U, int ld, v
       constexpr int NU = R == 3 ? 2 : 1;  // n <= 12 / 2^level tile rows over 8 / 2^level warps
       // dc_rows has a barrier, so every node of the level takes the instance of its largest
       const int tn = ((N + (1 << lev) - 1 >> lev) + 7) / 8;
+      constexpr int M = cta_eig_max(R, T) / 8;
       if (tn <= 1) dc_rows<1, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);
       else if (tn <= 2) dc_rows<2, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);
-      else if (tn <= 4) dc_rows<4, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);
-      else if (tn <= 8) dc_rows<8, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);
-      else if constexpr (R == 3) dc_rows<12, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);
+      else if (M > 2 && tn <= 4) dc_rows<M < 4 ? M : 4, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);
+      else if (M > 4 && tn <= 8) dc_rows<M < 8 ? M : 8, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);
+      else if (M > 8) dc_rows<M, NU>(Un, Zn, ld, srow + lo, n, K, wn, nw);
     }
     if (gt < n) {
       bool ok = true;
@@ -548,27 +565,27 @@ NRG_DEV bool tiny_column(double alpha, double sigma) { return fma(alpha, alpha, 
 NRG_DEV double tiny_squares(double sum) { return sum > 1e-160 ? sum : 0.0; }
 
 // Householder reduction A = Q T Q^T of the symmetric matrix A of order n <= 32 R (2 <= n) in shared memory
-// (row stride ld, both triangles), 256 threads. On exit d, e, taus and the reflectors v_k packed
+// (row stride ld, both triangles), T threads. On exit d, e, taus and the reflectors v_k packed
 // one after another in V (v_k's n-k-1 entries from row k+1 on, the first one 1).
-// The matrix moves to registers: warp w has the columns w + 8 q, lane l the rows l + 32 s. As in
+// The matrix moves to registers: warp w of nw has the columns w + nw q, lane l the rows l + 32 s. As in
 // tridiag_dsm_kernel (eig_large.cu) the previous rank-2 update and the product with the new
 // reflector are one pass, and a column costs one barrier: the products and the next row go
 // through shared memory, and every warp builds the reflector for itself.
 // Scratch: yb, rb 2n doubles each, pr 16 n doubles (a (v, w) copy per warp).
-template <int R>
+template <int R, int T = kCtaEigThreads>
 NRG_DEV void cta_tridiagonalise(const double* A, int ld, int n, double* d, double* e, double* taus, double* V,
                                 double* yb, double* rb, double* pr) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int Q = 4 * R;
+  constexpr int nw = T / 32, Q = cta_eig_max(R, T) / nw;
   double x[R][Q];
 #pragma unroll
   for (int s = 0; s < R; s++)
 #pragma unroll
     for (int q = 0; q < Q; q++) {
-      const int i = lane + 32 * s, j = warp + 8 * q;
+      const int i = lane + 32 * s, j = warp + nw * q;
       x[s][q] = i < n && j < n ? A[i * ld + j] : 0.0;
     }
-  for (int i = tid; i < n; i += kCtaEigThreads) {
+  for (int i = tid; i < n; i += T) {
     yb[i] = 0.0;
     rb[i] = A[i];
   }
@@ -614,7 +631,7 @@ NRG_DEV void cta_tridiagonalise(const double* A, int ld, int n, double* d, doubl
       for (int s = 0; s < R; s++)
 #pragma unroll
         for (int q = 0; q < Q; q++)
-          if (lane + 32 * s == n - 1 && warp + 8 * q == n - 1) d[n - 1] = x[s][q] - 2.0 * v[s] * w[s];
+          if (lane + 32 * s == n - 1 && warp + nw * q == n - 1) d[n - 1] = x[s][q] - 2.0 * v[s] * w[s];
       if (tid == 0) {
         e[k] = alpha;
         e[n - 1] = 0.0;
@@ -647,7 +664,7 @@ NRG_DEV void cta_tridiagonalise(const double* A, int ld, int n, double* d, doubl
     // behind a branch would wait for one another
     double2 c[Q];
 #pragma unroll
-    for (int q = 0; q < Q; q++) c[q] = vw[min(warp + 8 * q, n - 1)];
+    for (int q = 0; q < Q; q++) c[q] = vw[min(warp + nw * q, n - 1)];
 #pragma unroll
     for (int q = 0; q < Q; q++)
 #pragma unroll
@@ -673,7 +690,7 @@ NRG_DEV void cta_tridiagonalise(const double* A, int ld, int n, double* d, doubl
       if (lane + 32 * s == k + 1) {
 #pragma unroll
         for (int q = 0; q < Q; q++)
-          if (warp + 8 * q < n) nr[warp + 8 * q] = x[s][q];
+          if (warp + nw * q < n) nr[warp + nw * q] = x[s][q];
       }
 #pragma unroll
     for (int g = 0; g < (Q + 7) / 8; g++) {
@@ -681,7 +698,7 @@ NRG_DEV void cta_tridiagonalise(const double* A, int ld, int n, double* d, doubl
 #pragma unroll
       for (int c = 0; c < 8; c++) t[c] = cs[8 * g + c];
       const double sum = colsum8(t, lane);
-      const int j = warp + 8 * (8 * g + (lane >> 2));
+      const int j = warp + nw * (8 * g + (lane >> 2));
       if ((lane & 3) == 0 && j < n) ny[j] = sum;
     }
     __syncthreads();
@@ -691,11 +708,11 @@ NRG_DEV void cta_tridiagonalise(const double* A, int ld, int n, double* d, doubl
 
 // Rows of Z <- rows of Z Q^T: every row z becomes H_0 H_1 ... H_{n-3} z. Four lanes hold a row in
 // registers (columns 4 q + l), so the reflectors follow one another without a barrier.
-template <int R>
+template <int R, int T = kCtaEigThreads>
 NRG_DEV void cta_apply_q(double* Z, int ld, int n, const double* taus, const double* V) {
   const int tid = threadIdx.x, l = tid & 3;
-  constexpr int Q = 8 * R;
-  for (int r0 = 0; r0 < n; r0 += kCtaEigThreads / 4) {  // uniform
+  constexpr int Q = cta_eig_max(R, T) / 4;
+  for (int r0 = 0; r0 < n; r0 += T / 4) {  // uniform
     const int r = r0 + (tid >> 2);
     double z[Q];
 #pragma unroll

@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "nrg_b200.h"
 
 namespace nrg {
@@ -75,7 +77,10 @@ constexpr int kMidMaxNLimit = 236;   // the packed triangle of the most the 227 
 constexpr int kClusterMaxN = 600;    // default: cluster (distributed shared memory) reduction up to here
 constexpr int kClusterMaxNLimit = 640;  // the most an 8-CTA cluster's shared memory holds
 
-cudaError_t eig_small_launch(const EigBlock* d_blocks, int nblk, int maxn, cudaStream_t stream);
+// First blocks of the launches for blocks of orders n (falling) on nsm SMs.
+std::vector<int> eig_small_split(const std::vector<int>& n, int nsm);
+// One of them: nblk blocks up to order maxn.
+cudaError_t eig_small_launch(const EigBlock* d_blocks, int nblk, int maxn, int nsm, cudaStream_t stream);
 
 // ---------------------------------------------------------------- Hamiltonian assembly
 // One block of nrg_hamiltonian_batch: its matrix, order, first tile and its pieces

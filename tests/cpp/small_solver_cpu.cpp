@@ -13,11 +13,14 @@ struct EigBlock {
 
 using namespace nrg;
 
-// Status of the block (or of emu_run); H is n x n, both triangles set.
-extern "C" int solve(int n, double* H, double* evals, double* evecs, double fill) {
+// Status of the block (or of emu_run) with the CTA of `threads`; H is n x n, both triangles set.
+extern "C" int solve(int n, int threads, double* H, double* evals, double* evecs, double fill) {
   int info = 0;
   EigBlock b{H, evals, evecs, &info, n};
-  const int run = emu_run(1, kCtaEigThreads, small_smem_bytes(n) / 8, fill, [&] { eig_small_kernel(&b); });
+  const size_t smem = small_smem_bytes(n) / 8;
+  const int run =
+      threads == kTinyEigThreads ? emu_run(1, kTinyEigThreads, smem, fill, [&] { eig_small_kernel<1, kTinyEigThreads, 1>(&b); })
+                                 : emu_run(1, kCtaEigThreads, smem, fill, [&] { eig_small_kernel<3, kCtaEigThreads, 1>(&b); });
   return run ? run : info;
 }
 

@@ -30,7 +30,7 @@ def solver(tmp_path_factory):
     common = _replace(common, r"// FP64 tensor-core MMA: D\(16x8\).*\Z", "}\n")
     small = _replace(read("eig_small.cu"), r'#include "kernels.h"\n', "")
     small = _replace(small, r"extern __shared__ __align__\(16\) double sm\[\];", "double* sm = emu_smem();")
-    small = _replace(small, r"}  // namespace\s+cudaError_t eig_small_launch.*\Z", "}\n}\n")
+    small = _replace(small, r"template <int R, int T, int CTAS>\s+cudaError_t launch.*\Z", "}\n}\n")
     for name, text in (("cuda_runtime.h", '#include "cta_emulator.h"\n'), ("common.cuh", common),
                        ("eig_small.cuh", read("eig_small.cuh")), ("eig_small.cu", small)):
         (tmp / name).write_text(text)
@@ -42,19 +42,26 @@ def solver(tmp_path_factory):
     return ctypes.CDLL(str(lib))
 
 
-def solve(lib, h):
-    """Status, eigenvalues and eigenvector rows of the symmetric matrix with h's upper triangle."""
+def solve(lib, h, threads=256):
+    """Status, eigenvalues and eigenvector rows of the symmetric matrix with h's upper triangle; by 64 threads up
+    to order 16."""
     H = np.ascontiguousarray(np.triu(h) + np.triu(h, 1).T)
     n = len(H)
     w, v = np.full(n, np.nan), np.full((n, n), np.nan)
-    st = lib.solve(n, *(x.ctypes.data_as(PTR) for x in (H, w, v)), ctypes.c_double(np.nan))
+    st = lib.solve(n, threads, *(x.ctypes.data_as(PTR) for x in (H, w, v)), ctypes.c_double(np.nan))
     return st, w, v
 
 
 def check(lib, h, unit=1.0):
+    for threads in (64, 256) if len(h) <= 16 else (256,):
+        w = check_with(lib, h, unit, threads)
+    return w
+
+
+def check_with(lib, h, unit, threads):
     """`unit`: a power of two that brings the matrix to order one. Tolerances: 2 n roundings of relative size
     2^-53 per entry of a vector, in norm."""
-    st, w, v = solve(lib, h)
+    st, w, v = solve(lib, h, threads)
     n = len(w)
     assert st == 0 and np.isfinite(w).all() and np.isfinite(v).all()
     H = (np.triu(h) + np.triu(h, 1).T) * unit
@@ -80,8 +87,9 @@ def test_degenerate_pair(solver, n, t):
 @pytest.mark.parametrize("norm", [2.0 ** -1000, 2.0 ** -1022, 2.0 ** -1060, 2.0 ** 1020])
 def test_norms_without_room_for_the_scale(solver, norm):
     """Norms whose reciprocal, or the power of two that scales them, is out of range."""
-    for h in (np.array([[1.0, 0.5], [0.0, 1.0]]), np.array([[0.0, 1.0], [0.0, 0.0]])):
-        st, w, v = solve(solver, h * norm)
+    for h, threads in ((h, t) for t in (64, 256) for h in (np.array([[1.0, 0.5], [0.0, 1.0]]),
+                                                           np.array([[0.0, 1.0], [0.0, 0.0]]))):
+        st, w, v = solve(solver, h * norm, threads)
         ref = np.linalg.eigvalsh(np.triu(h) + np.triu(h, 1).T)
         assert st == 0 and np.abs(v @ v.T - np.eye(2)).max() <= 1e-15
         assert np.abs(w / norm - ref).max() <= 1e-15 + 2 * 5e-324 / norm
