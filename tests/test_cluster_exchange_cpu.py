@@ -62,6 +62,24 @@ def reduce(lib, h, C, slow):
     return st, d, e, tau, W1
 
 
+@pytest.mark.parametrize("n,C", [(19, 2), (34, 16)])
+@pytest.mark.parametrize("kind", ["diagonal", "tridiagonal", "two parts", "last rows", "every other column"])
+def test_columns_that_are_reduced_already(reduction, n, C, kind):
+    h = np.triu(np.random.default_rng(n).standard_normal((n, n)))
+    i, j = np.indices((n, n))
+    h[{"diagonal": i != j, "tridiagonal": j > i + 1, "two parts": (i < n // 2) & (j >= n // 2),
+       "last rows": (i != j) & (i < n - 5), "every other column": (i % 2 == 0) & (j > i + 1)}[kind]] = 0.0
+    st, d, e, tau, W1 = reduce(reduction, h, C, -1)
+    H = np.triu(h) + np.triu(h, 1).T
+    Q = np.eye(n)
+    for k in range(n - 3, -1, -1):
+        v = np.r_[np.zeros(k + 1), W1[k, k + 1:n]]
+        Q -= tau[k] * np.outer(v, v @ Q)
+    T = np.diag(d) + np.diag(e[:-1], 1) + np.diag(e[:-1], -1)
+    assert st == 0 and np.abs(Q @ Q.T - np.eye(n)).max() <= 1e-14
+    assert np.abs(Q @ T @ Q.T - H).max() <= 1e-14 * np.abs(H).max() * n
+
+
 @pytest.mark.parametrize("n,C", [(19, 2), (21, 4), (21, 8), (21, 16), (34, 16)])
 def test_any_cta_may_lag(reduction, n, C):
     h = np.triu(np.random.default_rng(n).standard_normal((n, n)))

@@ -100,3 +100,16 @@ def test_low_rank_in_large_batches(nb, n, count):
         Hf, m = h + torch.triu(h, 1).T, h.shape[0]
         assert torch.linalg.norm(v @ Hf - e[:, None] * v, dim=1).max().item() <= 1e-12 * e.abs().max().item() * m ** 0.5
         assert (v @ v.T - torch.eye(m, dtype=torch.float64, device="cuda")).abs().max().item() < 1e-10
+
+
+@pytest.mark.parametrize("n", [40, 96, 150, 300, 700, 1100])
+def test_columns_that_are_reduced_already(nb, oracle, n):
+    """Columns without a reflector: all of them (a subspace with one ancestor), whole panels, every other one."""
+    i, j = np.indices((n, n))
+    blocks = []
+    for zero in (i != j, j > i + 1, (i < n // 2) & (j >= n // 2), (i != j) & (i < n - 20), (i % 2 == 0) & (j > i + 1),
+                 (i % 48 < 32) & (j > i + 1)):
+        h = np.triu(np.random.default_rng(n).standard_normal((n, n)))
+        h[zero] = 0.0
+        blocks.append(h)
+    check_all(nb, oracle, blocks, small_max_n=96)

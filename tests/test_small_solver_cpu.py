@@ -143,6 +143,12 @@ def test_graded_in_small_and_large_norms(solver, norm):
         check(solver, rng.standard_normal((n, n)) * np.outer(s, s) * norm, unit=1.0 / norm)
 
 
+def test_diagonal(solver):
+    for n in (1, 2, 16, 17, 64, 96):
+        w = check(solver, np.diag(np.round(np.random.default_rng(n).standard_normal(n), 1)))
+        assert len(w) == n
+
+
 def test_every_order(solver):
     """All orders, and that all threads of the CTA come to the same barriers (nodes of a level differ in
     size: of order 67, eighths are of 8 and 9 rows)."""
