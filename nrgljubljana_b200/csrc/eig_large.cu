@@ -1752,7 +1752,7 @@ __global__ void __launch_bounds__(512) dc_prep_kernel(const LargeBlock* __restri
   if (__syncthreads_or(badidx)) {
     for (int s = tid; s < N; s += nt) B.slot[a + s] = make_int2(s, a + s < m ? 1 : 2);
     if (tid == 0) {
-      atomicMin(B.info, -3);
+      atomicCAS(B.info, 0, -3);
       DcState st{};
       st.rho = rho;
       states[blockIdx.x] = st;
