@@ -722,7 +722,7 @@ __global__ void __launch_bounds__(kMidThreads) tridiag_smem_kernel(const LargeBl
       B.tau[k] = tau;
     }
     __syncthreads();
-    if (tau == 0.0) continue;  // uniform: every thread computed the same sigma
+    if (sigma == 0.0) continue;  // uniform; with a sigma that is not a number the update has to spread it
     // w = tau * A22 v over rows/columns k+1..n-1; thread i reads row i left of the
     // diagonal and column i from the diagonal down: n-k-1 entries for every i
     for (int i = k + 1 + tid; i < n; i += nt) {

@@ -5,7 +5,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,count", [(12, 3), (40, 5), (64, 400), (100, 1), (230, 3), (240, 528), (480, 2), (700, 2)])
+@pytest.mark.parametrize("n,count", [(12, 3), (40, 5), (64, 400), (100, 1), (170, 400), (230, 3), (240, 528), (480, 2), (700, 2)])
 @pytest.mark.parametrize("x", [float("nan"), float("inf")])
 def test_status(n, count, x):
     import torch
