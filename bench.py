@@ -327,27 +327,19 @@ def main():
     value = world * args.steps * flop_step / elapsed / 1e9
     launches = int(sum(v[1] for v in phases.values()))
 
-    # roofline of the dominant kernel
+    # roofline of the dominant phase: the kernels that reduce the blocks run side by side, so the
+    # phase is taken as a whole, with the bytes that streaming every block's triangle once per column takes
     peaks = measured_peaks()
     top = max(phases.items(), key=lambda kv: kv[1][0])
-    roof = None
-    # DRAM bytes per launch of tridiag_kernel relative to its algorithmic bytes, from one ncu
-    # capture of the kernel as the benchmark's batch launches it (three CTAs per SM, the slabs
-    # of the trailing triangle loaded with an L2 evict-first hint, the panel vectors with an
-    # evict-last one) on 1400 blocks of n = 608: dram__bytes_read.sum + dram__bytes_write.sum =
-    # 516.49 + 28.50 GB for 467.99 GB algorithmic; the ratio carries over to larger launches
-    # because both grow with the per-column reads of the trailing triangle.
-    tridiag_traffic_ratio = (516.49 + 28.50) / 467.99
     if top[0] == "tridiag":
-        per_launch_bytes = args.steps * sum(tridiag_bytes(int(n)) for n in sizes if n > 64) / top[1][1]
-        avg = top[1][0] / 1e3 / top[1][1]
-        ach = per_launch_bytes / avg / 1e9
+        step_bytes = sum(tridiag_bytes(int(n)) for n in sizes if n > 64)
+        sec = top[1][0] / 1e3 / args.steps
+        ach = step_bytes / sec / 1e9
         pk = peaks.get("hbm_gbs", 6650.0)
-        roof = {"kernel": "tridiag_kernel", "bound": "hbm", "achieved": ach, "peak": pk, "unit": "GB/s",
-                "frac": ach / pk, "traffic": per_launch_bytes * tridiag_traffic_ratio,
-                "traffic_source": "ncu dram bytes of an earlier tridiag_kernel (three CTAs per SM) on 1400 x n=608 (profiles/tridiag_kernel_1400x608.md), scaled by algorithmic bytes",
+        roof = {"kernel": "tridiag_kernel beside tridiag_grid_kernel, tridiag_dsm_kernel and tridiag_smem_kernel",
+                "bound": "hbm", "achieved": ach, "peak": pk, "unit": "GB/s", "frac": ach / pk, "traffic": None,
                 "peak_source": "measured" if "hbm_gbs" in peaks else "fallback",
-                "bytes_per_launch": per_launch_bytes, "avg_launch_ms": avg * 1e3}
+                "bytes_per_step": step_bytes, "phase_ms_per_step": sec * 1e3}
     else:
         roof = {"kernel": top[0], "bound": "tensor", "achieved": None, "peak": None, "unit": "TFLOP/s",
                 "frac": None, "traffic": None}

@@ -68,7 +68,8 @@ NRG_API int nrg_trim(nrg_ctx* ctx);
  *   mid_max_n      in batches of many blocks, larger ones up to this order are reduced to
  *                  tridiagonal form in the shared memory of one CTA (small_max_n..236)
  *   cluster_max_n  larger blocks up to this order are reduced in the distributed shared
- *                  memory of a thread-block cluster of 1 to 16 CTAs (mid_max_n..640);
+ *                  memory of a thread-block cluster of 1 to 16 CTAs (mid_max_n..640; 16 CTAs
+ *                  hold orders up to 624, and those above count as larger);
  *                  larger ones by groups of CTAs through L2; in batches of many blocks
  *                  the streaming reduction, two CTAs per SM, takes those above mid_max_n
  *                  that it finishes in the time the batch needs
@@ -98,8 +99,10 @@ NRG_API int nrg_set_tuning(nrg_ctx* ctx, const nrg_tuning* in);
  *              as the reference consumes its argument (c++/diag.hpp:259-260)
  *   evals[b]   n doubles, ascending
  *   evecs[b]   n x n row-major, row r = eigenvector of evals[b][r]
- *   info       host array of nblk status words: 0 ok; -2 non-finite input; > 0 the
- *              tridiagonal iteration did not converge (the reference's INFO != 0)
+ *   info       host array of nblk status words: 0 ok; -2 non-finite input (or overflow on the
+ *              way); > 0 the solution of the tridiagonal problem did not converge (the
+ *              reference's INFO != 0); -5 a bounded wait inside a kernel ran out; -3 poles of a
+ *              merge that are not finite. A block with a status other than 0 has no results.
  * H, evals, evecs are host arrays of device pointers; evecs[b] must not alias H[b]. */
 #define NRG_DIAG_MAX_N 10240
 NRG_API int nrg_diag_batch(nrg_ctx* ctx, int nblk, const int* n, double* const* H, double* const* evals,

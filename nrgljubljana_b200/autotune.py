@@ -1,10 +1,11 @@
 """Autotuner of the batched eigensolver's launch parameters (nrg_tuning, include/nrg_b200.h).
 
-The eigensolver sends each block of a step down one of four paths by its order: the
+The eigensolver sends each block of a step down one of five paths by its order: the
 one-CTA solver (n <= small_max_n), the reduction in the shared memory of one CTA or of a
 cluster (n <= cluster_max_n; one CTA up to mid_max_n in large batches), the reduction by groups of
-CTAs through L2 and, in batches of many blocks, the streaming reduction from HBM (not used with
-reduction_ctas_per_sm = 1). Where the crossovers lie depends on the device, so they are measured, not assumed: the reference's own
+CTAs through L2, in batches of many blocks the streaming reduction from HBM (not used with
+reduction_ctas_per_sm = 1) and, where band_min_n switches it on, the two-stage reduction. Where the
+crossovers lie depends on the device, so they are measured, not assumed: the reference's own
 scheduler (c++/core.hpp:98-107, c++/subspaces.hpp:103-123) only orders the blocks largest
 first; on a GPU the choice of path per block is the equivalent decision.
 
@@ -45,12 +46,12 @@ SEED = 20261203
 GRID = {
     "small_max_n": [32, 48, 64, 80, 96],
     "mid_max_n": [128, 160, 192, 224, 236],
-    "cluster_max_n": [400, 480, 560, 600, 640],
+    "cluster_max_n": [400, 480, 560, 600, 624],
     # The two-stage path's bulge chasing has a critical path of about 3n dependent steps; the
     # reduction by groups of CTAs overtakes it at every order measured (a step of 24 blocks in
     # [200, 7049] takes 468 ms, 663 with the blocks from 3072 on in two stages).
     "band_min_n": [0, 2048, 3072, 4096],
-    "reduction_ctas_per_sm": [1, 2, 3],
+    "reduction_ctas_per_sm": [1, 3],  # 1: nothing streams; 2 and 3 are the same plan
     "band_max_blocks": [4, 8, 16, 32, 64],
 }
 KEYS = ("small_max_n", "mid_max_n", "cluster_max_n", "reduction_ctas_per_sm", "band_min_n", "band_max_blocks")

@@ -807,7 +807,7 @@ __global__ void __launch_bounds__(kMidThreads) tridiag_smem_kernel(const LargeBl
 // of its back-transform panel up to k).
 constexpr int kDsmThreads = 256;
 constexpr int kDsmWarps = kDsmThreads / 32;
-constexpr int kDsmMaxN = 640;                        // the largest cluster_max_n; what shared memory holds ends at 607
+constexpr int kDsmMaxN = 640;                        // the largest cluster_max_n; 16 CTAs hold orders up to 624
 constexpr int kDsmRows = (kDsmMaxN + kDsmThreads - 1) / kDsmThreads;  // rows of the vectors per thread
 constexpr int kRowSplit = 4, kColSplit = kDsmWarps / kRowSplit;
 
@@ -2892,8 +2892,8 @@ int eig_large_run(nrg_ctx* c, const std::vector<int>& which, const int* n, doubl
       }
     }
 
-    // ---- 1. tridiagonalisation: blocks beyond cluster_max_n (sorted first) stream through
-    //         TMA, the rest are reduced in the shared memory of a cluster or one CTA
+    // ---- 1. tridiagonalisation, split by reduction_plan: blocks sorted by falling order go to the groups
+    //         of CTAs, then to the clusters, the streaming kernel and the one-CTA kernel
     {
       int nsm = 148;
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);

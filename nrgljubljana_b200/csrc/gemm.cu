@@ -274,7 +274,7 @@ constexpr int kStagesL = 2, kMinL = 4, kStagesS = 3, kMinS = 5;
 template <int BM, int BN, int STAGES>
 constexpr size_t gemm_smem() { return sizeof(double) * (stage_doubles(BM) + stage_doubles(BN)) * STAGES; }
 
-// Dynamic shared memory beyond 48 KB has to be asked for, once per device and kernel.
+// Dynamic shared memory beyond 48 KB has to be asked for, per device and kernel; every launch does.
 template <typename F>
 cudaError_t allow_smem(F* fn, size_t bytes) {
   return cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,

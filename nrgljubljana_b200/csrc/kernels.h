@@ -70,12 +70,12 @@ struct EigBlock {
   int n, pad_;
 };
 
-constexpr int kSmallMaxN = 64;   // default: blocks up to this size are solved entirely in shared memory
-constexpr int kSmallMaxNLimit = 96;  // the most the one-CTA solver's shared memory holds
+constexpr int kSmallMaxN = 64;   // default: blocks up to this size are solved whole by one CTA
+constexpr int kSmallMaxNLimit = 96;  // the one-CTA solver's warps hold three rows of a column per lane
 constexpr int kMidMaxN = 224;        // default: one-CTA shared-memory reduction up to this order
 constexpr int kMidMaxNLimit = 236;   // the packed triangle of the most the 227 KB of one CTA holds
 constexpr int kClusterMaxN = 600;    // default: cluster (distributed shared memory) reduction up to here
-constexpr int kClusterMaxNLimit = 640;  // the most an 8-CTA cluster's shared memory holds
+constexpr int kClusterMaxNLimit = 640;  // largest cluster_max_n (16 CTAs hold orders up to 624; the rest go to the groups)
 
 // First blocks of the launches for blocks of orders n (falling) on nsm SMs.
 std::vector<int> eig_small_split(const std::vector<int>& n, int nsm);
